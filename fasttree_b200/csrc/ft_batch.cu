@@ -34,6 +34,7 @@
 #include "ft_common.cuh"
 #include "ft_cta_build.cuh"
 #include "ft_internal.h"
+#include "ft_qtree.cuh"
 
 namespace ft {
 
@@ -293,20 +294,26 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// The fast walks' view of every set's tree, as qtree_kernel's for one tree: global leaf g and,
+// inside its set, the internal node of the same number.
 template <class T>
 __global__ void __launch_bounds__(256)
-    batch_collapse_kernel(const long long *__restrict__ off, const long long *__restrict__ node_off,
-                          const long long *__restrict__ rec_off, int S, long long N, const int32_t *__restrict__ left,
-                          const int32_t *__restrict__ right, const T *mnx, const T *mxx, const T *mny, const T *mxy,
-                          const T *mnz, const T *mxz, WideRec<T> *wide) {
-    const long long total = rec_off[S];
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N && g < total;
-         g += (long long)gridDim.x * blockDim.x) {
-        const int       s  = find_set(rec_off, S, g);
+    batch_qtree_kernel(const long long *__restrict__ off, const long long *__restrict__ node_off,
+                       const long long *__restrict__ rec_off, int S, long long N, const NodeRec<T> *__restrict__ recs,
+                       const int32_t *__restrict__ leaves, const T *mnx, const T *mxx, const T *mny, const T *mxy,
+                       const T *mnz, const T *mxz, int periodic, QRec *qrec, QPoint *qpts, uint32_t *flag) {
+    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
+        const int       s  = find_set(off, S, g);
         const long long ro = rec_off[s], no = node_off[s];
-        const int       n  = (int)(off[s + 1] - off[s]);
-        const T *const  soa[6] = {mnx + no, mxx + no, mny + no, mxy + no, mnz + no, mxz + no};
-        collapse_node<T>((int)(g - ro), n, left + ro, right + ro, soa, wide + ro);
+        const int       n  = (int)(off[s + 1] - off[s]), j = (int)(g - off[s]);
+        const T         rb[6] = {mnx[no], mxx[no], mny[no], mxy[no], mnz[no], mxz[no]};
+        QFrame<T>       f;
+        f.make(rb, n, periodic != 0);
+        if (!f.ok && j == 0) atomicOr(flag + s, f.flag());
+        const long long slot = no + n - 1 + j;
+        qpts[g]              = qpoint<T>(mnx[slot], mny[slot], mnz[slot], f, periodic != 0, flag + s);
+        if (j < n - 1 && (j == 0 || leaves[ro + j] > kBucket))
+            qrec_node<T>(j, n, recs + ro, leaves + ro, f, qrec + ro, flag + s);
     }
 }
 
@@ -440,7 +447,9 @@ BatchImpl *batch_create(Context &ctx, size_t max_points, size_t max_sets) {
     s.height      = dalloc<uint8_t>(P);
     s.counters    = dalloc<int32_t>(P);
     s.leafcount   = dalloc<int32_t>(P);
-    s.wide        = dalloc<unsigned char>(P * wide_bytes(o.coord_type));
+    s.qrec        = dalloc<QRec>(P);
+    s.qpts        = dalloc<QPoint>(P);
+    s.qflag       = dalloc<uint32_t>(max_sets);
     s.key_lo      = (uint64_t *)dalloc<unsigned long long>(P);
     s.tmp_lo      = (uint64_t *)dalloc<unsigned long long>(P);
     if (o.coord_type == U64) { // 126-bit keys (built by the persistent launch only)
@@ -570,8 +579,10 @@ static void batch_build_typed(Context &ctx, BatchImpl &b, const long long *in_of
     batch_refit_stream_kernel<T><<<grid_of((size_t)N, 256, sm * 8), 256, 0, st>>>(
         b.off, b.node_off, b.rec_off, S, N, t.left_child, t.right_child, t.parent, mnx, mxx, mny, mxy, mnz, mxz,
         (NodeRec<T> *)s.recs, s.height, s.counters, s.leafcount, s.counters + (N - 1));
-    batch_collapse_kernel<T><<<gK, 256, 0, st>>>(b.off, b.node_off, b.rec_off, S, N, t.left_child, t.right_child,
-                                                 mnx, mxx, mny, mxy, mnz, mxz, (WideRec<T> *)s.wide);
+    FT_CUDA(cudaMemsetAsync(s.qflag, 0, (size_t)S * sizeof(uint32_t), st));
+    batch_qtree_kernel<T><<<gK, 256, 0, st>>>(b.off, b.node_off, b.rec_off, S, N, (const NodeRec<T> *)s.recs,
+                                              s.leafcount, mnx, mxx, mny, mxy, mnz, mxz, o.periodic, (QRec *)s.qrec,
+                                              (QPoint *)s.qpts, s.qflag);
     batch_heights_kernel<<<grid_of((size_t)S, 256, sm * 4), 256, 0, st>>>(b.off, b.rec_off, S, s.height,
                                                                           b.set_height);
     FT_CUDA(cudaGetLastError());
@@ -603,6 +614,7 @@ static void batch_build_persistent(Context &ctx, BatchImpl &b, const long long *
     FT_CUDA(cudaMemsetAsync(b.ctl, 0, 4 * sizeof(uint32_t), st));
     FT_CUDA(cudaMemsetAsync(b.ready, 0xFF, S * sizeof(int32_t), st));
     FT_CUDA(cudaMemsetAsync(b.chunk_next, 0, S * sizeof(int32_t), st));
+    FT_CUDA(cudaMemsetAsync(b.scr.qflag, 0, S * sizeof(uint32_t), st));
     if (q) FT_CUDA(cudaMemsetAsync(b.counters, 0, 8 * sizeof(uint32_t), st));
     batch_order_kernel<<<1, 1024, 0, st>>>(b.off, (int)S, b.order);
     FT_CUDA(cudaGetLastError());
@@ -759,7 +771,9 @@ void batch_tree_view(Context &ctx, BatchImpl &b, size_t s, ft_tree &out, cudaStr
     FT_CUDA(cudaMemcpyAsync(o, b.off + s, 2 * sizeof(long long), cudaMemcpyDeviceToHost, st));
     FT_CUDA(cudaMemcpyAsync(&no, b.node_off + s, sizeof(long long), cudaMemcpyDeviceToHost, st));
     FT_CUDA(cudaMemcpyAsync(&ro, b.rec_off + s, sizeof(long long), cudaMemcpyDeviceToHost, st));
+    uint32_t  fl = 0;
     FT_CUDA(cudaMemcpyAsync(&h, b.set_height + s, 1, cudaMemcpyDeviceToHost, st));
+    FT_CUDA(cudaMemcpyAsync(&fl, b.scr.qflag + s, sizeof(fl), cudaMemcpyDeviceToHost, st));
     FT_CUDA(cudaStreamSynchronize(st));
     if (b.views.size() < b.max_sets) b.views.resize(b.max_sets);
     if (!b.views[s]) b.views[s].reset(new TreeImpl());
@@ -772,7 +786,11 @@ void batch_tree_view(Context &ctx, BatchImpl &b, size_t s, ft_tree &out, cudaStr
     v.recs           = (unsigned char *)b.scr.recs + (size_t)ro * 16 * cb;
     v.height         = b.scr.height + ro;
     v.leafcount      = b.scr.leafcount + ro;
-    v.wide           = (unsigned char *)b.scr.wide + (size_t)ro * wide_bytes(ctx.opts.coord_type);
+    v.qrec           = (QRec *)b.scr.qrec + ro;
+    v.qpts           = (QPoint *)b.scr.qpts + o[0];
+    v.qflag          = b.scr.qflag + s;
+    v.framed         = fl == 0u;
+    v.plain_only     = (fl & kQFlagPlain) != 0u;
     v.height_root    = n >= 2 ? (int)h : 0;
     v.clean42        = false;
     std::memset(&out, 0, sizeof(out));

@@ -16,6 +16,7 @@
 #include "ft_build_dev.cuh"
 #include "ft_common.cuh"
 #include "ft_internal.h"
+#include "ft_qtree.cuh"
 
 namespace ft {
 
@@ -512,15 +513,23 @@ __global__ void __launch_bounds__(256) refit_stream_kernel(int n, const int32_t 
     }
 }
 
-// 4-wide records of every internal node (collapse_node), after the refit.
+// The fast walks' view of the tree (ft_qtree.cuh), after the refit: leaf j's position, and the
+// record of every internal node of more than kBucket leaves (and of the root), the only ones
+// a walk reaches.
 template <class T>
-__global__ void __launch_bounds__(256) collapse_kernel(int n, const int32_t *__restrict__ left,
-                                                       const int32_t *__restrict__ right, const T *mnx,
-                                                       const T *mxx, const T *mny, const T *mxy, const T *mnz,
-                                                       const T *mxz, WideRec<T> *wide) {
-    const T *const soa[6] = {mnx, mxx, mny, mxy, mnz, mxz};
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n - 1; v += gridDim.x * blockDim.x)
-        collapse_node<T>(v, n, left, right, soa, wide);
+__global__ void __launch_bounds__(256) qtree_kernel(int n, const NodeRec<T> *__restrict__ recs,
+                                                    const int32_t *__restrict__ leaves, const T *mnx, const T *mxx,
+                                                    const T *mny, const T *mxy, const T *mnz, const T *mxz,
+                                                    int periodic, QRec *qrec, QPoint *qpts, uint32_t *flag) {
+    const T   rb[6] = {mnx[0], mxx[0], mny[0], mxy[0], mnz[0], mxz[0]};
+    QFrame<T> f;
+    f.make(rb, n, periodic != 0);
+    if (!f.ok && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(flag, f.flag());
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const int s = j + n - 1;
+        qpts[j]     = qpoint<T>(mnx[s], mny[s], mnz[s], f, periodic != 0, flag);
+        if (j < n - 1 && (j == 0 || leaves[j] > kBucket)) qrec_node<T>(j, n, recs, leaves, f, qrec, flag);
+    }
 }
 
 // =========================================================================================
@@ -544,7 +553,7 @@ template <class T> static void *alloc_dev(size_t count) {
 }
 
 void free_scratch(TreeImpl &s) {
-    void *ptrs[] = {s.recs, s.height, s.counters, s.leafcount, s.wide, s.key_lo, s.key_hi, s.tmp_lo, s.tmp_hi,
+    void *ptrs[] = {s.recs, s.height, s.counters, s.leafcount, s.qrec, s.qpts, s.qflag, s.key_lo, s.key_hi, s.tmp_lo, s.tmp_hi,
                     s.perm, s.tmp_perm, s.bbox, s.bbox_partial, s.hist, s.lookback, s.tile_counter, s.status};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -571,7 +580,9 @@ void ensure_scratch(TreeImpl &s, const ft_options &o, size_t n) {
     s.height   = (uint8_t *)alloc_dev<uint8_t>(cap);
     s.counters = (int32_t *)alloc_dev<int32_t>(cap);
     s.leafcount = (int32_t *)alloc_dev<int32_t>(cap);
-    s.wide      = alloc_dev<unsigned char>((cap > 1 ? cap - 1 : 1) * wide_bytes(o.coord_type));
+    s.qrec      = alloc_dev<QRec>(cap > 1 ? cap - 1 : 1);
+    s.qpts      = alloc_dev<QPoint>(cap);
+    s.qflag     = (uint32_t *)alloc_dev<uint32_t>(1);
     s.key_lo   = (uint64_t *)alloc_dev<uint64_t>(cap);
     s.tmp_lo   = (uint64_t *)alloc_dev<uint64_t>(cap);
     if (W == 2) {
@@ -586,7 +597,7 @@ void ensure_scratch(TreeImpl &s, const ft_options &o, size_t n) {
     s.lookback_words = 16 * sort_tiles(cap, W) * 256;
     s.lookback     = (uint32_t *)alloc_dev<uint32_t>(s.lookback_words);
     s.tile_counter = (uint32_t *)alloc_dev<uint32_t>(kTicketWords);
-    s.status       = (uint32_t *)alloc_dev<uint32_t>(4);
+    s.status       = (uint32_t *)alloc_dev<uint32_t>(4 + sizeof(TreeSummary) / 4);
     FT_CUDA(cudaMemset(s.status, 0, 16));
 }
 
@@ -841,6 +852,16 @@ template <class T> struct SoA {
 };
 
 template <class T>
+static void build_qtree(const ft_options &o, ft_tree &t, TreeImpl &s, size_t n, cudaStream_t st) {
+    SoA<T> a(t);
+    FT_CUDA(cudaMemsetAsync(s.qflag, 0, sizeof(uint32_t), st));
+    qtree_kernel<T><<<grid_for(n, 256, 148 * 32), 256, 0, st>>>((int)n, (const NodeRec<T> *)s.recs, s.leafcount, a.mnx,
+                                                                a.mxx, a.mny, a.mxy, a.mnz, a.mxz, o.periodic,
+                                                                (QRec *)s.qrec, (QPoint *)s.qpts, s.qflag);
+    FT_CUDA(cudaGetLastError());
+}
+
+template <class T>
 static void topology_and_refit(const ft_options &o, ft_tree &t, TreeImpl &s, size_t n, cudaStream_t st,
                                Context *prof = nullptr) {
     if (n < 2) {
@@ -867,9 +888,8 @@ static void topology_and_refit(const ft_options &o, ft_tree &t, TreeImpl &s, siz
         (int)n, t.left_child, t.right_child, t.parent, a.mnx, a.mxx, a.mny, a.mxy, a.mnz, a.mxz,
         (NodeRec<T> *)s.recs, s.height, s.counters, s.leafcount, s.counters + (n - 1));
     stage_mark(prof, BS_REFIT, st);
-    collapse_kernel<T><<<blocks, 256, 0, st>>>((int)n, t.left_child, t.right_child, a.mnx, a.mxx, a.mny, a.mxy,
-                                               a.mnz, a.mxz, (WideRec<T> *)s.wide);
     FT_CUDA(cudaGetLastError());
+    build_qtree<T>(o, t, s, n, st);
     stage_mark(prof, BS_RECORDS, st);
 }
 
@@ -966,7 +986,7 @@ static void build_tree_typed(Context &ctx, ft_tree &t, const void *keys_ref, con
 // result is the tree build_tree (src/hlbvh.hpp:773-982) makes from the same sorted keys with
 // the new positions as its leaf arrays.
 template <class T>
-static void refit_typed(ft_tree &t, const void *x, const void *y, const void *z, size_t n, bool leaf_order,
+static void refit_typed(const ft_options &o, ft_tree &t, const void *x, const void *y, const void *z, size_t n, bool leaf_order,
                         cudaStream_t st) {
     TreeImpl &s = *(TreeImpl *)t.impl;
     SoA<T>    a(t);
@@ -975,23 +995,21 @@ static void refit_typed(ft_tree &t, const void *x, const void *y, const void *z,
                                                              a.mny, a.mxy, a.mnz, a.mxz, s.status);
     FT_CUDA(cudaGetLastError());
     if (n < 2) return;
-    const int blocks = grid_for(n, 256, 148 * 32);
     FT_CUDA(cudaMemsetAsync(s.counters, 0, n * sizeof(int32_t), st));
     refit_stream_kernel<T><<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(
         (int)n, t.left_child, t.right_child, t.parent, a.mnx, a.mxx, a.mny, a.mxy, a.mnz, a.mxz,
         (NodeRec<T> *)s.recs, s.height, s.counters, s.leafcount, s.counters + (n - 1));
-    collapse_kernel<T><<<blocks, 256, 0, st>>>((int)n, t.left_child, t.right_child, a.mnx, a.mxx, a.mny, a.mxy,
-                                               a.mnz, a.mxz, (WideRec<T> *)s.wide);
     FT_CUDA(cudaGetLastError());
+    build_qtree<T>(o, t, s, n, st);
 }
 
 void refit_bvh(Context &ctx, ft_tree &t, const void *x, const void *y, const void *z, size_t n, bool leaf_order,
                cudaStream_t st) {
     switch (ctx.opts.coord_type) {
-    case F32: refit_typed<float>(t, x, y, z, n, leaf_order, st); break;
-    case F64: refit_typed<double>(t, x, y, z, n, leaf_order, st); break;
-    case U32: refit_typed<uint32_t>(t, x, y, z, n, leaf_order, st); break;
-    case U64: refit_typed<unsigned long long>(t, x, y, z, n, leaf_order, st); break;
+    case F32: refit_typed<float>(ctx.opts, t, x, y, z, n, leaf_order, st); break;
+    case F64: refit_typed<double>(ctx.opts, t, x, y, z, n, leaf_order, st); break;
+    case U32: refit_typed<uint32_t>(ctx.opts, t, x, y, z, n, leaf_order, st); break;
+    case U64: refit_typed<unsigned long long>(ctx.opts, t, x, y, z, n, leaf_order, st); break;
     }
 }
 
@@ -1006,6 +1024,39 @@ void recompute_from_keys(Context &ctx, ft_tree &t, cudaStream_t st) {
     case U32: topology_and_refit<uint32_t>(ctx.opts, t, s, n, st); break;
     case U64: topology_and_refit<unsigned long long>(ctx.opts, t, s, n, st); break;
     }
+}
+
+template <class T>
+__global__ void tree_summary_kernel(int n, const T *mxx, const T *mxy, const T *mxz, const uint8_t *height,
+                                    const uint32_t *status, const uint32_t *qflag, TreeSummary *out) {
+    TreeSummary m;
+    m.mx[0]  = Coord<T>::is_float ? 0ull : (unsigned long long)mxx[0];
+    m.mx[1]  = Coord<T>::is_float ? 0ull : (unsigned long long)mxy[0];
+    m.mx[2]  = Coord<T>::is_float ? 0ull : (unsigned long long)mxz[0];
+    m.status = *status;
+    m.height = n > 1 ? height[0] : 0u;
+    m.qflag  = n > 1 ? *qflag : 0u;
+    m.pad    = 0u;
+    *out     = m;
+}
+
+void tree_summary(const ft_options &o, const ft_tree &t, TreeSummary &out, cudaStream_t st) {
+    const TreeImpl &s   = *(const TreeImpl *)t.impl;
+    TreeSummary    *dev = reinterpret_cast<TreeSummary *>(s.status + 4);
+    auto            run = [&](auto *p) {
+        using T = std::remove_pointer_t<decltype(p)>;
+        tree_summary_kernel<T><<<1, 1, 0, st>>>((int)t.num_leaves, (const T *)t.max_x, (const T *)t.max_y,
+                                                (const T *)t.max_z, s.height, s.status, s.qflag, dev);
+    };
+    switch (o.coord_type) {
+    case F32: run((float *)nullptr); break;
+    case F64: run((double *)nullptr); break;
+    case U32: run((uint32_t *)nullptr); break;
+    case U64: run((unsigned long long *)nullptr); break;
+    }
+    FT_CUDA(cudaGetLastError());
+    FT_CUDA(cudaMemcpyAsync(&out, dev, sizeof(out), cudaMemcpyDeviceToHost, st));
+    FT_CUDA(cudaStreamSynchronize(st));
 }
 
 void build_tree_from_keys(Context &ctx, ft_tree &t, const void *keys_ref, const void *sx, const void *sy,

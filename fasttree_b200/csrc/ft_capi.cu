@@ -10,6 +10,7 @@
 
 #include "ft_common.cuh"
 #include "ft_internal.h"
+#include "ft_qtree.cuh"
 
 namespace ft {
 
@@ -440,7 +441,22 @@ ft_status ft_sfc_encode(ft_context *ctx, const void *x, const void *y, const voi
     FT_API_END
 }
 
-static bool root_in_period(const ft_context *ctx, const ft_tree *tree, cudaStream_t st);
+// What the host keeps of a finished build: one small launch, one copy, one wait.  Throws what
+// the kernels recorded; sets the height, the frame and whether every coordinate of an integer
+// tree lies below the period 2^42 (64-bit) / 2^21 (32-bit), i.e. the root box maxima do.
+static void finish_build(const ft_context *ctx, ft_tree *tree, cudaStream_t st) {
+    TreeImpl    &impl = *(TreeImpl *)tree->impl;
+    TreeSummary  m;
+    tree_summary(ctx->opts, *tree, m, st);
+    if (m.status) check_device_status(impl.status, st);
+    const int      ct = ctx->opts.coord_type;
+    const uint64_t P  = ct == FT_COORD_U64 ? 1ull << 42 : 1ull << 21;
+    impl.height_root  = (int)m.height;
+    impl.framed       = m.qflag == 0u;
+    impl.plain_only   = (m.qflag & kQFlagPlain) != 0u;
+    impl.in_period    = ct == FT_COORD_F32 || ct == FT_COORD_F64 || (m.mx[0] < P && m.mx[1] < P && m.mx[2] < P);
+    impl.clean42      = impl.clean42_ok && ct == FT_COORD_U64 && impl.in_period;
+}
 
 // ---------------------------------------------------------------------------------------
 // Tree serialisation (raw SoA arrays + sorted keys behind a fixed header)
@@ -569,38 +585,17 @@ ft_status ft_tree_import(ft_context *ctx, const void *buf, size_t bytes, ft_tree
         FT_CUDA(cudaMemcpyAsync(impl.bbox, box, 6 * cb, cudaMemcpyHostToDevice, st));
         recompute_from_keys(*ctx, *tree, st);
     }
-    if (n > 1) {
-        uint8_t hr = 0;
-        FT_CUDA(cudaMemcpyAsync(&hr, impl.height, 1, cudaMemcpyDeviceToHost, st));
-        check_status_word(impl, st);
-        impl.height_root = hr;
+    impl.clean42_ok = h.clean42_ok != 0;
+    if (n) {
+        finish_build(ctx, tree, st);
     } else {
         FT_CUDA(cudaStreamSynchronize(st));
         impl.height_root = 0;
+        impl.in_period   = true;
+        impl.clean42     = impl.clean42_ok && ctx->opts.coord_type == FT_COORD_U64;
     }
-    impl.own_keys   = h.own_keys != 0;
-    impl.clean42_ok = h.clean42_ok != 0;
-    impl.in_period = root_in_period(ctx, tree, st);
-    impl.clean42   = impl.clean42_ok && ctx->opts.coord_type == FT_COORD_U64 && impl.in_period;
+    impl.own_keys = h.own_keys != 0;
     FT_API_END
-}
-
-// Root box maxima of an integer tree below the period 2^42 (64-bit) / 2^21 (32-bit), i.e.
-// every coordinate is (TreeImpl::in_period).  Blocking.
-static bool root_in_period(const ft_context *ctx, const ft_tree *tree, cudaStream_t st) {
-    const int ct = ctx->opts.coord_type;
-    if (ct == FT_COORD_F32 || ct == FT_COORD_F64 || tree->num_leaves == 0) return true;
-    const void *src[3] = {tree->max_x, tree->max_y, tree->max_z};
-    if (ct == FT_COORD_U64) {
-        uint64_t m[3] = {0, 0, 0};
-        for (int a = 0; a < 3; ++a) FT_CUDA(cudaMemcpyAsync(&m[a], src[a], 8, cudaMemcpyDefault, st));
-        FT_CUDA(cudaStreamSynchronize(st));
-        return m[0] < (1ull << 42) && m[1] < (1ull << 42) && m[2] < (1ull << 42);
-    }
-    uint32_t m[3] = {0, 0, 0};
-    for (int a = 0; a < 3; ++a) FT_CUDA(cudaMemcpyAsync(&m[a], src[a], 4, cudaMemcpyDefault, st));
-    FT_CUDA(cudaStreamSynchronize(st));
-    return m[0] < (1u << 21) && m[1] < (1u << 21) && m[2] < (1u << 21);
 }
 
 ft_status ft_refit_bvh(ft_context *ctx, const void *x, const void *y, const void *z, size_t n, int leaf_order,
@@ -621,17 +616,7 @@ ft_status ft_refit_bvh(ft_context *ctx, const void *x, const void *y, const void
     sy.init(y, n * cb, true, false, st);
     sz.init(z, n * cb, true, false, st);
     ft::refit_bvh(*ctx, *tree, sx.dev, sy.dev, sz.dev, n, leaf_order != 0, st);
-    // the 42-bit periodic fast form needs every coordinate below 2^42: the root box's maxima
-    uint64_t mx[3] = {0, 0, 0};
-    if (ctx->opts.coord_type == FT_COORD_U64) {
-        FT_CUDA(cudaMemcpyAsync(&mx[0], tree->max_x, 8, cudaMemcpyDefault, st));
-        FT_CUDA(cudaMemcpyAsync(&mx[1], tree->max_y, 8, cudaMemcpyDefault, st));
-        FT_CUDA(cudaMemcpyAsync(&mx[2], tree->max_z, 8, cudaMemcpyDefault, st));
-    }
-    check_status_word(impl, st);
-    impl.clean42 = impl.clean42_ok && ctx->opts.coord_type == FT_COORD_U64 && mx[0] < (1ull << 42) &&
-                   mx[1] < (1ull << 42) && mx[2] < (1ull << 42);
-    impl.in_period = root_in_period(ctx, tree, st);
+    finish_build(ctx, tree, st);
     FT_API_END
 }
 
@@ -665,23 +650,8 @@ ft_status ft_build_bvh(ft_context *ctx, const void *x, const void *y, const void
                   sk.dev, st);
     impl.own_keys = keys == nullptr; // the sorted keys are this library's encoding of bbox
     if (keys) sk.copy_back();
-    uint64_t box[6] = {0, 0, 0, 0, 0, 0};
-    if (ctx->opts.coord_type == FT_COORD_U64)
-        FT_CUDA(cudaMemcpyAsync(box, impl.bbox, sizeof(box), cudaMemcpyDeviceToHost, st));
-    if (n > 1) {
-        uint8_t h = 0;
-        FT_CUDA(cudaMemcpyAsync(&h, impl.height, 1, cudaMemcpyDeviceToHost, st));
-        check_status_word(impl, st);
-        impl.height_root = h;
-    } else {
-        check_status_word(impl, st);
-        impl.height_root = 0;
-    }
-    // boxes of a 42-bit tree stay below 2^42 when every coordinate does (max entries 1, 3, 5)
-    impl.clean42 = ctx->opts.coord_type == FT_COORD_U64 && box[1] < (1ull << 42) && box[3] < (1ull << 42) &&
-                   box[5] < (1ull << 42);
     impl.clean42_ok = true;
-    impl.in_period  = root_in_period(ctx, tree, st);
+    finish_build(ctx, tree, st);
     FT_API_END
 }
 
@@ -715,16 +685,7 @@ ft_status ft_build_tree(ft_context *ctx, ft_tree *tree, const void *sorted_keys,
     impl.height_root   = -1;
     build_tree_from_keys(*ctx, *tree, sk.dev, sx.dev, sy.dev, sz.dev, (const uint32_t *)sid.dev,
                          (const int8_t *)sgh.dev, (const int32_t *)sor.dev, st);
-    if (n > 1) {
-        uint8_t h = 0;
-        FT_CUDA(cudaMemcpyAsync(&h, impl.height, 1, cudaMemcpyDeviceToHost, st));
-        check_status_word(impl, st);
-        impl.height_root = h;
-    } else {
-        check_status_word(impl, st);
-        impl.height_root = 0;
-    }
-    impl.in_period = root_in_period(ctx, tree, st);
+    finish_build(ctx, tree, st);
     FT_API_END
 }
 

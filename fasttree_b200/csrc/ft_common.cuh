@@ -161,6 +161,30 @@ template <class T> struct Metric {
             return sq(ax) + sq(ay) + sq(az);
         }
     }
+
+    // dist() for a leaf's box (min == max), the same value with fewer operations.  Floating
+    // point: one of the two gaps is |x - p|, the other its negative, and c_fmax with 0 turns a
+    // NaN into 0.  Clean 42-bit periodic positions: |sext(x - v)| >> dist_shift, taken from the
+    // high word of the difference shifted to the top.
+    static FT_D unsigned long long point_axis_clean(T v, T x) {
+        static_assert(sizeof(T) == 8, "42-bit positions only");
+        const unsigned long long y = ((unsigned long long)x - (unsigned long long)v) << C::shift_bits;
+        const uint32_t           h = (uint32_t)(y >> 32);
+        const uint32_t           g = (int32_t)h < 0 ? ~h + ((uint32_t)y == 0u ? 1u : 0u) : h; // |y| >> 32
+        return (unsigned long long)(g >> (C::shift_bits + C::dist_shift - 32));
+    }
+    template <bool PERIODIC, bool CLEAN = false>
+    static FT_D dist_t point(T px, T py, T pz, T x, T y, T z) {
+        if constexpr (C::is_float) {
+            const T dx = fmax(fabs(sub_rn(x, px)), T(0)), dy = fmax(fabs(sub_rn(y, py)), T(0)),
+                    dz = fmax(fabs(sub_rn(z, pz)), T(0));
+            return (double)add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
+        } else if constexpr (PERIODIC && CLEAN && sizeof(T) == 8) {
+            return sq(point_axis_clean(px, x)) + sq(point_axis_clean(py, y)) + sq(point_axis_clean(pz, z));
+        } else {
+            return dist<PERIODIC, CLEAN>(px, py, pz, x, x, y, y, z, z);
+        }
+    }
 };
 
 // ---------------------------------------------------------------------------------------
@@ -188,15 +212,6 @@ FT_HD uint32_t info_height(uint32_t w) { return w >> 25; }
 static_assert(sizeof(NodeRec<float>) == 64, "record size");
 static_assert(sizeof(NodeRec<double>) == 128, "record size");
 
-// 4-wide record of an internal node for the fast walk: the node's grandchildren (a child
-// that is a leaf stands for itself), up to four boxes and their node indices (-1: absent).
-template <class T> struct alignas(16) WideRec {
-    T       box[4][6];
-    int32_t child[4];
-};
-static_assert(sizeof(WideRec<float>) == 112, "wide record size");
-static_assert(sizeof(WideRec<double>) == 208, "wide record size");
-
 // Record loads: through the read-only path by default.  COH: an ordinary (weak, L1-cached)
 // global load instead, for kernels that read records other blocks wrote earlier in the same
 // launch -- the read-only path is only valid for data that stays unchanged while the kernel
@@ -210,22 +225,6 @@ template <bool COH> FT_D uint4 ld_rec16(const uint4 *p) {
     } else {
         return __ldg(p);
     }
-}
-
-template <class T, bool COH = false> FT_D void load_wide(const WideRec<T> *w, int node, T b[4][6], int c[4]) {
-    constexpr int NW = (int)(sizeof(WideRec<T>) / 16);
-    const uint4  *p  = reinterpret_cast<const uint4 *>(w + node);
-    uint4         v[NW];
-#pragma unroll
-    for (int i = 0; i < NW; ++i) v[i] = ld_rec16<COH>(p + i);
-    const T *f = reinterpret_cast<const T *>(v);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int d = 0; d < 6; ++d) b[i][d] = f[6 * i + d];
-    const int32_t *ci = reinterpret_cast<const int32_t *>(f + 24);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) c[i] = ci[i];
 }
 
 // load_rec plus the two children's info words (rec_child_info).
@@ -310,6 +309,20 @@ template <class T, class F> inline void met_dispatch(int met, F &&f) {
     }
 }
 
+// The fast walks' node and leaf formats, in 32-bit units of the tree's frame (ft_qtree.cuh).
+struct alignas(16) QPoint {
+    int32_t x, y, z, w;
+};
+// 4-wide node: child i's box centre and half extent (margin included) in words 6i .. 6i + 5,
+// then the children's references (a node, a bucket of leaves or absent) and leaf counts.
+// Children are in leaf order.
+struct alignas(128) QRec {
+    int32_t  c[4][6];
+    uint32_t ref[4];
+    uint32_t cnt[4];
+};
+static_assert(sizeof(QRec) == 128, "one line per record");
+
 // Device view of a built tree.
 template <class T> struct TreeDev {
     const T *min_x, *max_x, *min_y, *max_y, *min_z, *max_z;
@@ -317,7 +330,9 @@ template <class T> struct TreeDev {
     const NodeRec<T> *recs;
     const uint8_t    *height; // subtree height of each internal node
     const int32_t    *leaves; // leaf count of each internal node
-    const WideRec<T> *wide;   // 4-wide record of each internal node
+    const QRec       *qrec;   // fast walks: 4-wide records in the 32-bit frame (ft_qtree.cuh)
+    const QPoint     *qpts;   // fast walks: leaf positions in that frame
+    const uint32_t   *qflag;  // not 0: the frame does not serve this tree
     int               n;      // leaves
 };
 
@@ -334,7 +349,9 @@ template <class T> inline TreeDev<T> tree_view(const ft_tree &tr) {
     v.recs     = (const NodeRec<T> *)((TreeImpl *)tr.impl)->recs;
     v.height   = ((TreeImpl *)tr.impl)->height;
     v.leaves   = ((TreeImpl *)tr.impl)->leafcount;
-    v.wide     = (const WideRec<T> *)((TreeImpl *)tr.impl)->wide;
+    v.qrec     = (const QRec *)((TreeImpl *)tr.impl)->qrec;
+    v.qpts     = (const QPoint *)((TreeImpl *)tr.impl)->qpts;
+    v.qflag    = ((TreeImpl *)tr.impl)->qflag;
     v.n        = (int)tr.num_leaves;
     return v;
 }
@@ -366,7 +383,9 @@ template <class T> FT_D TreeDev<T> set_view(const TreeDev<T> &all, const BatchDe
     t.recs     = all.recs + rb;
     t.height   = all.height + rb;
     t.leaves   = all.leaves + rb;
-    t.wide     = all.wide + rb;
+    t.qrec     = all.qrec + rb;
+    t.qpts     = all.qpts + b.off[s];
+    t.qflag    = all.qflag + s;
     t.n        = (int)(b.off[s + 1] - b.off[s]);
     return t;
 }

@@ -14,6 +14,7 @@
 
 #include "ft_build_dev.cuh"
 #include "ft_common.cuh"
+#include "ft_qtree.cuh"
 
 namespace ft {
 
@@ -56,9 +57,12 @@ template <class T> struct CtaTreeOut {
     int8_t     *ghost;
     int32_t    *orig;
     NodeRec<T> *recs;
-    WideRec<T> *wide;
     uint8_t    *height;
     int32_t    *counters, *leaves;
+    QRec       *qrec;  // the fast walks' records and leaf positions, and the set's flag word
+    QPoint     *qpts;
+    uint32_t   *qflag; // (zero at launch)
+    int         periodic;
 };
 
 // Exclusive prefix sums of a[0..256) in place, by the block's first warp (8 entries a lane).
@@ -425,7 +429,13 @@ FT_D void cta_build_set(int n, const T *__restrict__ x, const T *__restrict__ y,
     }
     if (tid == 0) o.parent[0] = -1;
     if (n < 2) {
-        if (tid == 0) *set_height = 0;
+        if (tid == 0) {
+            QFrame<T> f;
+            const T   rb[6] = {x[0], x[0], y[0], y[0], z[0], z[0]};
+            f.make(rb, n, o.periodic != 0);
+            o.qpts[0]   = qpoint<T>(x[0], y[0], z[0], f, o.periodic != 0, o.qflag); // (a query reads it)
+            *set_height = 0;
+        }
         __syncthreads();
         return;
     }
@@ -439,30 +449,18 @@ FT_D void cta_build_set(int n, const T *__restrict__ x, const T *__restrict__ y,
     __syncthreads();
     for (int j = tid; j < n; j += PT) climb_build<T>(j, n, delta, o.counters, o);
     __syncthreads();
-    T *const soa[6] = {o.mnx, o.mxx, o.mny, o.mxy, o.mnz, o.mxz};
-    // 7. 4-wide records (boxes read through L2, where the refit wrote them)
-    for (int v = tid; v < n - 1; v += PT) {
-        int       ch[4] = {-1, -1, -1, -1};
-        int       c     = 0;
-        const int l = o.left[v], r = o.right[v];
-        if (l >= n - 1) ch[c++] = l;
-        else {
-            ch[c++] = o.left[l];
-            ch[c++] = o.right[l];
+    // 7. the fast walks' records and leaf positions
+    {
+        const T   rb[6] = {__ldcg(o.mnx), __ldcg(o.mxx), __ldcg(o.mny), __ldcg(o.mxy), __ldcg(o.mnz), __ldcg(o.mxz)};
+        QFrame<T> f;
+        f.make(rb, n, o.periodic != 0);
+        if (!f.ok && tid == 0) atomicOr(o.qflag, f.flag());
+        for (int j = tid; j < n; j += PT) {
+            const int slot = n - 1 + j;
+            o.qpts[j]      = qpoint<T>(o.mnx[slot], o.mny[slot], o.mnz[slot], f, o.periodic != 0, o.qflag);
+            if (j < n - 1 && (j == 0 || o.leaves[j] > kBucket))
+                qrec_node<T>(j, n, o.recs, o.leaves, f, o.qrec, o.qflag);
         }
-        if (r >= n - 1) ch[c++] = r;
-        else {
-            ch[c++] = o.left[r];
-            ch[c++] = o.right[r];
-        }
-        WideRec<T> w;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-#pragma unroll
-            for (int d = 0; d < 6; ++d) w.box[i][d] = ch[i] >= 0 ? __ldcg(soa[d] + ch[i]) : T(0);
-            w.child[i] = ch[i];
-        }
-        o.wide[v] = w;
     }
     if (tid == 0) *set_height = __ldcg(o.height);
     __syncthreads();

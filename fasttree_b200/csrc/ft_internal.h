@@ -35,7 +35,9 @@ struct TreeImpl {
     uint8_t  *height       = nullptr; // subtree height of internal nodes
     int32_t  *counters     = nullptr; // refit arrival counters
     int32_t  *leafcount    = nullptr; // leaves under each internal node (Karras range size)
-    void     *wide         = nullptr; // WideRec<T>[cap-1]: grandchildren of each internal node
+    void     *qrec         = nullptr; // QRec[cap-1]: the fast walks' records (ft_qtree.cuh)
+    void     *qpts         = nullptr; // QPoint[cap]: leaf positions in the walks' frame
+    uint32_t *qflag        = nullptr; // device word, not 0: the frame does not serve the tree
     uint64_t *key_lo       = nullptr; // sorted keys (low word)
     uint64_t *key_hi       = nullptr; // sorted keys (high word, 126-bit keys only)
     uint64_t *tmp_lo       = nullptr; // sort ping-pong
@@ -48,7 +50,7 @@ struct TreeImpl {
     uint32_t *lookback     = nullptr; // onesweep tile status
     size_t    lookback_words = 0;
     uint32_t *tile_counter = nullptr; // per-pass tile ticket
-    uint32_t *status       = nullptr; // device status word
+    uint32_t *status       = nullptr; // device status word, then (from word 4) a TreeSummary
     bool      managed      = false;
     int       height_root  = -1;    // host copy after a build
     bool      clean42      = false; // 64-bit integer tree with every coordinate below 2^42
@@ -56,6 +58,8 @@ struct TreeImpl {
     bool      in_period    = true;  // integer coordinates all below 2^bits (42 for 64-bit, 21
                                     // for 32-bit): the periodic distance is then monotone over
                                     // nested boxes, which the fast walks rely on
+    bool      framed       = false; // the 32-bit frame serves the tree (qflag was 0 after the build)
+    bool      plain_only   = false; // box distances are not monotone (kQFlagPlain)
     bool      view         = false; // one set of a batch: arrays owned by the batch, no builds
     bool      own_keys     = false; // key_lo / key_hi hold keys this library encoded (build_bvh
                                     // without caller keys), with the box in bbox
@@ -79,6 +83,7 @@ struct BatchDev {
 // integer one on coordinates at or above the period (2^42 / 2^21), whose unmasked box bounds
 // break it; such trees keep the reference traversal.
 inline bool fast_walk_applies(const ft_options &o, const TreeImpl &t) {
+    if (t.plain_only) return false; // a coordinate that is not finite, or squares beyond 64 bits
     return !o.periodic || o.coord_type == FT_COORD_F32 || o.coord_type == FT_COORD_F64 || t.in_period;
 }
 
@@ -215,6 +220,13 @@ void free_query_sort(Context &ctx);
 // this library's own encoding.  Valid until the next call on the context.
 const uint32_t *sfc_query_order(Context &ctx, const ft_tree &tree, const void *qx, const void *qy, const void *qz,
                                 size_t nq, cudaStream_t st);
+// A finished build in one read: root box maxima (integer coordinates), the status word, the
+// root's height and the frame's flag (ft_build.cu).  Waits for the stream.
+struct TreeSummary {
+    uint64_t mx[3];
+    uint32_t status, height, qflag, pad;
+};
+void tree_summary(const ft_options &o, const ft_tree &tree, TreeSummary &out, cudaStream_t st);
 void recompute_from_keys(Context &ctx, ft_tree &tree, cudaStream_t st);
 void refit_bvh(Context &ctx, ft_tree &tree, const void *x, const void *y, const void *z, size_t n, bool leaf_order,
                cudaStream_t st);
@@ -288,7 +300,6 @@ void range(Context &ctx, const ft_tree &tree, const void *qx, const void *qy, co
            int max_per_q, cudaStream_t st);
 
 size_t coord_bytes(int coord);
-inline size_t wide_bytes(int coord) { return coord_bytes(coord) == 8 ? 208 : 112; } // sizeof(WideRec<T>)
 
 // ---- batched sets (ft_batch.cu) ----
 struct BatchImpl;

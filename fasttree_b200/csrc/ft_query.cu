@@ -19,6 +19,7 @@
 
 #include "ft_common.cuh"
 #include "ft_internal.h"
+#include "ft_qtree.cuh"
 
 namespace ft {
 
@@ -641,90 +642,189 @@ FT_D int range_one(const TreeDev<T> &t, T px, T py, T pz, typename Coord<T>::dis
     return count;
 }
 
-// One query's range walk over the 4-wide records (trees of height <= 62 whose box distance
-// is monotone over nested boxes): each expansion judges up to four grandchildren at once,
-// and they are stacked rightmost first, so the walk stays depth-first and left-first and
-// writes the row in the reference's order.  Skipping the binary level between is exact here:
-// a grandchild beyond r_max has a parent beyond it too, and the reference prunes there.  Once
-// the row is full, a leaf is counted at once and an internal grandchild inside the shell is
-// counted from its leaf count.
-// STOP: return as soon as the row is full (*filled set), leaving the count to range_count_group.
-template <class T, int PER, bool STOP = false>
-FT_D int range_one_wide(const TreeDev<T> &t, T px, T py, T pz, typename Coord<T>::dist_t rm2,
-                        typename Coord<T>::dist_t RM2, int32_t *__restrict__ results, size_t off, int max_per,
-                        int ret_orig, uint32_t *status, bool *filled = nullptr) {
-    using D     = typename Coord<T>::dist_t;
-    const int n = t.n;
-    int       count = 0;
-    int       sn[kStack * 2];
-    int       sp = 0;
-    const D   d0 = node_dist_soa<T, PER>(t, 0, px, py, pz);
-    if (d0 <= RM2 && (n > 1 || d0 >= rm2)) {
-        sn[0] = 0;
-        sp    = 1;
+// -----------------------------------------------------------------------------------------
+// range_query over the fast walks' records (QRec / QPoint, ft_qtree.cuh), on trees of height
+// <= 62 whose box distance is monotone over nested boxes and that the 32-bit frame serves.
+// There the reference's rows are the leaves of the query's shell (rmin^2 <= d <= rmax^2 by
+// each leaf's own distance) in leaf order, and its count their number, so any pruning by a
+// lower bound of the distance gives the same rows.
+// -----------------------------------------------------------------------------------------
+// A query's limits on the frame's squared bounds: a box whose bound exceeds `out` holds no leaf
+// within r_max; one whose upper bound is at most `in` only leaves within r_max; one whose lower
+// bound is at least `ge` only leaves at or beyond r_min; one whose upper bound is below `lt`
+// only leaves nearer than r_min.  (QFrame::limit rounds up by 2^-17, covering the rounding of
+// bounds and distances; `in` and `lt` are rounded down by 2^-16 at least.)
+struct RangeLimits {
+    float out, in, ge, lt;
+};
+template <class T, class D> FT_D RangeLimits range_limits(const QFrame<T> &f, D rm2, D RM2) {
+    auto up = [](D d) {
+        if constexpr (std::is_floating_point<D>::value) return __double2float_ru(d);
+        else return __ull2float_ru(d);
+    };
+    auto down = [](D d) {
+        if constexpr (std::is_floating_point<D>::value) return __double2float_rd(d);
+        else return __ull2float_rd(d);
+    };
+    RangeLimits l;
+    l.out = f.limit(up(RM2));
+    l.in  = down(RM2) * f.k2 * (1.0f - 0x1p-15f) - f.slack;
+    l.ge  = rm2 > D(0) ? f.limit(up(rm2)) : 0.0f;
+    l.lt  = down(rm2) * f.k2 * (1.0f - 0x1p-15f) - f.slack;
+    return l;
+}
+
+// The point test of one leaf: exactly node_distance_sq's distance against the shell.  From the
+// QPoint where it holds the whole position; else the frame's bound first.
+template <class T, int PER> struct RangePoint {
+    using D = typename Coord<T>::dist_t;
+    T           px, py, pz;
+    int32_t     u[3];
+    uint32_t    ul[3], m;
+    D           rm2, RM2;
+    float       out;
+    const T    *lx, *ly, *lz; // leaf coordinates by rank
+    FT_D bool operator()(const uint4 &v, int leaf) const {
+        D d;
+        if constexpr (std::is_same<T, float>::value) {
+            d = Metric<T>::template point<false>(px, py, pz, __uint_as_float(v.x), __uint_as_float(v.y),
+                                                 __uint_as_float(v.z));
+        } else if constexpr (qpoint_whole<T, PER>()) {
+            d = qexact42(v, u, ul);
+        } else {
+            if (qdist(u, (int32_t)v.x, (int32_t)v.y, (int32_t)v.z, m, m, m) > out) return false;
+            d = Metric<T>::template point<(PER != 0), (PER == 2)>(px, py, pz, lx[leaf], ly[leaf], lz[leaf]);
+        }
+        return d >= rm2 && d <= RM2;
     }
+};
+
+// Upper bound of the squared distance, in units^2, between the query and any point of a box.
+FT_D float qfar(const int32_t u[3], const uint32_t w[6]) {
+    float f[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        f[a] = (float)(uint32_t)abs((int32_t)((uint32_t)u[a] - w[a])) + (float)w[3 + a];
+    return fmaf(f[2], f[2], fmaf(f[1], f[1], f[0] * f[0])) * (1.0f + 0x1p-20f);
+}
+
+// The rows of a warp's queries (every lane calls it; lanes without `go` idle): each lane walks
+// its own ball, leftmost child first, so it meets its leaves in leaf order.  Lanes whose next
+// node is an internal one expand together and lanes whose next is a bucket test it together.
+// STOP: a lane ends as soon as its row is full (*filled), leaving the count to
+// range_count_group; otherwise it counts on, subtrees inside the shell whole.
+template <class T, int PER, bool STOP>
+FT_D int range_rows(const TreeDev<T> &t, bool go, const RangePoint<T, PER> &pt, const RangeLimits &lim,
+                    int32_t *__restrict__ results, size_t off, int max_per, int ret_orig, uint32_t *status,
+                    bool *filled = nullptr) {
+    constexpr int  kRows = 100; // right siblings of a path: at most 1.5 per level of a tree of height <= 62
+    const unsigned FULL  = 0xffffffffu;
+    const int      n     = t.n;
+    uint32_t       st[kRows];
+    uint32_t       cur = 0;
+    int            sp = 0, count = 0;
+    bool           have = go;
     if constexpr (STOP) {
         *filled = false;
-        if (max_per <= 0) {
-            *filled = sp > 0;
-            return 0;
+        if (max_per <= 0 && have) { // no row: only the count is wanted
+            *filled = true;
+            have    = false;
         }
     }
-    long long budget = 2ll * n + 64;
-    while (sp > 0) {
-        if (--budget < 0) {
-            atomicOr(status, STATUS_TRAVERSAL_LIMIT);
-            break;
-        }
-        const int node = sn[--sp];
-        if (node >= n - 1) { // leaf in the shell (the n == 1 root included)
-            if (count < max_per) results[off + count] = ret_orig ? t.orig_idx[node] : node - (n - 1);
-            ++count;
+    const uint4 *pts    = reinterpret_cast<const uint4 *>(t.qpts);
+    long long    budget = 2ll * n + 64;
+    for (;;) {
+        const bool     inner = have && !(cur & kQBucket);
+        const unsigned mi    = __ballot_sync(FULL, inner);
+        const unsigned mb    = __ballot_sync(FULL, have && !inner);
+        if (!(mi | mb)) break;
+        bool pop = false;
+        if (mb == 0u || 2 * __popc(mi) >= __popc(mb)) {
+            if (inner) {
+                const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + cur);
+                uint4        v[8];
+#pragma unroll
+                for (int i = 0; i < (STOP ? 7 : 8); ++i) v[i] = __ldg(p + i);
+                const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
+                if (--budget < 0 || sp + 3 > kRows) {
+                    atomicOr(status, STATUS_TRAVERSAL_LIMIT);
+                    have = false;
+                } else {
+                    pop = true;
+#pragma unroll
+                    for (int i = 3; i >= 0; --i) {
+                        const uint32_t r = w[24 + i];
+                        const float    d = qdist(pt.u, (int32_t)w[6 * i], (int32_t)w[6 * i + 1], (int32_t)w[6 * i + 2],
+                                                 w[6 * i + 3], w[6 * i + 4], w[6 * i + 5]);
+                        bool           in = r != kQEmpty && !(d > lim.out);
+                        if constexpr (!STOP) {
+                            if (in && count >= max_per && d >= lim.ge && qfar(pt.u, w + 6 * i) <= lim.in) {
+                                count += (int)w[28 + i]; // every leaf below lies in the shell
+                                in = false;
+                            }
+                        }
+                        if (in) { // the leftmost so far is next, the one it displaces is stacked
+                            if (!pop) st[sp++] = cur;
+                            cur = r;
+                            pop = false;
+                        }
+                    }
+                }
+            }
+        } else if (have && !inner) {
+            const int first = qref_first(cur), cnt = qref_count(cur);
+            unsigned  near  = 0;
+#pragma unroll
+            for (int j = 0; j < kBucket; ++j) {
+                const uint4 v = __ldg(pts + first + min(j, cnt - 1));
+                if (j < cnt && pt(v, first + j)) near |= 1u << j;
+            }
+            while (near) {
+                const int j = __ffs(near) - 1;
+                near &= near - 1;
+                if (count < max_per) results[off + count] = ret_orig ? t.orig_idx[first + j + n - 1] : first + j;
+                ++count;
+                if constexpr (STOP) {
+                    if (count >= max_per) near = 0;
+                }
+            }
+            pop = true;
             if constexpr (STOP) {
                 if (count >= max_per) {
                     *filled = true;
-                    break;
+                    have    = false;
                 }
             }
-            continue;
         }
-        T   bx[4][6];
-        int ch[4];
-        load_wide(t.wide, node, bx, ch);
-        D d[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) d[i] = ch[i] >= 0 ? box_dist<T, PER>(px, py, pz, bx[i]) : D(0);
-        const bool full = count >= max_per;
-        bool       over = false;
-#pragma unroll
-        for (int i = 3; i >= 0; --i) {
-            const int c = ch[i];
-            if (c < 0 || !(d[i] <= RM2)) continue;
-            if (c >= n - 1) {             // a leaf
-                if (!(d[i] >= rm2)) continue; // inside r_min
-                if (full) {
-                    ++count;
-                    continue;
-                }
-            } else if (full && d[i] >= rm2) {
-                D far;
-                if (far_dist_box<T, PER>(px, py, pz, bx[i], far) && far <= RM2) {
-                    count += t.leaves[c]; // every leaf below lies in the shell
-                    continue;
-                }
-            }
-            if (sp >= kStack * 2) {
-                over = true;
-                break;
-            }
-            sn[sp++] = c;
-        }
-        if (over) {
-            atomicOr(status, STATUS_TRAVERSAL_LIMIT);
-            break;
+        __syncwarp();
+        if (pop && have) {
+            have = sp > 0;
+            if (have) cur = st[--sp];
         }
     }
     return count;
+}
+
+// The query's place in the frame and its limits; false when the frame does not hold it (the
+// caller then walks the binary records).
+template <class T, int PER>
+FT_D bool range_prepare(const TreeDev<T> &t, QFrame<T> &fr, RangePoint<T, PER> &pt, RangeLimits &lim) {
+    const T rb[6] = {t.min_x[0], t.max_x[0], t.min_y[0], t.max_y[0], t.min_z[0], t.max_z[0]};
+    fr.make(rb, t.n, PER != 0);
+    const bool a = fr.template query<(PER != 0)>(pt.px, 0, pt.u[0]), b = fr.template query<(PER != 0)>(pt.py, 1, pt.u[1]),
+               c = fr.template query<(PER != 0)>(pt.pz, 2, pt.u[2]);
+    if constexpr (PER == 2 && sizeof(T) == 8) {
+        pt.ul[0] = (uint32_t)pt.px << 22;
+        pt.ul[1] = (uint32_t)pt.py << 22;
+        pt.ul[2] = (uint32_t)pt.pz << 22;
+    }
+    pt.m   = fr.m;
+    lim    = range_limits<T>(fr, pt.rm2, pt.RM2);
+    pt.out = lim.out;
+    pt.lx  = t.min_x + (t.n - 1);
+    pt.ly  = t.min_y + (t.n - 1);
+    pt.lz  = t.min_z + (t.n - 1);
+    return fr.ok && a && b && c;
 }
 
 template <class T, int PER>
@@ -733,284 +833,206 @@ __global__ void __launch_bounds__(128)
                       const T *__restrict__ rmin, const T *__restrict__ rmax, int nq, int32_t *__restrict__ results,
                       int32_t *__restrict__ counts, int max_per, int ret_orig, const uint32_t *__restrict__ order,
                       uint32_t *status) {
-    using D     = typename Coord<T>::dist_t;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nq) return;
-    const int q = order ? (int)order[i] : i;
-    D         rm2, RM2;
-    range_radii<T>(rmin, rmax, q, rm2, RM2);
-    counts[q] = range_one_wide<T, PER>(t, qx[q], qy[q], qz[q], rm2, RM2, results, (size_t)q * (size_t)max_per,
-                                       max_per, ret_orig, status);
+    const int  base   = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
+    if (base >= nq) return; // warp-uniform
+    const int  i      = base + (threadIdx.x & 31);
+    const bool active = i < nq;
+    const int  q      = active ? (order ? (int)order[i] : i) : (order ? (int)order[base] : base);
+    RangePoint<T, PER> pt;
+    pt.px = qx[q];
+    pt.py = qy[q];
+    pt.pz = qz[q];
+    range_radii<T>(rmin, rmax, q, pt.rm2, pt.RM2);
+    QFrame<T>    fr;
+    RangeLimits  lim;
+    const bool   framed = range_prepare<T, PER>(t, fr, pt, lim);
+    const size_t off    = (size_t)q * (size_t)max_per;
+    int          cnt    = range_rows<T, PER, false>(t, active && framed, pt, lim, results, off, max_per, ret_orig, status);
+    if (active && !framed)
+        cnt = range_one<T, PER>(t, pt.px, pt.py, pt.pz, pt.rm2, pt.RM2, results, off, max_per, ret_orig, status);
+    if (active) counts[q] = cnt;
 }
 
 // -----------------------------------------------------------------------------------------
-// range_query counts, a warp's queries together.  A row's count is the number of leaves in
-// the query's shell (rmin^2 <= d <= rmax^2): on trees where the box distance is monotone over
-// nested boxes (the 4-wide walk's condition) a leaf's own distance decides it, whatever order
-// the walk takes, so the count needs no walk order.  The lanes that still need a count (their
-// rows are full) are neighbours on the curve; their query points lie in a small group box.
-// For a node box, group_near_far bounds, per axis, the gap node_distance_sq measures between
-// any of the group's points and any point of the box (near: no gap is smaller; far: none is
-// larger); the squared distances built from them bound every lane's distance to every leaf
-// below the node, since the shift, the squares, rounding and the sums are monotone.  A node
-// beyond every lane's r_max is skipped; one inside every lane's shell adds its leaf count to
-// every lane; the rest are expanded, and their leaves are staged for a test by each lane.
+// range_query counts, a warp's queries together.  The lanes that still need a count (their
+// rows are full) are neighbours on the curve; their query points lie in a small group box of
+// the frame.  For a node box, the gaps between the two boxes' centres, less or plus both half
+// extents, bound every lane's distance to every leaf below it.  A node beyond every lane's
+// r_max is skipped; one inside every lane's shell adds its leaf count to every lane; the rest
+// are expanded, and the leaves of their buckets are staged for a test by each lane.
 // -----------------------------------------------------------------------------------------
-// Group frame: per axis the group's points lie in [g0, g0 + span] (for the 42-bit periodic
-// metric an arc of the circle starting at g0; for floating point, [g0, g1]).
-template <class T> struct RangeGroup {
-    T                  g0[3], g1[3];
-    unsigned long long span[3];
-};
-
-template <class T, int PER>
-FT_D void group_near_far(const RangeGroup<T> &g, const T b[6], typename Coord<T>::dist_t &near,
-                         typename Coord<T>::dist_t &far) {
-    using C = Coord<T>;
-    if constexpr (C::is_float) {
-        T n3[3], f3[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const T lo = b[2 * a], hi = b[2 * a + 1];
-            n3[a] = c_fmax(c_fmax(T(0), sub_rn(lo, g.g1[a])), sub_rn(g.g0[a], hi));
-            f3[a] = c_fmax(sub_rn(hi, g.g0[a]), sub_rn(g.g1[a], lo));
-        }
-        near = (double)add_rn(add_rn(mul_rn(n3[0], n3[0]), mul_rn(n3[1], n3[1])), mul_rn(n3[2], n3[2]));
-        far  = (double)add_rn(add_rn(mul_rn(f3[0], f3[0]), mul_rn(f3[1], f3[1])), mul_rn(f3[2], f3[2]));
-    } else if constexpr (PER == 2) {
-        // gaps between the arc G = [g0, g0 + span] and the box [lo, hi] are the circular
-        // distances w(u) = min(u, P - u) of the differences u in D = [lo - g0 - span, hi - g0]
-        // (mod P), an arc of length len: w is 0 where D holds 0, P/2 where it holds P/2, and
-        // otherwise takes its extremes at D's ends
-        constexpr unsigned long long P = 1ull << C::bits, M = P - 1ull, H = P >> 1;
-        unsigned long long sn = 0, sf = 0;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const unsigned long long lo = (unsigned long long)b[2 * a], hi = (unsigned long long)b[2 * a + 1];
-            const unsigned long long st  = (lo - (unsigned long long)g.g0[a] - g.span[a]) & M;
-            const unsigned long long len = (hi - lo) + g.span[a];
-            unsigned long long       gn = 0, gf = H;
-            if (len < P) {
-                const unsigned long long en = (st + len) & M;
-                const unsigned long long wa = st <= H ? st : P - st, we = en <= H ? en : P - en;
-                const bool               z  = st == 0 || st + len >= P;
-                const bool               h  = ((H - st) & M) <= len;
-                gn = z ? 0ull : (wa < we ? wa : we);
-                gf = h ? H : (wa > we ? wa : we);
-            }
-            sn += Metric<T>::sq((unsigned long long)(uint32_t)(gn >> C::dist_shift));
-            sf += Metric<T>::sq((unsigned long long)(uint32_t)(gf >> C::dist_shift));
-        }
-        near = sn;
-        far  = sf;
-    } else {
-        unsigned long long sn = 0, sf = 0;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const T lo = b[2 * a], hi = b[2 * a + 1], g0 = g.g0[a], g1 = g.g1[a];
-            const unsigned long long gn = lo > g1   ? (unsigned long long)(T)(lo - g1)
-                                          : g0 > hi ? (unsigned long long)(T)(g0 - hi)
-                                                    : 0ull;
-            const unsigned long long fa = g1 > lo ? (unsigned long long)(T)(g1 - lo) : 0ull;
-            const unsigned long long fb = hi > g0 ? (unsigned long long)(T)(hi - g0) : 0ull;
-            sn += Metric<T>::sq(gn >> C::dist_shift);
-            sf += Metric<T>::sq((fa > fb ? fa : fb) >> C::dist_shift);
-        }
-        near = sn;
-        far  = sf;
-    }
-}
-
-// Offset of coordinate v from the group's corner, as a float for the leaf filter: the signed
-// 42-bit wrapped difference (periodic), else the plain difference.
-template <class T, int PER> FT_D float group_off(T v, const RangeGroup<T> &g, int a) {
-    if constexpr (Coord<T>::is_float) {
-        return (float)sub_rn(v, g.g0[a]);
-    } else if constexpr (PER == 2) {
-        constexpr int sh = 64 - Coord<T>::bits;
-        return (float)((long long)(((unsigned long long)v - (unsigned long long)g.g0[a]) << sh) >> sh);
-    } else {
-        return (float)((long long)(unsigned long long)v - (long long)(unsigned long long)g.g0[a]);
-    }
-}
-
-// range_split_kernel's shape: two-warp blocks (a block keeps its SM slots until its slowest
-// warp ends, and the warps' work is very uneven) compiled for 8 resident blocks (124
-// registers a thread, no spills).  Measured on 10M clustered points, all N queries, back to
-// back on one GPU: 4-warp blocks 2.83 s, 2-warp 2.85 s, 1-warp 2.80 s (123 registers each),
-// 2-warp with 10 / 12 resident blocks 2.42 / 2.44 s; with the threshold leaf filter, 8 / 10 /
-// 12 resident blocks 1.93 / 2.05 / 2.11 s (the tighter budgets spill).
 #ifndef FT_RANGE_WARPS
 #define FT_RANGE_WARPS 2
 #endif
 #ifndef FT_RANGE_MINB
 #define FT_RANGE_MINB 8
 #endif
-static constexpr int kRangeWarps = FT_RANGE_WARPS, kRangeGStack = 512, kRangeStage = 256;
+static constexpr int kRangeWarps = FT_RANGE_WARPS, kRangeGStack = 512, kRangeStage = 256, kRangeList = 160;
 // The group counts a warp's full rows together when its points' largest axis extent is at
-// most 1/FT_RANGE_SPREAD of the smallest radius (measured on 10M clustered points, r = 2e-3 of
-// the box, all N queries: factors 1 / 4 / 16 2.38 / 2.39 / 3.48 s, every group together
-// 2.37 s, the per-query 4-wide walk 5.87 s; then 2.04 s with the threshold leaf filter, of
-// which the rows take 0.12 s).
-#ifndef FT_RANGE_SPREAD
-#define FT_RANGE_SPREAD 1
-#endif
+// most the smallest radius (measured on 10M clustered points, r = 2e-3 of the box, all N
+// queries: factors 1 / 4 / 16 of the extent 2.38 / 2.39 / 3.48 s).
+struct alignas(16) RangeShared {
+    int32_t  stk[kRangeGStack];
+    uint32_t list[kRangeList]; // buckets whose leaves the lanes test
+    float4   stage[kRangeStage];
+};
 
 // The group count of the lanes with `need` (every lane of the warp calls it).  Returns false
 // (counts unset) when the group is too spread out for its bounds to help (FORCE: only when
 // the float filter's accuracy needs it), or a stack would overflow; the caller then counts
 // per lane.  count: this lane's shell count.
 template <class T, int PER, bool FORCE = false>
-FT_D bool range_count_group(const TreeDev<T> &t, bool need, T px, T py, T pz, typename Coord<T>::dist_t rm2,
-                            typename Coord<T>::dist_t RM2, int32_t *stk, float4 *stage, int &count) {
+FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr, const RangePoint<T, PER> &pt,
+                            const RangeLimits &lim, RangeShared &sh, int &count) {
     using C                = Coord<T>;
     using D                = typename C::dist_t;
     const unsigned FULL    = 0xffffffffu;
     const int      lane    = threadIdx.x & 31;
     const int      n       = t.n;
-    if (n < 2) return false;
-    if constexpr (PER == 1) return false; // the general periodic form: no group bounds
-    RangeGroup<T> g;
-    T             v[3] = {px, py, pz};
-    if constexpr (PER == 2) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) v[a] = (T)((unsigned long long)v[a] & ((1ull << C::bits) - 1ull));
-    }
-    if constexpr (C::is_float) {
-        bool fin = true;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) fin = fin && isfinite((double)v[a]);
-        if (!__all_sync(FULL, !need || fin)) return false;
-    }
-    const unsigned nm  = __ballot_sync(FULL, need);
-    const int      ref = __ffs(nm) - 1;
-    double         spread = 0.0; // largest axis extent, in coordinate units
+    const unsigned nm      = __ballot_sync(FULL, need);
+    const int      ref     = __ffs(nm) - 1;
+    // the group's box: centre gc and half extent gh per axis, corner g0
+    int32_t  g0[3], gc[3];
+    uint32_t gh[3], spread = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        if constexpr (PER == 2) {
-            constexpr int sh = 64 - C::bits;
-            const T       r  = __shfl_sync(FULL, v[a], ref);
-            long long     o  = (long long)(((unsigned long long)v[a] - (unsigned long long)r) << sh) >> sh;
-            long long     lo = need ? o : LLONG_MAX, hi = need ? o : LLONG_MIN;
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1) {
-                lo = min(lo, __shfl_xor_sync(FULL, lo, m));
-                hi = max(hi, __shfl_xor_sync(FULL, hi, m));
-            }
-            g.g0[a]   = (T)(((unsigned long long)r + (unsigned long long)lo) & ((1ull << C::bits) - 1ull));
-            g.span[a] = (unsigned long long)(hi - lo);
-            g.g1[a]   = g.g0[a];
-            spread    = fmax(spread, (double)g.span[a]);
-        } else {
-            const T r  = __shfl_sync(FULL, v[a], ref);
-            T       lo = need ? v[a] : r, hi = lo;
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1) {
-                const T u = __shfl_xor_sync(FULL, lo, m), w = __shfl_xor_sync(FULL, hi, m);
-                lo        = u < lo ? u : lo;
-                hi        = w > hi ? w : hi;
-            }
-            g.g0[a]   = lo;
-            g.g1[a]   = hi;
-            g.span[a] = C::is_float ? 0ull : (unsigned long long)(T)(hi - lo);
-            spread    = fmax(spread, (double)hi - (double)lo);
-        }
+        const int32_t  r  = __shfl_sync(FULL, pt.u[a], ref);
+        const int32_t  o  = need ? (int32_t)((uint32_t)pt.u[a] - (uint32_t)r) : 0;
+        const int32_t  lo = __reduce_min_sync(FULL, o), hi = __reduce_max_sync(FULL, o);
+        const uint32_t sp = (uint32_t)hi - (uint32_t)lo;
+        g0[a]             = (int32_t)((uint32_t)r + (uint32_t)lo);
+        gc[a]             = (int32_t)((uint32_t)g0[a] + (sp >> 1));
+        gh[a]             = sp - (sp >> 1);
+        spread            = max(spread, sp);
     }
-    // the lanes' radii
-    D R_lo = need ? RM2 : dist_heap_max<D>(), R_hi = need ? RM2 : D(0);
-    D r_lo = need ? rm2 : dist_heap_max<D>(), r_hi = need ? rm2 : D(0);
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {
-        const D a = __shfl_xor_sync(FULL, R_lo, m), b = __shfl_xor_sync(FULL, R_hi, m);
-        const D c = __shfl_xor_sync(FULL, r_lo, m), d = __shfl_xor_sync(FULL, r_hi, m);
-        R_lo = a < R_lo ? a : R_lo;
-        R_hi = b > R_hi ? b : R_hi;
-        r_lo = c < r_lo ? c : r_lo;
-        r_hi = d > r_hi ? d : r_hi;
-    }
+    // the lanes' limits (not negative: their bits order as integers)
+    auto fmin_warp = [&](float v) { return __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(v))); };
+    auto fmax_warp = [&](float v) { return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(v))); };
+    const float inf   = __int_as_float(0x7f800000);
+    const float R_out = fmax_warp(need ? lim.out : 0.0f);            // beyond every ball
+    const float R_in  = fmin_warp(need ? fmaxf(lim.in, 0.0f) : inf); // inside every ball
+    const float r_ge  = fmax_warp(need ? lim.ge : 0.0f);             // at or beyond every r_min
+    const float r_lt  = fmin_warp(need ? fmaxf(lim.lt, 0.0f) : inf); // inside every r_min
     // worth it only when the group is small against the radius (its fuzzy shell thin), and the
     // leaf filter's float offsets stay accurate: every staged leaf lies within
-    // lam = spread + (sqrt(R_hi) + 2) 2^shift of the group's corner on each axis
-    const double unit = C::is_float ? 1.0 : (double)(1ull << C::dist_shift);
-    const double rad  = sqrt((double)R_lo) * unit, Rad = (sqrt((double)R_hi) + 2.0) * unit;
-    const double lam  = spread + Rad * (1.0 + 0x1p-20);
-    bool         ok   = (FORCE || spread * (double)FT_RANGE_SPREAD <= rad) && lam > 0.0;
-    // (floating point: squared offsets stay normal floats)
-    if constexpr (C::is_float) ok = ok && lam < 0x1p60 && lam > 0x1p-60;
-    else ok = ok && lam < 0x1p40;
-    if (!ok) return false; // warp-uniform
-    // Leaf filter.  In shifted units u (offsets / 2^shift for integers, plain offsets for
-    // floating point) a lane's float estimate of a gap is y = |e - q|, within eps of the exact
-    // gap (conversions and the subtraction: at most 2^-22 lam, taken as 2^-20 lam).  Integer
-    // terms floor the shifted gap, t in (y - eps - 1, y + eps], so with Y = sum y^2 and
+    // lam = spread + sqrt(R_out) + 2 m of the group's corner on each axis
+    const double rad = sqrt((double)R_in);
+    const double lam = (double)spread + sqrt((double)R_out) + 2.0 * (double)fr.m + 2.0;
+    if (!((FORCE || (double)spread <= rad) && lam < 0x1p31)) return false; // warp-uniform
+    // Leaf filter (float coordinates: the staged coordinates give the exact distance).  S frame
+    // units make one distance unit (2^dist_shift coordinate units for integers, one coordinate
+    // for floating point).  A lane's float estimate of a gap, |e - q| from the offsets of leaf
+    // and query from the group's corner, is within 1 + 2^-20 lam frame units of the real one
+    // (both positions floored; two conversions and a subtraction), eps distance units.  Integer
+    // terms floor the gap, t in (y - eps - 1, y + eps], so with Y = sum y^2 and
     // sum y <= sqrt(3 Y) the exact distance lies in [Y - c_lo sqrt(Y), Y + c_hi sqrt(Y) + 3 eps^2],
     // c_lo = 2 sqrt(3) (1 + eps), c_hi = 2 sqrt(3) eps; floating-point terms have no floor
     // (c_lo = c_hi) and the reference's rounded sum lies within 1 +- 2^-20 of the real one.
     // Each bound is monotone in Y, so four thresholds on Y decide a leaf: beyond r_max, inside
     // r_max, at least r_min, below r_min.  The leaf's Y is computed in float (relative error
-    // under 2^-22, covered by a factor 1 +- 2^-21 on the thresholds) from offsets in units of
-    // 2^shift: 3 subtractions and 3 multiply-adds a leaf, the exact distance only in the thin
-    // band around the lane's spheres.
-    const double eps  = lam * 0x1p-20 / unit;
-    const double c_lo = 3.4641016151377546 * ((C::is_float ? 0.0 : 1.0) + eps) * (1.0 + 0x1p-40);
-    const double c_hi = 3.4641016151377546 * eps * (1.0 + 0x1p-40);
-    const double rho  = C::is_float ? 0x1p-20 : 0.0;
-    const double u2   = unit * unit; // shifted units^2 -> offset units^2
-    // smallest Y whose lower bound exceeds (or reaches) X, and largest Y whose upper bound
-    // stays at or below X (-1: none)
-    auto y_lower = [&](double X) {
-        const double r = (c_lo + sqrt(c_lo * c_lo + 4.0 * X)) * 0.5;
-        return r * r;
-    };
-    auto y_upper = [&](double X) {
-        const double a = X - 3.0 * eps * eps;
-        if (a < 0.0) return -1.0;
-        const double r = (-c_hi + sqrt(c_hi * c_hi + 4.0 * a)) * 0.5;
-        return r * r;
-    };
-    const double Rd = (double)RM2, rd = (double)rm2;
-    // out if Y > t_out; in r_max if Y <= t_in; at least r_min if Y >= t_ge; below r_min if Y < t_lt
-    const float t_out = __double2float_ru(y_lower(Rd / (1.0 - rho)) * u2 * (1.0 + 0x1p-21));
-    const float t_in  = __double2float_rd(fmax(y_upper(Rd / (1.0 + rho)), -1.0) * u2 * (1.0 - 0x1p-21));
-    const float t_ge  = rd <= 0.0 ? 0.0f : __double2float_ru(y_lower(rd / (1.0 - rho)) * u2 * (1.0 + 0x1p-21));
-    const float t_lt  = rd <= 0.0 ? -1.0f : __double2float_rd(fmax(y_upper(rd / (1.0 + rho)), -1.0) * u2 * (1.0 - 0x1p-21));
-    const float qf[3] = {group_off<T, PER>(v[0], g, 0), group_off<T, PER>(v[1], g, 1), group_off<T, PER>(v[2], g, 2)};
-
-    int       mine = 0;    // this lane's count from staged leaves
-    long long part = 0;    // leaves in nodes inside every lane's shell, found by this lane
-    int       top = 0, cc = 0;
-    bool      overflow = false;
-    {
-        const T rb[6] = {t.min_x[0], t.max_x[0], t.min_y[0], t.max_y[0], t.min_z[0], t.max_z[0]};
-        D       rn, rf;
-        group_near_far<T, PER>(g, rb, rn, rf);
-        if (rn <= R_hi) {
-            if (rn >= r_hi && rf <= R_lo) part = lane == 0 ? n : 0;
-            else if (!(rf < r_lo)) top = 1;
-        }
+    // under 2^-22, covered by a factor 1 +- 2^-21 on the thresholds): 3 subtractions and 3
+    // multiply-adds a leaf, the exact distance only in the thin band around the lane's spheres.
+    float t_out, t_in, t_ge, t_lt;
+    float qf[3];
+    if constexpr (std::is_same<T, float>::value) {
+        t_in  = __double2float_rd(pt.RM2);
+        t_ge  = __double2float_ru(pt.rm2);
+        t_out = t_in;
+        t_lt  = t_ge;
+        qf[0] = pt.px;
+        qf[1] = pt.py;
+        qf[2] = pt.pz;
+    } else {
+        const double S    = C::is_float ? fr.s
+                                        : __longlong_as_double((long long)(1023 + C::dist_shift - fr.shift) << 52);
+        const double eps  = (1.0 + lam * 0x1p-20) / S;
+        const double c_lo = 3.4641016151377546 * ((C::is_float ? 0.0 : 1.0) + eps) * (1.0 + 0x1p-40);
+        const double c_hi = 3.4641016151377546 * eps * (1.0 + 0x1p-40);
+        const double rho  = C::is_float ? 0x1p-20 : 0.0;
+        const double u2   = S * S; // distance units^2 -> frame units^2
+        // smallest Y whose lower bound exceeds (or reaches) X, and largest Y whose upper bound
+        // stays at or below X (-1: none)
+        auto y_lower = [&](double X) {
+            const double r = (c_lo + sqrt(c_lo * c_lo + 4.0 * X)) * 0.5;
+            return r * r;
+        };
+        auto y_upper = [&](double X) {
+            const double a = X - 3.0 * eps * eps;
+            if (a < 0.0) return -1.0;
+            const double r = (-c_hi + sqrt(c_hi * c_hi + 4.0 * a)) * 0.5;
+            return r * r;
+        };
+        const double Rd = (double)pt.RM2, rd = (double)pt.rm2;
+        t_out = __double2float_ru(y_lower(Rd / (1.0 - rho)) * u2 * (1.0 + 0x1p-21));
+        t_in  = __double2float_rd(fmax(y_upper(Rd / (1.0 + rho)), -1.0) * u2 * (1.0 - 0x1p-21));
+        t_ge  = rd <= 0.0 ? 0.0f : __double2float_ru(y_lower(rd / (1.0 - rho)) * u2 * (1.0 + 0x1p-21));
+        t_lt  = rd <= 0.0 ? -1.0f : __double2float_rd(fmax(y_upper(rd / (1.0 + rho)), -1.0) * u2 * (1.0 - 0x1p-21));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) qf[a] = (float)(int32_t)((uint32_t)pt.u[a] - (uint32_t)g0[a]);
     }
-    if (lane == 0) stk[0] = 0;
+    if (!need) { // no leaf is near such a lane
+        t_out = t_in = -1.0f;
+        t_lt = t_ge = inf;
+    }
+
+    int       mine = 0; // this lane's count from staged leaves
+    long long part = 0; // leaves in nodes inside every lane's shell, found by this lane
+    int       top = 1, lc = 0;
+    bool      overflow = false;
+    const uint4 *pts = reinterpret_cast<const uint4 *>(t.qpts);
+    if (lane == 0) sh.stk[0] = 0;
     __syncwarp();
-    // each lane tests every staged leaf: the float filter, then the exact distance where the
-    // filter cannot decide
+    // the listed buckets' leaves are staged, 32 buckets at a time, and each lane tests every
+    // staged leaf: the float filter, then the exact distance where the filter cannot decide
     auto flush = [&]() {
-        for (int j = 0; j < cc; ++j) {
-            const float4 e = stage[j];
-            if (!need) continue;
-            const float dx = e.x - qf[0], dy = e.y - qf[1], dz = e.z - qf[2];
-            const float Y  = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-            if (Y > t_out || Y < t_lt) continue; // surely outside the shell
-            if (Y <= t_in && Y >= t_ge) {        // surely inside
-                ++mine;
-                continue;
+        for (int b = 0; b < lc; b += 32) {
+            const uint32_t r     = b + lane < lc ? sh.list[b + lane] : kQEmpty;
+            const int      first = qref_first(r), cnt = r != kQEmpty ? qref_count(r) : 0;
+            int            incl  = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int w = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += w;
             }
-            const int s = __float_as_int(e.w);
-            const T   x = t.min_x[s], y = t.min_y[s], z = t.min_z[s];
-            const D   d = Metric<T>::template dist<(PER != 0), (PER == 2)>(px, py, pz, x, x, y, y, z, z);
-            mine += (d >= rm2 && d <= RM2) ? 1 : 0;
+            const int tot = __shfl_sync(FULL, incl, 31);
+            const int at  = incl - cnt;
+#pragma unroll
+            for (int j = 0; j < kBucket; ++j)
+                if (j < cnt) {
+                    const uint4 v = __ldg(pts + first + j);
+                    float4      e;
+                    if constexpr (std::is_same<T, float>::value) {
+                        e.x = __uint_as_float(v.x);
+                        e.y = __uint_as_float(v.y);
+                        e.z = __uint_as_float(v.z);
+                    } else {
+                        e.x = (float)(int32_t)(v.x - (uint32_t)g0[0]);
+                        e.y = (float)(int32_t)(v.y - (uint32_t)g0[1]);
+                        e.z = (float)(int32_t)(v.z - (uint32_t)g0[2]);
+                    }
+                    e.w              = __int_as_float(first + j);
+                    sh.stage[at + j] = e;
+                }
+            __syncwarp();
+            for (int j = 0; j < tot; ++j) {
+                const float4 e  = sh.stage[j];
+                const float  dx = e.x - qf[0], dy = e.y - qf[1], dz = e.z - qf[2];
+                if constexpr (std::is_same<T, float>::value) {
+                    const float d = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
+                    mine += (d <= t_in && d >= t_ge) ? 1 : 0;
+                } else {
+                    const float Y  = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                    const bool  in = Y <= t_in && Y >= t_ge;
+                    mine += in ? 1 : 0;
+                    if (!in && !(Y > t_out || Y < t_lt)) {
+                        const int leaf = __float_as_int(e.w);
+                        mine += pt(__ldg(pts + leaf), leaf) ? 1 : 0;
+                    }
+                }
+            }
+            __syncwarp();
         }
-        cc = 0;
-        __syncwarp();
+        lc = 0;
     };
     long long budget = 2ll * n + 64;
     while (top > 0) {
@@ -1020,23 +1042,36 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, T px, T py, T pz, ty
             break;
         }
         const int base = top - m;
-        const int node = lane < m ? stk[base + lane] : -1;
+        const int node = lane < m ? sh.stk[base + lane] : -1;
         top            = base;
         __syncwarp();
-        T        bx[4][6];
-        int      ch[4] = {-1, -1, -1, -1};
         unsigned kl = 0, ki = 0;
+        uint32_t rf[4] = {0, 0, 0, 0};
         if (node >= 0) {
-            load_wide(t.wide, node, bx, ch);
+            const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + node);
+            uint4        v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __ldg(p + i);
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                if (ch[i] < 0) continue;
-                D dn, dfar;
-                group_near_far<T, PER>(g, bx[i], dn, dfar);
-                if (!(dn <= R_hi) || dfar < r_lo) continue; // outside every ball, or inside every r_min
-                const bool leaf = ch[i] >= n - 1;
-                if (dn >= r_hi && dfar <= R_lo) part += leaf ? 1 : t.leaves[ch[i]]; // inside every shell
-                else if (leaf) kl |= 1u << i;
+                rf[i] = w[24 + i];
+                if (rf[i] == kQEmpty) continue;
+                float nr[3], fa[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const uint32_t d = (uint32_t)abs((int32_t)((uint32_t)gc[a] - w[6 * i + a]));
+                    const uint32_t h = w[6 * i + 3 + a];
+                    uint32_t       s = h + gh[a];
+                    if (s < h) s = 0xffffffffu;
+                    nr[a] = (float)(d - min(d, s));
+                    fa[a] = (float)d + (float)h + (float)gh[a];
+                }
+                const float near = fmaf(nr[2], nr[2], fmaf(nr[1], nr[1], nr[0] * nr[0]));
+                const float far  = fmaf(fa[2], fa[2], fmaf(fa[1], fa[1], fa[0] * fa[0])) * (1.0f + 0x1p-20f);
+                if (near > R_out || far < r_lt) continue; // outside every ball, or inside every r_min
+                if (near >= r_ge && far <= R_in) part += (long long)w[28 + i]; // inside every shell
+                else if (rf[i] & kQBucket) kl |= 1u << i;
                 else ki |= 1u << i;
             }
         }
@@ -1044,20 +1079,18 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, T px, T py, T pz, ty
         int       incl = nl | (ni << 16);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += u;
+            const int w = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += w;
         }
         const int tot = __shfl_sync(FULL, incl, 31);
-        if (cc + (tot & 0xffff) > kRangeStage) flush();
-        int pl = cc + (incl & 0xffff) - nl, pi = top + (incl >> 16) - ni;
+        if (lc + (tot & 0xffff) > kRangeList) flush();
+        int pl = lc + (incl & 0xffff) - nl, pi = top + (incl >> 16) - ni;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            if ((kl >> i) & 1u)
-                stage[pl++] = make_float4(group_off<T, PER>(bx[i][0], g, 0), group_off<T, PER>(bx[i][2], g, 1),
-                                          group_off<T, PER>(bx[i][4], g, 2), __int_as_float(ch[i]));
-            if ((ki >> i) & 1u) stk[pi++] = ch[i];
+            if ((kl >> i) & 1u) sh.list[pl++] = rf[i];
+            if ((ki >> i) & 1u) sh.stk[pi++] = (int32_t)rf[i];
         }
-        cc += tot & 0xffff;
+        lc += tot & 0xffff;
         top += tot >> 16;
         __syncwarp();
     }
@@ -1070,41 +1103,42 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, T px, T py, T pz, ty
 }
 
 // range_query on trees of height <= 62 with a monotone box distance (default): phase 1 writes
-// each row in the reference's order with the 4-wide walk and stops once the row is full;
-// phase 2 counts the full rows' shells with range_count_group (per lane when the group's
-// bounds cannot help).  Counts, rows and their order equal range_wide_kernel's.
+// each row in the reference's order and stops once the row is full; phase 2 counts the full
+// rows' shells with range_count_group (per lane when the group's bounds cannot help).  Lanes
+// whose query the frame does not hold walk the binary records.
 template <class T, int PER, bool FORCE = false>
 __global__ void __launch_bounds__(32 * kRangeWarps, FT_RANGE_MINB)
     range_split_kernel(TreeDev<T> t, const T *__restrict__ qx, const T *__restrict__ qy, const T *__restrict__ qz,
                        const T *__restrict__ rmin, const T *__restrict__ rmax, int nq, int32_t *__restrict__ results,
                        int32_t *__restrict__ counts, int max_per, int ret_orig, const uint32_t *__restrict__ order,
                        uint32_t *status) {
-    using D = typename Coord<T>::dist_t;
-    __shared__ int32_t s_stk[kRangeWarps][kRangeGStack];
-    __shared__ float4  s_stage[kRangeWarps][kRangeStage];
+    __shared__ RangeShared s_sh[kRangeWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int base = (blockIdx.x * kRangeWarps + warp) * 32;
     if (base >= nq) return; // warp-uniform
     const int  i      = base + lane;
     const bool active = i < nq;
     const int  q      = active ? (order ? (int)order[i] : i) : (order ? (int)order[base] : base);
-    D          rm2 = D(0), RM2 = D(0);
-    range_radii<T>(rmin, rmax, q, rm2, RM2);
-    const T      px = qx[q], py = qy[q], pz = qz[q];
-    const size_t off = (size_t)q * (size_t)max_per;
+    RangePoint<T, PER> pt;
+    pt.px = qx[q];
+    pt.py = qy[q];
+    pt.pz = qz[q];
+    range_radii<T>(rmin, rmax, q, pt.rm2, pt.RM2);
+    QFrame<T>    fr;
+    RangeLimits  lim;
+    const bool   framed = range_prepare<T, PER>(t, fr, pt, lim);
+    const size_t off    = (size_t)q * (size_t)max_per;
     bool         filled = false;
-    int          cnt    = 0;
-    if (active)
-        cnt = range_one_wide<T, PER, true>(t, px, py, pz, rm2, RM2, results, off, max_per, ret_orig, status, &filled);
+    int cnt = range_rows<T, PER, true>(t, active && framed, pt, lim, results, off, max_per, ret_orig, status, &filled);
     const bool need = active && filled;
     if (__any_sync(0xffffffffu, need)) {
-        int total = 0;
-        if (range_count_group<T, PER, FORCE>(t, need, px, py, pz, rm2, RM2, s_stk[warp], s_stage[warp], total)) {
-            if (need) cnt = total;
-        } else if (need) {
-            cnt = range_one_wide<T, PER>(t, px, py, pz, rm2, RM2, results, off, 0, ret_orig, status);
-        }
+        int        total = 0;
+        const bool done  = range_count_group<T, PER, FORCE>(t, need, fr, pt, lim, s_sh[warp], total);
+        if (!done) total = range_rows<T, PER, false>(t, need, pt, lim, results, off, 0, ret_orig, status);
+        if (need) cnt = total;
     }
+    if (active && !framed)
+        cnt = range_one<T, PER>(t, pt.px, pt.py, pt.pz, pt.rm2, pt.RM2, results, off, max_per, ret_orig, status);
     if (active) counts[q] = cnt;
 }
 
@@ -1691,9 +1725,9 @@ static void range_typed(const ft_options &o, const ft_tree &tr, const void *qx, 
     // trees of height <= 62 never reach the reference's stack guard (range_short_kernel)
     const TreeImpl *impl  = (const TreeImpl *)tr.impl;
     const bool      short_walk = impl && impl->height_root >= 0 && impl->height_root <= 62;
-    // the 4-wide walk skips the binary level between a node and its grandchildren, exact when
-    // the box distance is monotone over nested boxes (the fast walks' condition)
-    const bool      wide = impl && fast_walk_applies(o, *impl);
+    // the walks over the 32-bit records prune by lower bounds, exact when the box distance is
+    // monotone over nested boxes (the fast walks' condition)
+    const bool      wide = impl && tr.num_leaves > 1 && impl->framed && fast_walk_applies(o, *impl);
     met_dispatch<T>(metric_mode<T>(o, tr), [&](auto M) {
         auto fn = !short_walk ? range_kernel<T, decltype(M)::value>
                   : walk == 2 ? range_group_kernel<T, decltype(M)::value>

@@ -8,8 +8,8 @@
 // context.  Later calls with default options take the kept choice.
 //  * build: keys per thread of a onesweep tile (8 / 12 / 16 / 20 for one-word keys, 8 / 12 /
 //    16 for two-word keys), timed over whole builds of the caller's points;
-//  * self-kNN (single tree and batched sets): the walk variant (4-wide per-lane walk, compact
-//    binary walk, group walk), the SFC seeding half-window (k/2, k, 2k) and the block shape
+//  * self-kNN (single tree and batched sets): the walk variant (4-wide walk, exact binary
+//    walk), the SFC seeding half-window (k/2, k, 2k) and the block shape
 //    (two-warp blocks with 32-entry heaps, or one-warp blocks), timed on up to 2^18 queries
 //    (four stretches of consecutive leaves, the order the walk takes them in) or, for a batch,
 //    on the whole batch.
@@ -105,9 +105,9 @@ struct WalkCandidate {
 std::vector<WalkCandidate> walk_candidates(int k, bool batch) {
     const int                  kc_default = k <= 32 ? 32 : 64;
     std::vector<WalkCandidate> c;
-    // the defaults first: the 4-wide walk (the compact binary walk for k <= 4), half-window k
-    c.push_back({k <= 4 ? 2 : 4, k, kc_default});
-    const int variants[3] = {4, 2, 5};
+    // the defaults first: the 4-wide walk, half-window k
+    c.push_back({4, k, kc_default});
+    const int variants[2] = {4, 2};
     const int halves[3]   = {k, std::max(1, k / 2), 2 * k};
     for (int v : variants)
         for (int h : halves) {

@@ -445,7 +445,7 @@ def _method(method) -> int:
 def _qopts(max_k: int, method="fast", half_window: int = 0, variant: int = 0):
     o = capi.FtQueryOptions(int(max_k), _method(method))
     o.reserved[0] = int(half_window)  # fast walk: SFC seeding half-window (0 = k)
-    o.reserved[1] = int(variant)      # fast walk: 0 default, 1 per-lane, 2 compact, 3 warp-shared, 4 4-wide, 5 group
+    o.reserved[1] = int(variant)      # fast walk: 0 default, 2 exact binary, 1 and 3 to 5 the 4-wide walk
     return o
 
 

@@ -93,7 +93,8 @@ typedef struct ft_query_options {
     int32_t max_k;        /* _MAX_K_ template argument; 0 = the reference's default         */
     int32_t method;       /* FT_METHOD_DEFAULT / FT_METHOD_FAST / FT_METHOD_PLAIN           */
     int32_t reserved[6];  /* [0] SFC seeding half-window (0 = k), [1] walk variant (0 = the
-                             tuned default), others 0                                      */
+                             tuned default, 2 the exact binary walk, 1 and 3 to 5 the 4-wide
+                             walk), others 0                                               */
 } ft_query_options;
 
 /* Statistics of the last query on a context (fallback rate, visits). */
@@ -441,7 +442,7 @@ ft_status ft_batch_query_stats(ft_context *ctx, ft_batch *batch, ft_query_stats 
 /* Blocking; they allocate scratch of their own.                                            */
 /* ---------------------------------------------------------------------------------- */
 typedef struct ft_tune_result {
-    int32_t walk_variant;  /* fast walk: 2 compact binary, 4 4-wide per-lane, 5 group walk  */
+    int32_t walk_variant;  /* fast walk: 2 exact binary, 4 4-wide                           */
     int32_t half_window;   /* SFC seeding half-window                                      */
     int32_t block_threads; /* 64 (two warps, 32-entry heap template) or 32 (one warp)      */
     int32_t sort_items;    /* build: keys per thread of a onesweep tile                    */

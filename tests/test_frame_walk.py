@@ -1,0 +1,189 @@
+"""The walks over the 32-bit records (knn, self-kNN, range) against the walks that use exact
+distances throughout: the reference traversal for kNN, the binary walk for range queries.
+
+The inputs sit where the frame's bounds or its rules could go wrong: fewer leaves than a
+bucket or a node holds, coordinates on a coarse lattice (ties), planes and lines, boxes far
+from the origin, spans at the frame's limits, tight clusters in a long box, the periodic wrap,
+and query points on, beyond and far outside the box.  Rows and counts must be equal bit for
+bit: both sides return the same neighbours by contract."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+import fasttree_b200 as ft  # noqa: E402
+
+NP = {"f32": np.float32, "f64": np.float64, "u32": np.uint32, "u64": np.uint64}
+CFGS = [("f32", "morton", False), ("f64", "ph", False), ("u32", "ph", True), ("u32", "ph", False),
+        ("u64", "ph", True), ("u64", "ph", False)]
+IDS = [f"{c}-{s}{'-per' if p else ''}" for c, s, p in CFGS]
+
+
+def box(coord):
+    """Side of the usual box in coordinate units."""
+    return {"f32": 1.0, "f64": 1.0, "u32": float(1 << 21), "u64": float(1 << 42)}[coord]
+
+
+def points(kind, n, coord, seed):
+    """(3, n) float64 in units of the usual box."""
+    rng = np.random.default_rng(seed)
+    p = rng.random((3, n))
+    if kind == "lattice":
+        p = np.floor(p * 8) / 8
+    elif kind == "plane":
+        p[2] = 0.25
+    elif kind == "line":
+        p[1:] = 0.5
+    elif kind == "clusters":  # two tight clusters at opposite corners of a long box
+        p = np.where(np.arange(n) % 2 == 0, 0.001 + 1e-5 * p, 0.999 - 1e-5 * p)
+    elif kind == "edges":  # around the periodic wrap
+        p = np.where(rng.random((3, n)) < 0.5, 1e-4 * p, 1.0 - 1e-4 * (1 - p))
+    return p
+
+
+def to_coord(p, coord):
+    if coord[0] == "u":
+        return [np.clip(np.floor(a * box(coord)), 0, box(coord) - 1).astype(NP[coord]) for a in p]
+    return [a.astype(NP[coord]) for a in p]
+
+
+def build(coord, sfc, per, xyz):
+    ctx = ft.Context(coord, sfc, periodic=per)
+    tree = ft.TreeSoA(ctx, len(xyz[0]))
+    ft.build_bvh(ctx, ft.particles(*xyz), tree)
+    return ctx, tree
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def same(a, b):
+    torch.cuda.synchronize()
+    return torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+def check_self(ctx, tree, ks):
+    for k in ks:
+        for excl in (True, False):
+            a = ft.self_knn_query(ctx, tree, k, exclude_self=excl, max_k=64, method="plain")
+            a = (a[0].clone(), a[1].clone())
+            assert same(a, ft.self_knn_query(ctx, tree, k, exclude_self=excl, max_k=64)), (k, excl)
+
+
+def check_points(ctx, tree, q, ks):
+    for k in ks:
+        a = ft.knn_query(ctx, tree, *q, k, max_k=256, method="plain")
+        a = (a[0].clone(), a[1].clone())
+        assert same(a, ft.knn_query(ctx, tree, *q, k, max_k=256)), k
+
+
+def check_range(ctx, tree, q, r0, r1, rows):
+    """The default walk, the one per query and the forced group counts against the binary walk."""
+    n = len(q[0])
+    lo, hi = (dev(np.full(n, r, NP[{0: "f32", 1: "f64", 2: "u32", 3: "u64"}[ctx.coord]])) for r in (r0, r1))
+    want = None
+    for walk in (1, 0, 3, 4):
+        ctx.set_range_walk(walk)
+        res = torch.full((n * max(rows, 1),), -1, dtype=torch.int32, device="cuda")
+        cnt = torch.zeros(n, dtype=torch.int32, device="cuda")
+        ft.range_query(ctx, tree, *q, lo, hi, rows, res, cnt)
+        torch.cuda.synchronize()
+        if want is None:
+            want = (res, cnt)
+        else:
+            assert torch.equal(cnt, want[1]) and torch.equal(res, want[0]), (walk, r0, r1, rows)
+    ctx.set_range_walk(0)
+
+
+@pytest.mark.parametrize("coord,sfc,per", CFGS, ids=IDS)
+def test_small_trees(coord, sfc, per):
+    """Around one bucket, one node and two levels of nodes."""
+    for n in (2, 3, 4, 7, 8, 9, 10, 16, 17, 31, 33, 65, 130):
+        xyz = to_coord(points("uniform", n, coord, n), coord)
+        ctx, tree = build(coord, sfc, per, xyz)
+        check_self(ctx, tree, (1, 8, 20))
+        q = [dev(a) for a in to_coord(points("uniform", 40, coord, 99), coord)]
+        check_points(ctx, tree, q, (1, 9))
+        for r in (0.0, 0.1 * box(coord), 2.0 * box(coord)):
+            check_range(ctx, tree, q, 0, min(r, 2.0**31 if coord == "u32" else 2.0**60), 5)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "lattice", "plane", "line", "clusters", "edges"])
+@pytest.mark.parametrize("coord,sfc,per", CFGS, ids=IDS)
+def test_shapes_of_the_box(coord, sfc, per, kind):
+    n = 6007
+    xyz = to_coord(points(kind, n, coord, 5), coord)
+    ctx, tree = build(coord, sfc, per, xyz)
+    check_self(ctx, tree, (1, 16, 33))
+    q = [dev(a) for a in to_coord(points("uniform", 700, coord, 6), coord)]
+    near = [dev(a[::7]) for a in xyz]
+    check_points(ctx, tree, q, (4, 40))
+    check_points(ctx, tree, near, (4,))
+    b = box(coord)
+    for r0, r1, rows in ((0, 1e-3 * b, 16), (0, 0.06 * b, 8), (0.03 * b, 0.08 * b, 8), (0, 0.4 * b, 0)):
+        check_range(ctx, tree, near, r0, r1, rows)
+    check_range(ctx, tree, q, 0, 0.1 * b, 30)
+
+
+@pytest.mark.parametrize("coord,span,lo", [("f64", 1e-10, 0.0), ("f64", 3e-9, 1.0), ("f64", 1e-3, 1e6), ("f64", 1e20, 0.0),
+                                           ("f64", 1e26, -5e25), ("f32", 1e-12, 0.0), ("f32", 1e-4, 0.0),
+                                           ("f32", 4.0, 1000.0), ("f32", 1e18, 0.0), ("u64", 100.0, 5.0),
+                                           ("u64", 2.0**13, 2.0**50), ("u64", 2.0**42, 0.0), ("u64", 2.0**45, 7.0),
+                                           ("u32", 50.0, 3.0), ("u32", 2.0**31, 9.0)])
+def test_spans_of_open_boxes(coord, span, lo):
+    """Spans inside, at and beyond what the frame serves; integers over few and many cells."""
+    rng = np.random.default_rng(8)
+    xyz = [(lo + span * rng.random(5000)).astype(NP[coord]) for _ in range(3)]
+    ctx, tree = build(coord, "ph", False, xyz)
+    check_self(ctx, tree, (1, 24))
+    out = [(lo + span * (a * 1.2 - 0.1)).clip(0 if coord[0] == "u" else None, None).astype(NP[coord])
+           for a in rng.random((3, 500))]
+    check_points(ctx, tree, [dev(a) for a in out], (3, 40))
+    for r in (0.02 * span, 0.3 * span):
+        check_range(ctx, tree, [dev(a) for a in out], 0, r, 12)
+
+
+@pytest.mark.parametrize("coord", ["f32", "f64", "u32", "u64"])
+def test_points_outside_the_box(coord):
+    """Query points beyond the frame walk the binary records; the others of their warp do not."""
+    rng = np.random.default_rng(3)
+    side = 1000.0
+    xyz = [(2000 + side * rng.random(4000)).astype(NP[coord]) for _ in range(3)]
+    ctx, tree = build(coord, "ph", False, xyz)
+    q = 2000 + side * rng.random((3, 640))
+    far = rng.random(640)
+    scale = np.select([far < 0.3, far < 0.4, far < 0.5, far < 0.6], [0.9, 1.1, 3.0, 1e5], 0.0)
+    q = q + np.sign(rng.random((3, 640)) - 0.3) * scale * side
+    q = [dev(a.clip(0 if coord[0] == "u" else None, None).astype(NP[coord])) for a in q]
+    check_points(ctx, tree, q, (1, 8, 40))
+    for r in (0.1 * side, 2.5 * side):
+        check_range(ctx, tree, q, 0, r, 20)
+
+
+def test_dense_parts_of_a_long_box():
+    """A cluster the frame cannot resolve (a cell of it holds hundreds of leaves): the exact walk
+    serves the tree, and rows stay equal."""
+    rng = np.random.default_rng(4)
+    p = rng.random((3, 3000)) * 1e-11 + 0.5
+    p = np.concatenate([p, rng.random((3, 50))], axis=1)
+    ctx, tree = build("f64", "morton", False, [a.copy() for a in p])
+    check_self(ctx, tree, (8, 33))
+    q = [dev(a[:400]) for a in p]
+    check_points(ctx, tree, q, (8,))
+    check_range(ctx, tree, q, 0, 3e-12, 10)
+
+
+@pytest.mark.parametrize("n", [1, 3, 33, 300, 3000, 25_000, 60_000])
+def test_query_counts_spread_over_warps(n):
+    """Small calls give a warp fewer queries: every split returns the rows of the full walk."""
+    xyz = to_coord(points("uniform", 70_000, "f32", 2), "f32")
+    ctx, tree = build("f32", "morton", False, xyz)
+    ids = torch.from_numpy(np.sort(np.random.default_rng(n).choice(70_000, n, replace=False)).astype(np.int32)).cuda()
+    a = ft.self_knn_query_subset(ctx, tree, ids, 12, method="plain")
+    a = (a[0].clone(), a[1].clone())
+    assert same(a, ft.self_knn_query_subset(ctx, tree, ids, 12))
