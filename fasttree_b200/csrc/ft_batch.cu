@@ -726,9 +726,13 @@ void batch_build_query_graph(Context &ctx, BatchImpl &b, const long long *in_off
         FT_CUDA(cudaStreamBeginCapture(b.cap_stream, cudaStreamCaptureModeRelaxed));
         cudaGraph_t graph = nullptr;
         try {
-            // the persistent launch is the default for the fast walk's k (measured faster than
-            // the launch sequence on the 4096-set workload); FT_METHOD_FAST names the sequence
-            const bool persistent = q.method == FT_METHOD_PERSISTENT || q.method == FT_METHOD_DEFAULT;
+            // The launch sequence is the default: a block that builds a whole set alone makes the
+            // largest sets the launch's tail (4096 sets, 65.6M points 224 against 208 ms; 512 sets
+            // 70 against 28 ms; 64 sets 31 against 5.2 ms; 4096 sets of at most 14K points 18
+            // against 5.4 ms).  126-bit keys build in one block a set either way, so there the
+            // queries overlap the builds of one persistent launch.
+            const bool persistent = q.method == FT_METHOD_PERSISTENT ||
+                                    (q.method == FT_METHOD_DEFAULT && ctx.opts.coord_type == U64);
             if (persistent && !model && k >= 1 && k <= 64) {
                 check_query_args(k, q);
                 PersistQuery pq;

@@ -623,7 +623,7 @@ class BatchedSets:
     def build_knn(self, set_offsets, pos_x, pos_y, pos_z, k: int, results, result_dists, exclude_self=True,
                   max_k: int = 32, method="default", id=None, is_ghost=None, stream=None):
         """build + self_knn as one CUDA graph (captured on the first call with these arrays, replayed
-        afterwards): "default" / "persistent", one persistent launch (k <= 64); "fast" / "plain",
+        afterwards): "persistent", one persistent launch (k <= 64; "default" too for u64); otherwise
         the launch sequence.  The arrays must stay alive and in place between calls: pass device
         tensors of the right dtype, which are used as they are."""
         off, xyz, ids, gh = self._inputs(set_offsets, pos_x, pos_y, pos_z, id, is_ghost)

@@ -84,9 +84,8 @@ typedef struct ft_tree {
 #define FT_METHOD_PLAIN   2 /* the reference traversal and heap alone                       */
 #define FT_METHOD_PERSISTENT 3 /* ft_batch_build_knn: one persistent launch builds every set
                                   and walks its queries (k <= 64; else its build, then the fast
-                                  walk) -- also what FT_METHOD_DEFAULT does there, while
-                                  FT_METHOD_FAST selects the launch sequence; other calls
-                                  treat it as FT_METHOD_FAST                                  */
+                                  walk) -- also what FT_METHOD_DEFAULT does there for 64-bit
+                                  integer positions; other calls treat it as FT_METHOD_FAST  */
 
 /* Per-query-call options (the reference's template parameters and dispatch choices). */
 typedef struct ft_query_options {
@@ -380,11 +379,11 @@ ft_status ft_batch_self_knn(ft_context *ctx, ft_batch *batch, int k, int exclude
 
 /* ft_batch_build + ft_batch_self_knn as one CUDA graph, captured on the first call with
  * these arguments and replayed by later calls with the same arguments (array contents may
- * change between calls).  With method FT_METHOD_DEFAULT or FT_METHOD_PERSISTENT (and k <= 64)
- * the graph holds one persistent kernel: each block builds whole sets (largest first, the
- * same trees as ft_batch_build), then its warps take chunks of queries of the finished sets;
- * tied queries are replayed by a second launch.  FT_METHOD_FAST / FT_METHOD_PLAIN select the
- * launch sequence (ft_batch_build, then ft_batch_self_knn).  Same rows either way.
+ * change between calls).  With method FT_METHOD_PERSISTENT (and k <= 64; for 64-bit integer
+ * positions FT_METHOD_DEFAULT too) the graph holds one persistent kernel: each block builds
+ * whole sets (largest first, the same trees as ft_batch_build), then its warps take chunks of
+ * queries of the finished sets; tied queries are replayed by a second launch.  Otherwise it
+ * holds the launch sequence (ft_batch_build, then ft_batch_self_knn).  Same rows either way.
  * Asynchronous. */
 ft_status ft_batch_build_knn(ft_context *ctx, ft_batch *batch, const int64_t *set_offsets, size_t num_sets,
                              size_t num_points, const void *x, const void *y, const void *z, const uint32_t *id,
