@@ -17,6 +17,7 @@
 #include "ft_common.cuh"
 #include "ft_internal.h"
 #include "ft_qtree.cuh"
+#include "ft_treelet.cuh"
 
 namespace ft {
 
@@ -66,53 +67,6 @@ template <class T> __global__ void __launch_bounds__(kBboxThreads) bbox_final_ke
         for (int d = 0; d < 6; ++d) out[d] = m[d];
 }
 
-// =========================================================================================
-// SFC keys (sfc_encode, src/hlbvh.hpp:357-423).  Internal key format: lo (and hi for the
-// 126-bit Peano-Hilbert key of 42-bit integer positions).  Also writes perm = iota.
-// =========================================================================================
-template <class T, int SFC>
-__global__ void __launch_bounds__(256) encode_kernel(const T *__restrict__ x, const T *__restrict__ y,
-                                                     const T *__restrict__ z, size_t n, const T *__restrict__ bbox,
-                                                     unsigned long long *klo, unsigned long long *khi, uint32_t *perm) {
-    using C = Coord<T>;
-    __shared__ uint8_t s_rot[48 * 8], s_sub[48 * 8];
-    __shared__ T       s_par[6]; // lo, inv per axis
-    for (int i = threadIdx.x; i < 48 * 8; i += blockDim.x) {
-        s_rot[i] = c_rot[i];
-        s_sub[i] = c_sub[i];
-    }
-    if constexpr (C::is_float)
-        if (threadIdx.x < 3) sfc_axis_params(bbox[2 * threadIdx.x], bbox[2 * threadIdx.x + 1], s_par[2 * threadIdx.x],
-                                             s_par[2 * threadIdx.x + 1]);
-    __syncthreads();
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        unsigned long long hi, lo;
-        encode_point<T, SFC>(x[i], y[i], z[i], s_par, s_rot, s_sub, hi, lo);
-        klo[i] = lo;
-        if (C::key_words == 2) khi[i] = hi;
-        perm[i] = (uint32_t)i;
-    }
-}
-
-// Key layout conversions between the reference's sfc_key and the internal (hi, lo) pair.
-// mode 0: Morton uint64; 1: {hs,is,ls} uint32; 2: {hs,is,ls} uint64.
-__global__ void keys_from_ref_kernel(const void *ref, size_t n, int mode, unsigned long long *klo,
-                                     unsigned long long *khi, uint32_t *perm) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        if (mode == 0) {
-            klo[i] = ((const unsigned long long *)ref)[i];
-        } else if (mode == 1) {
-            const uint32_t *w = (const uint32_t *)ref + 3 * i;
-            klo[i]            = ((unsigned long long)w[1] << 32) | w[2];
-        } else {
-            const unsigned long long *w = (const unsigned long long *)ref + 3 * i;
-            khi[i]                      = w[1];
-            klo[i]                      = w[2];
-        }
-        if (perm) perm[i] = (uint32_t)i;
-    }
-}
-
 __global__ void keys_to_ref_kernel(const unsigned long long *klo, const unsigned long long *khi, size_t n, int mode,
                                    void *ref) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -133,72 +87,67 @@ __global__ void keys_to_ref_kernel(const unsigned long long *klo, const unsigned
 }
 
 // =========================================================================================
-// Onesweep LSD radix sort of (key, perm): 8-bit digits, one upfront histogram pass for all
-// digit positions, then one pass per non-constant digit.  Each pass: a tile of 256 threads x
-// ITEMS keys ranks its keys with warp match-any histograms, publishes its digit counts,
-// resolves its global offsets by decoupled look-back over preceding tiles (tiles are
-// numbered by an atomic ticket so every predecessor is running or done), stages the tile
-// in shared memory in digit order and writes each digit run contiguously.  Stable, so equal
-// keys keep their original index order.
+// LSD radix sort of (64-bit key, 32-bit value) pairs: 8-bit digits, one upfront histogram of all
+// digit positions, then one onesweep pass per non-constant digit.  Each pass: a tile of 256
+// threads x ITEMS keys ranks its keys per warp (the lanes that share a digit are found with eight
+// ballots), publishes its digit counts, resolves its global offsets by decoupled look-back
+// over preceding tiles (tiles are numbered by an atomic ticket so every predecessor is running
+// or done), stages the tile in shared memory in digit order and writes each digit run
+// contiguously.  Stable, so equal keys keep their incoming order.
+//
+// A pass moves 24 bytes a key; what bounds it is the chain of steps of a tile.  Two-word keys and
+// the hardware's match instruction took 176 us a pass over 10M keys, the sort word alone (126-bit
+// keys: the high word; the low one rides with the packed points) and ballots 120 us: the match
+// costs an SM about 57 cycles a warp, the ballots some 10 in issue slots.  The encode kernel adds
+// its counts to the histograms with plain shared-memory atomics (a launch of its own with
+// match-aggregated counts took 495 us for 10M keys), and a constant digit's pass moves nothing
+// (83 us as a copy).
 // =========================================================================================
 static constexpr int kSortThreads = 256;
 static constexpr int kSortWarps   = kSortThreads / 32;
-// Tile tickets of build_bvh's sort: [0, 16) one per digit pass, [16, 32) the two-word
-// fallback's passes; [32] the fallback switch (a long run of equal high words).
-static constexpr int kTicketWords = 64;
+static constexpr int kSortDigits  = 8;
+// Words of TreeImpl::tile_counter: [0, 8) one tile ticket per pass; [32] build_bvh of 126-bit keys
+// met a run of equal high words too long to order in place.
+static constexpr int kTicketWords = 64, kLongRunWord = 32;
 static constexpr uint32_t kFlagAgg = 1u << 30, kFlagInc = 2u << 30, kFlagMask = 3u << 30,
                           kCountMask = (1u << 30) - 1u;
 
-// A onesweep tile: 256 threads x ITEMS keys (ITEMS 0: the default, 8; the autotuner chose 8
-// on every shape measured -- 100K float64 Morton, 10M and 50M uint64 Peano-Hilbert points --
-// where the larger tiles' registers leave one block per SM: 10M points, untuned 12-key tiles
-// 2.83 ms against 2.15 ms).  The build's sort takes the tile the autotuner chose for the shape
-// (sort_items); every tile size gives the same order.
-template <int W, int ITEMS = 0> struct SortCfg {
-    static constexpr int items = ITEMS ? ITEMS : 8;
-    static constexpr int tile  = kSortThreads * items;
-    static constexpr size_t smem = (size_t)tile * (8 * W + 4) + (size_t)kSortWarps * 256 * 4;
+// A onesweep tile: 256 threads x ITEMS keys (8 by default; the autotuner's choice for a shape
+// otherwise; every tile size gives the same order).
+template <int ITEMS> struct SortCfg {
+    static constexpr int    tile = kSortThreads * ITEMS;
+    static constexpr size_t smem = (size_t)tile * 12 + (size_t)kSortWarps * 256 * 4;
 };
-static constexpr int kSortItemsMin = 8; // the smallest tile sizes the look-back scratch
+static constexpr int kSortItems = 8; // the smallest tile: it sizes the look-back scratch
 
-// Digit histograms of digit positions [d0, d0 + ND) (ND = 8 * W by default: every digit).
-// enable: null, or a device word whose 0 makes the launch a no-op.
-template <int W, int ND = 8 * W>
-__global__ void __launch_bounds__(256) radix_hist_kernel(const unsigned long long *__restrict__ klo,
-                                                         const unsigned long long *__restrict__ khi, size_t n,
-                                                         uint32_t *hist, int d0 = 0,
-                                                         const uint32_t *enable = nullptr) {
-    constexpr int D = ND;
-    if (enable && *enable == 0u) return;
-    __shared__ uint32_t s[D * 256];
-    for (int i = threadIdx.x; i < D * 256; i += blockDim.x) s[i] = 0;
-    __syncthreads();
-    const unsigned lane = threadIdx.x & 31;
-    const size_t   stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t base = blockIdx.x * (size_t)blockDim.x; base < n; base += stride) {
-        size_t i     = base + threadIdx.x;
-        bool   valid = i < n;
-        unsigned long long w[2] = {valid ? klo[i] : 0ull, (W == 2 && valid) ? khi[i] : 0ull};
-        unsigned active = __ballot_sync(0xffffffffu, valid);
+// The pairs' two buffers.  A constant digit's pass moves nothing, so the buffer that holds them
+// follows from the passes that ran (sort_parity, ft_treelet.cuh).
+struct SortPairs {
+    unsigned long long *k[2];
+    uint32_t           *v[2];
+};
+FT_D void hist_add(uint32_t *s, unsigned long long key) {
 #pragma unroll
-        for (int j = 0; j < D; ++j) {
-            const int d     = d0 + j;
-            unsigned  digit = (unsigned)(w[d >> 3] >> (8 * (d & 7))) & 255u;
-            unsigned peers = __match_any_sync(0xffffffffu, valid ? digit : 256u + lane);
-            if (valid && lane == (unsigned)(__ffs(peers) - 1)) atomicAdd(&s[j * 256 + digit], __popc(peers & active));
-        }
-    }
+    for (int d = 0; d < kSortDigits; ++d) atomicAdd(&s[d * 256 + ((unsigned)(key >> (8 * d)) & 255u)], 1u);
+}
+
+// Digit histograms of every digit position (hist zero at launch).
+__global__ void __launch_bounds__(256) radix_hist_kernel(const unsigned long long *__restrict__ keys, size_t n,
+                                                         uint32_t *hist) {
+    __shared__ uint32_t s[kSortDigits * 256];
+    for (int i = threadIdx.x; i < kSortDigits * 256; i += blockDim.x) s[i] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < D * 256; i += blockDim.x)
-        if (s[i]) atomicAdd(&hist[d0 * 256 + i], s[i]);
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        hist_add(s, keys[i]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSortDigits * 256; i += blockDim.x)
+        if (s[i]) atomicAdd(&hist[i], s[i]);
 }
 
 // Exclusive offsets per digit position; skip[d] = 1 when one digit value holds every key.
-// enable: as radix_hist_kernel's.
-__global__ void radix_scan_kernel(uint32_t *hist, size_t n, uint32_t *skip, const uint32_t *enable = nullptr) {
+__global__ void radix_scan_kernel(uint32_t *hist, size_t n, uint32_t *skip) {
     __shared__ uint32_t s[256];
     __shared__ int      s_full;
-    if (enable && *enable == 0u) return;
     const int d = blockIdx.x, t = threadIdx.x;
     uint32_t  c = hist[d * 256 + t];
     if (t == 0) s_full = 0;
@@ -223,30 +172,36 @@ FT_D uint32_t ld_volatile(const uint32_t *p) {
 }
 FT_D void st_volatile(uint32_t *p, uint32_t v) { asm volatile("st.volatile.global.u32 [%0], %1;" ::"l"(p), "r"(v)); }
 
-// One onesweep pass over every tile.  The grid is persistent (at most the CTAs resident at
-// once): each CTA takes tiles by ticket until none are left, so a launch whose pass turns out
-// to have nothing to do costs one wave.  Device-side switches keep the host out of the loop:
-//  * enable (null or a device word): 0 makes the whole pass a no-op (passes of the two-word
-//    fallback, which only runs when a long run of equal high words was found);
-//  * skip (null or a device word): 1 when one digit value holds every key -- the pass then
-//    copies its tiles unchanged, so the ping-pong order the host planned still holds.
-// (8-key tiles are compiled for three resident blocks: 80 registers, no spills, 24 warps per SM)
-template <int W, int IT = 0>
-__global__ void __launch_bounds__(kSortThreads, (SortCfg<W, IT>::items <= 8 ? 3 : 1))
-    onesweep_kernel(const unsigned long long *__restrict__ in_lo, const unsigned long long *__restrict__ in_hi,
-                    const uint32_t *__restrict__ in_v, unsigned long long *__restrict__ out_lo,
-                    unsigned long long *__restrict__ out_hi, uint32_t *__restrict__ out_v, size_t n, size_t num_tiles,
-                    int word, int shift, const uint32_t *__restrict__ offsets, uint32_t *lookback,
-                    uint32_t *tile_counter, const uint32_t *enable, const uint32_t *skip, uint32_t *status) {
-    using Cfg           = SortCfg<W, IT>;
-    constexpr int ITEMS = Cfg::items;
-    constexpr int TILE  = Cfg::tile;
-    if (enable && *enable == 0u) return; // grid-uniform
-    const bool copy = skip && *skip != 0u;
+// The lanes of the warp whose digit equals this lane's, among the lanes with `valid`.
+FT_D unsigned digit_peers(uint32_t digit, bool valid) {
+    unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool     bit = (digit >> b) & 1u;
+        const unsigned has = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? has : ~has;
+    }
+    return peers;
+}
+
+// One onesweep pass.  The grid is persistent (at most the CTAs resident at once): each CTA takes
+// tiles by ticket until none are left.  skip: null, or the passes' skip words (then a pass of
+// a constant digit returns at once).
+template <int ITEMS>
+__global__ void __launch_bounds__(kSortThreads, (ITEMS <= 8 ? 4 : ITEMS <= 12 ? 3 : 2))
+    onesweep_kernel(const SortPairs pairs, size_t n, size_t num_tiles, int pass, int shift,
+                    const uint32_t *__restrict__ offsets, uint32_t *lookback, uint32_t *tile_counter,
+                    const uint32_t *__restrict__ skip, uint32_t *status) {
+    constexpr int TILE = SortCfg<ITEMS>::tile;
+    if (skip && skip[pass]) return; // grid-uniform
+    const int from = sort_parity(skip, pass);
+    const unsigned long long *__restrict__ in_k = pairs.k[from];
+    const uint32_t *__restrict__ in_v           = pairs.v[from];
+    unsigned long long *__restrict__ out_k      = pairs.k[from ^ 1];
+    uint32_t *__restrict__ out_v                = pairs.v[from ^ 1];
     extern __shared__ __align__(16) unsigned char smem[];
-    unsigned long long *s_lo = reinterpret_cast<unsigned long long *>(smem);
-    unsigned long long *s_hi = s_lo + TILE; // only used when W == 2
-    uint32_t           *s_v  = reinterpret_cast<uint32_t *>(s_lo + (size_t)TILE * W);
+    unsigned long long *s_k  = reinterpret_cast<unsigned long long *>(smem);
+    uint32_t           *s_v  = reinterpret_cast<uint32_t *>(s_k + TILE);
     uint32_t           *s_wh = s_v + TILE; // [warp][256]
     __shared__ uint32_t s_tile_excl[256];
     __shared__ uint32_t s_base[256];
@@ -263,37 +218,23 @@ __global__ void __launch_bounds__(kSortThreads, (SortCfg<W, IT>::items <= 8 ? 3 
         if (tile >= num_tiles) break; // grid-uniform per CTA
         const size_t base = tile * (size_t)TILE;
 
-        if (copy) { // constant digit: the tile moves unchanged
-            const size_t end = min(base + (size_t)TILE, n);
-            for (size_t pos = base + tid; pos < end; pos += kSortThreads) {
-                out_lo[pos] = in_lo[pos];
-                if (W == 2) out_hi[pos] = in_hi[pos];
-                out_v[pos] = in_v[pos];
-            }
-            __syncthreads();
-            continue;
-        }
-
-        unsigned long long klo[ITEMS], khi[ITEMS];
-        uint32_t           val[ITEMS], dig[ITEMS], rank[ITEMS];
+        unsigned long long key[ITEMS];
+        uint32_t           val[ITEMS], rank[ITEMS];
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
-            size_t pos   = base + (size_t)warp * 32 * ITEMS + (size_t)i * 32 + lane;
-            bool   valid = pos < n;
-            klo[i]       = valid ? in_lo[pos] : 0ull;
-            khi[i]       = (W == 2 && valid) ? in_hi[pos] : 0ull;
-            val[i]       = valid ? in_v[pos] : 0u;
-            unsigned long long w = (W == 2 && word == 1) ? khi[i] : klo[i];
-            dig[i]       = valid ? (uint32_t)(w >> shift) & 255u : 256u + lane;
+            const size_t pos = base + (size_t)warp * 32 * ITEMS + (size_t)i * 32 + lane;
+            key[i]           = pos < n ? in_k[pos] : 0ull;
+            val[i]           = pos < n ? in_v[pos] : 0u;
         }
         uint32_t *wh = s_wh + warp * 256;
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
-            unsigned peers  = __match_any_sync(0xffffffffu, dig[i]);
-            bool     valid  = dig[i] < 256u;
-            uint32_t before = valid ? wh[dig[i]] : 0u;
+            const bool     valid  = base + (size_t)warp * 32 * ITEMS + (size_t)i * 32 + lane < n;
+            const uint32_t d      = (uint32_t)(key[i] >> shift) & 255u;
+            const unsigned peers  = digit_peers(d, valid);
+            const uint32_t before = valid ? wh[d] : 0u;
             __syncwarp();
-            if (valid && lane == __ffs(peers) - 1) wh[dig[i]] = before + __popc(peers);
+            if (valid && (peers & lt_mask) == 0u) wh[d] = before + __popc(peers);
             __syncwarp();
             rank[i] = before + __popc(peers & lt_mask);
         }
@@ -303,17 +244,20 @@ __global__ void __launch_bounds__(kSortThreads, (SortCfg<W, IT>::items <= 8 ? 3 
         uint32_t run = 0;
 #pragma unroll
         for (int w = 0; w < kSortWarps; ++w) {
-            uint32_t c          = s_wh[w * 256 + tid];
+            const uint32_t c    = s_wh[w * 256 + tid];
             s_wh[w * 256 + tid] = run;
             run += c;
         }
         const uint32_t tile_count = run;
+        // (published at once: the next tiles' look-back may be waiting for it)
+        uint32_t *lb = lookback + tile * 256;
+        st_volatile(lb + tid, (tile == 0 ? kFlagInc : kFlagAgg) | tile_count);
 
         // exclusive scan of tile counts over digits (block scan, 256 threads)
         uint32_t incl = tile_count;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
             if (lane >= off) incl += v;
         }
         if (lane == 31) s_wsum[warp] = incl;
@@ -321,15 +265,23 @@ __global__ void __launch_bounds__(kSortThreads, (SortCfg<W, IT>::items <= 8 ? 3 
         uint32_t wpre = 0;
         for (int w = 0; w < warp; ++w) wpre += s_wsum[w];
         s_tile_excl[tid] = wpre + incl - tile_count;
+        __syncthreads();
+
+        // stage the tile in digit order
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            if (base + (size_t)warp * 32 * ITEMS + (size_t)i * 32 + lane < n) {
+                const uint32_t d  = (uint32_t)(key[i] >> shift) & 255u;
+                const uint32_t lp = s_tile_excl[d] + s_wh[warp * 256 + d] + rank[i];
+                s_k[lp]           = key[i];
+                s_v[lp]           = val[i];
+            }
+        }
 
         // decoupled look-back for digit tid (every earlier tile is held by a running CTA or
         // done, since tickets are taken in order and a CTA finishes its tile first)
-        uint32_t *lb     = lookback + tile * 256;
-        uint32_t  prefix = 0;
-        if (tile == 0) {
-            st_volatile(lb + tid, kFlagInc | tile_count);
-        } else {
-            st_volatile(lb + tid, kFlagAgg | tile_count);
+        uint32_t prefix = 0;
+        if (tile > 0) {
             for (long long j = (long long)tile - 1; j >= 0; --j) {
                 uint32_t sv;
                 int      spins = 0;
@@ -348,84 +300,402 @@ __global__ void __launch_bounds__(kSortThreads, (SortCfg<W, IT>::items <= 8 ? 3 
             }
             st_volatile(lb + tid, kFlagInc | (prefix + tile_count));
         }
-        s_base[tid] = offsets[tid] + prefix;
-        __syncthreads();
-
-        // stage the tile in digit order
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-            if (dig[i] < 256u) {
-                uint32_t lp = s_tile_excl[dig[i]] + s_wh[warp * 256 + dig[i]] + rank[i];
-                s_lo[lp]    = klo[i];
-                if (W == 2) s_hi[lp] = khi[i];
-                s_v[lp] = val[i];
-            }
-        }
+        s_base[tid] = offsets[tid] + prefix - s_tile_excl[tid];
         __syncthreads();
         const int tile_n = (int)min((size_t)TILE, n - base);
         for (int j = tid; j < tile_n; j += kSortThreads) {
-            unsigned long long lo = s_lo[j];
-            unsigned long long hi = (W == 2) ? s_hi[j] : 0ull;
-            unsigned long long w  = (W == 2 && word == 1) ? hi : lo;
-            uint32_t           d  = (uint32_t)(w >> shift) & 255u;
-            size_t             gp = (size_t)s_base[d] + (size_t)(j - (int)s_tile_excl[d]);
+            const unsigned long long k  = s_k[j];
+            const uint32_t           d  = (uint32_t)(k >> shift) & 255u;
+            const uint32_t           gp = s_base[d] + (uint32_t)j;
             if (gp >= n) { // only reachable after a failed look-back; never write out of bounds
                 atomicOr(status, STATUS_SPIN_LIMIT);
                 continue;
             }
-            out_lo[gp]             = lo;
-            if (W == 2) out_hi[gp] = hi;
-            out_v[gp]              = s_v[j];
+            out_k[gp] = k;
+            out_v[gp] = s_v[j];
         }
         __syncthreads(); // the tile's shared memory is free for the next ticket
     }
 }
 
 // =========================================================================================
-// Leaf gather (src/hlbvh.hpp:2266-2279): leaf slot n-1+i <- input point perm[i].
+// SFC keys (sfc_encode, src/hlbvh.hpp:357-423).
 // =========================================================================================
-template <class T>
-__global__ void gather_kernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ z,
-                              const uint32_t *__restrict__ perm, size_t n, const uint32_t *__restrict__ id,
-                              const int8_t *__restrict__ ghost, T *mnx, T *mxx, T *mny, T *mxy, T *mnz, T *mxz,
-                              uint32_t *tid_out, int8_t *ghost_out, int32_t *orig_out) {
+// Peano-Hilbert state tables of two levels at once: state and six bits of the position (the two
+// bits of x, then of y, then of z) -> next state << 6 | the two levels' key digits.  Half the
+// chain of dependent look-ups of the one-level tables.
+static constexpr int kPh2Entries = 48 * 64;
+FT_D void ph2_fill(uint16_t *t) { // (every thread of the block; a barrier follows)
+    for (int i = threadIdx.x; i < kPh2Entries; i += blockDim.x) {
+        const int st = i >> 6, x = (i >> 4) & 3, y = (i >> 2) & 3, z = i & 3;
+        const int p1 = ((x >> 1) << 2) | ((y >> 1) << 1) | (z >> 1), p0 = ((x & 1) << 2) | ((y & 1) << 1) | (z & 1);
+        const int r  = c_rot[st * 8 + p1];
+        t[i]         = (uint16_t)(((int)c_rot[r * 8 + p0] << 6) | (c_sub[st * 8 + p1] << 3) | c_sub[r * 8 + p0]);
+    }
+}
+// ph_key (ft_build_dev.cuh) by pairs of levels, after one plain level when their number is odd.
+template <int B>
+FT_D void ph2_key(unsigned long long px, unsigned long long py, unsigned long long pz, const uint16_t *t,
+                  unsigned long long &hi, unsigned long long &lo) {
+    unsigned long long h = 0, l = 0;
+    unsigned           st = 0;
+    if constexpr (B & 1) {
+        const unsigned p = (unsigned)((((px >> (B - 1)) & 1ull) << 2) | (((py >> (B - 1)) & 1ull) << 1) |
+                                      ((pz >> (B - 1)) & 1ull));
+        l  = c_sub[p];
+        st = c_rot[p];
+    }
+#pragma unroll 7
+    for (int b = (B & ~1) - 2; b >= 0; b -= 2) {
+        const unsigned p = ((unsigned)(px >> b) & 3u) << 4 | ((unsigned)(py >> b) & 3u) << 2 | ((unsigned)(pz >> b) & 3u);
+        const unsigned e = t[st * 64u + p];
+        h                = (h << 6) | (l >> 58);
+        l                = (l << 6) | (e & 63u);
+        st               = e >> 6;
+    }
+    hi = h;
+    lo = l;
+}
+template <class T, int SFC>
+FT_D void encode_point2(T x, T y, T z, const T *par, const uint16_t *t, unsigned long long &hi, unsigned long long &lo) {
+    using C = Coord<T>;
+    if constexpr (!C::is_float) {
+        const unsigned long long mask = (1ull << C::bits) - 1ull;
+        ph2_key<C::bits>((unsigned long long)x & mask, (unsigned long long)y & mask, (unsigned long long)z & mask, t, hi,
+                         lo);
+    } else if constexpr (SFC == MORTON) {
+        encode_point<T, SFC>(x, y, z, par, nullptr, nullptr, hi, lo);
+    } else {
+        unsigned long long c[3];
+        sfc_cells<T, SFC>(x, y, z, par, c);
+        ph2_key<21>(c[0], c[1], c[2], t, hi, lo);
+    }
+}
+// The sort word of a key: the high word of 126-bit keys (their low word rides in the packed point).
+template <class T> FT_D unsigned long long sort_word(unsigned long long hi, unsigned long long lo) {
+    return Coord<T>::key_words == 2 ? hi : lo;
+}
+
+// Keys of n points.  klo / khi: null, or the key words; with `pack`, the build's form: the sort
+// word in key, the input index in perm, the points packed, and the sort word's digit
+// histograms added to hist (zero at launch).
+template <class T, int SFC>
+__global__ void __launch_bounds__(256) encode_kernel(const T *__restrict__ x, const T *__restrict__ y,
+                                                     const T *__restrict__ z, size_t n, const T *__restrict__ bbox,
+                                                     unsigned long long *klo, unsigned long long *khi,
+                                                     unsigned long long *key, uint32_t *perm, PackedPoint<T> *pack,
+                                                     uint32_t *hist) {
+    using C = Coord<T>;
+    __shared__ uint16_t s_ph[SFC == PEANO_HILBERT ? kPh2Entries : 1];
+    __shared__ uint32_t s_hist[kSortDigits * 256];
+    __shared__ T        s_par[6]; // lo, inv per axis
+    if constexpr (SFC == PEANO_HILBERT) ph2_fill(s_ph);
+    for (int i = threadIdx.x; i < kSortDigits * 256; i += blockDim.x) s_hist[i] = 0;
+    if constexpr (C::is_float)
+        if (threadIdx.x < 3) sfc_axis_params(bbox[2 * threadIdx.x], bbox[2 * threadIdx.x + 1], s_par[2 * threadIdx.x],
+                                             s_par[2 * threadIdx.x + 1]);
+    __syncthreads();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        uint32_t src  = perm[i];
-        size_t   leaf = i + n - 1;
-        T        a = x[src], b = y[src], c = z[src];
-        mnx[leaf] = a;
-        mxx[leaf] = a;
-        mny[leaf] = b;
-        mxy[leaf] = b;
-        mnz[leaf] = c;
-        mxz[leaf] = c;
-        tid_out[leaf]   = id ? id[src] : src;
-        ghost_out[leaf] = ghost ? ghost[src] : (int8_t)0;
-        orig_out[leaf]  = (int32_t)src;
+        const T            a = x[i], b = y[i], c = z[i];
+        unsigned long long hi, lo;
+        encode_point2<T, SFC>(a, b, c, s_par, s_ph, hi, lo);
+        if (pack) {
+            const unsigned long long w = sort_word<T>(hi, lo);
+            key[i]                     = w;
+            perm[i]                    = (uint32_t)i;
+            PackedPoint<T> p{a, b, c, T(0)};
+            if constexpr (C::key_words == 2) p.pad = lo;
+            pack[i] = p;
+            hist_add(s_hist, w);
+        } else {
+            klo[i] = lo;
+            if (C::key_words == 2) khi[i] = hi;
+        }
+    }
+    if (!pack) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSortDigits * 256; i += blockDim.x)
+        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
+}
+
+// Key layout conversions between the reference's sfc_key and the internal (hi, lo) pair.
+// mode 0: Morton uint64; 1: {hs,is,ls} uint32; 2: {hs,is,ls} uint64.
+FT_D void key_from_ref(const void *ref, size_t i, int mode, unsigned long long &hi, unsigned long long &lo) {
+    hi = 0;
+    if (mode == 0) {
+        lo = ((const unsigned long long *)ref)[i];
+    } else if (mode == 1) {
+        const uint32_t *w = (const uint32_t *)ref + 3 * i;
+        lo                = ((unsigned long long)w[1] << 32) | w[2];
+    } else {
+        const unsigned long long *w = (const unsigned long long *)ref + 3 * i;
+        hi                          = w[1];
+        lo                          = w[2];
+    }
+}
+__global__ void keys_from_ref_kernel(const void *ref, size_t n, int mode, unsigned long long *klo,
+                                     unsigned long long *khi) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        unsigned long long hi, lo;
+        key_from_ref(ref, i, mode, hi, lo);
+        klo[i] = lo;
+        if (mode == 2) khi[i] = hi;
     }
 }
 
-// Refit-only update: leaf slot n-1+i takes the new position of the point it already holds
-// (input index orig_idx[n-1+i], or i itself when the positions come in leaf order).  An
-// index outside [0, n) leaves the slot unchanged and sets the bad-input status bit.
+// The build's form of caller keys (see encode_kernel).
 template <class T>
-__global__ void refit_gather_kernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ z,
-                                    const int32_t *__restrict__ orig, size_t n, T *mnx, T *mxx, T *mny, T *mxy,
-                                    T *mnz, T *mxz, uint32_t *status) {
+__global__ void __launch_bounds__(256) pack_ref_kernel(const T *__restrict__ x, const T *__restrict__ y,
+                                                       const T *__restrict__ z, size_t n, const void *ref, int mode,
+                                                       unsigned long long *key, uint32_t *perm, PackedPoint<T> *pack,
+                                                       uint32_t *hist) {
+    __shared__ uint32_t s_hist[kSortDigits * 256];
+    for (int i = threadIdx.x; i < kSortDigits * 256; i += blockDim.x) s_hist[i] = 0;
+    __syncthreads();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t  leaf = i + n - 1;
-        const int64_t src  = orig ? (int64_t)orig[leaf] : (int64_t)i;
-        if (src < 0 || src >= (int64_t)n) {
-            atomicOr(status, STATUS_BAD_INPUT);
+        unsigned long long hi, lo;
+        key_from_ref(ref, i, mode, hi, lo);
+        const unsigned long long w = sort_word<T>(hi, lo);
+        key[i]                     = w;
+        perm[i]                    = (uint32_t)i;
+        PackedPoint<T> p{x[i], y[i], z[i], T(0)};
+        if constexpr (Coord<T>::key_words == 2) p.pad = lo;
+        pack[i] = p;
+        hist_add(s_hist, w);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSortDigits * 256; i += blockDim.x)
+        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
+}
+
+// =========================================================================================
+// Box, keys and sort of a small set in one block: for at most kFrontMax points the launches of
+// the steps above (two for the box, keys, histogram scan, eight passes) are all latency.  Keys and
+// values stay in registers between the passes, which rank per warp like onesweep_kernel and
+// scatter in shared memory.  4K float points: some 95 us of kernels in 13 launches become 41 us
+// (67 us with all eight passes).
+// =========================================================================================
+static constexpr int kFrontThreads = 1024, kFrontItems = 8, kFrontMax = kFrontThreads * kFrontItems;
+static constexpr int kFrontRun     = 16;
+template <class T> struct alignas(16) FrontShared {
+    unsigned long long k[kFrontMax];
+    uint32_t           v[kFrontMax];
+    uint32_t           wh[256 * 33]; // [digit][warp], a word of padding per digit
+    uint32_t           tot[256];
+    uint16_t           ph[kPh2Entries];
+    T                  red[32][6], par[6];
+    int                same;
+};
+
+// box: the points' box goes to bbox (6), or behind it (6 .. 11) when bbox holds the caller's.
+template <class T, int SFC>
+__global__ void __launch_bounds__(kFrontThreads, 1)
+    front_kernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ z, int n, int caller_box,
+                 T *bbox, unsigned long long *key_out, uint32_t *perm, PackedPoint<T> *pack) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    FrontShared<T> &s   = *reinterpret_cast<FrontShared<T> *>(smem_raw);
+    const int       tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned  lt  = (1u << lane) - 1u, FULL = 0xffffffffu;
+    const int       items = (n + kFrontThreads - 1) / kFrontThreads;
+    if constexpr (SFC == PEANO_HILBERT) ph2_fill(s.ph);
+    {
+        T m[6];
+        bb_identity(m);
+        for (int i = tid; i < n; i += kFrontThreads) {
+            T v[6] = {x[i], x[i], y[i], y[i], z[i], z[i]};
+            bb_fold(m, v);
+        }
+        auto fold_warp = [&]() {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                T o[6];
+#pragma unroll
+                for (int d = 0; d < 6; ++d) o[d] = __shfl_down_sync(FULL, m[d], off);
+                bb_fold(m, o);
+            }
+        };
+        fold_warp();
+        if (lane == 0)
+#pragma unroll
+            for (int d = 0; d < 6; ++d) s.red[warp][d] = m[d];
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int d = 0; d < 6; ++d) m[d] = s.red[lane][d];
+            fold_warp();
+            if (lane == 0) {
+#pragma unroll
+                for (int d = 0; d < 6; ++d) bbox[(caller_box ? 6 : 0) + d] = m[d];
+                if constexpr (Coord<T>::is_float) {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const T lo = caller_box ? bbox[2 * d] : m[2 * d], hi = caller_box ? bbox[2 * d + 1] : m[2 * d + 1];
+                        sfc_axis_params(lo, hi, s.par[2 * d], s.par[2 * d + 1]);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    unsigned long long key[kFrontItems];
+    uint32_t           val[kFrontItems], rank[kFrontItems];
+    const int          first = warp * 32 * items + lane; // this thread's pairs: first + 32 i
+#pragma unroll
+    for (int i = 0; i < kFrontItems; ++i) {
+        const int e = first + 32 * i;
+        key[i]      = 0ull;
+        val[i]      = (uint32_t)e;
+        if (i < items && e < n) {
+            const T            a = x[e], b = y[e], c = z[e];
+            unsigned long long hi, lo;
+            encode_point2<T, SFC>(a, b, c, s.par, s.ph, hi, lo);
+            key[i] = sort_word<T>(hi, lo);
+            PackedPoint<T> p{a, b, c, T(0)};
+            if constexpr (Coord<T>::key_words == 2) p.pad = lo;
+            pack[e] = p;
+        }
+    }
+    // The upper half of the word first: few points share it, and a thread orders such a run of at
+    // most kFrontRun pairs in place.  A longer run takes the passes over the whole word from the
+    // current order (stable, so equal words keep their input order either way).
+    bool whole = false; // block-uniform
+    for (int d = kSortDigits / 2;; ++d) {
+        if (d == kSortDigits) {
+            if (whole) break;
+            if (tid == 0) s.same = 0;
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < kFrontItems; ++i) {
+                const int e = first + 32 * i;
+                if (i < items && e < n) {
+                    s.k[e] = key[i];
+                    s.v[e] = val[i];
+                }
+            }
+            __syncthreads();
+            for (int e = tid; e + 1 < n; e += kFrontThreads) { // run starts
+                const uint32_t up = (uint32_t)(s.k[e] >> 32);
+                if ((uint32_t)(s.k[e + 1] >> 32) != up || (e > 0 && (uint32_t)(s.k[e - 1] >> 32) == up)) continue;
+                int f = e + 2;
+                while (f < n && f - e <= kFrontRun && (uint32_t)(s.k[f] >> 32) == up) ++f;
+                if (f - e > kFrontRun) {
+                    s.same = 1;
+                    continue;
+                }
+                for (int j = e + 1; j < f; ++j) {
+                    const unsigned long long kj = s.k[j];
+                    const uint32_t           vj = s.v[j];
+                    int                      m  = j;
+                    for (; m > e && s.k[m - 1] > kj; --m) {
+                        s.k[m] = s.k[m - 1];
+                        s.v[m] = s.v[m - 1];
+                    }
+                    s.k[m] = kj;
+                    s.v[m] = vj;
+                }
+            }
+            __syncthreads();
+            whole = s.same != 0;
+#pragma unroll
+            for (int i = 0; i < kFrontItems; ++i) {
+                const int e = first + 32 * i;
+                if (i < items && e < n) {
+                    key[i] = s.k[e];
+                    val[i] = s.v[e];
+                }
+            }
+            __syncthreads();
+            if (!whole) break;
+            d = 0;
+        }
+        const int shift = 8 * d;
+        for (int i = tid; i < 256 * 33; i += kFrontThreads) s.wh[i] = 0;
+        if (tid == 0) s.same = 0;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kFrontItems; ++i) {
+            if (i < items) { // block-uniform
+                const bool     valid  = first + 32 * i < n;
+                const uint32_t g      = (uint32_t)(key[i] >> shift) & 255u;
+                const unsigned peers  = digit_peers(g, valid);
+                const uint32_t before = valid ? s.wh[g * 33 + warp] : 0u;
+                __syncwarp();
+                if (valid && (peers & lt) == 0u) s.wh[g * 33 + warp] = before + __popc(peers);
+                __syncwarp();
+                rank[i] = before + __popc(peers & lt);
+            }
+        }
+        __syncthreads();
+        // per digit: exclusive prefixes over the warps (a lane each) and the total
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int      g    = warp * 8 + j;
+            const uint32_t c    = s.wh[g * 33 + lane];
+            uint32_t       incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += u;
+            }
+            s.wh[g * 33 + lane] = incl - c;
+            if (lane == 31) {
+                s.tot[g] = incl;
+                if (incl == (uint32_t)n) s.same = 1;
+            }
+        }
+        __syncthreads();
+        if (s.same) { // one digit value holds every key (block-uniform)
+            __syncthreads();
             continue;
         }
-        const T a = x[src], b = y[src], c = z[src];
-        mnx[leaf] = a;
-        mxx[leaf] = a;
-        mny[leaf] = b;
-        mxy[leaf] = b;
-        mnz[leaf] = c;
-        mxz[leaf] = c;
+        if (warp == 0) { // exclusive prefixes of the totals
+            uint32_t v[8], sum = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                v[i] = s.tot[lane * 8 + i];
+                sum += v[i];
+            }
+            uint32_t incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += u;
+            }
+            uint32_t run = incl - sum;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                s.tot[lane * 8 + i] = run;
+                run += v[i];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kFrontItems; ++i) {
+            if (i < items && first + 32 * i < n) {
+                const uint32_t g  = (uint32_t)(key[i] >> shift) & 255u;
+                const uint32_t at = s.tot[g] + s.wh[g * 33 + warp] + rank[i];
+                s.k[at]           = key[i];
+                s.v[at]           = val[i];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kFrontItems; ++i) {
+            const int e = first + 32 * i;
+            if (i < items && e < n) {
+                key[i] = s.k[e];
+                val[i] = s.v[e];
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < kFrontItems; ++i) {
+        const int e = first + 32 * i;
+        if (i < items && e < n) {
+            key_out[e] = key[i];
+            perm[e]    = val[i];
+        }
     }
 }
 
@@ -442,93 +712,6 @@ __global__ void leaf_init_kernel(const T *sx, const T *sy, const T *sz, size_t n
         if (sid) tid_out[leaf] = sid[i];
         if (sghost) ghost_out[leaf] = sghost[i];
         if (sorig) orig_out[leaf] = sorig[i];
-    }
-}
-
-// =========================================================================================
-// Karras 2012 radix-tree topology (src/hlbvh.hpp:852-903).  delta() is the common prefix
-// length of two sorted keys (get_common_prefix_length, 283-340), with the index tie-break
-// for equal keys.
-// =========================================================================================
-template <int KIND>
-__global__ void __launch_bounds__(256) karras_kernel(const unsigned long long *__restrict__ klo,
-                                                     const unsigned long long *__restrict__ khi, int n,
-                                                     int32_t *left, int32_t *right, int32_t *parent,
-                                                     int32_t *leaves) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x)
-        karras_node<KIND>(klo, khi, n, i, left, right, parent, leaves);
-}
-
-// =========================================================================================
-// Bottom-up refit (src/hlbvh.hpp:925-969): climbs from the leaves, refit_step per level.
-// =========================================================================================
-// A climb ends at its first arrival at a node, so one thread per leaf (refit_leaf) leaves most
-// lanes of a warp idle while its longest climb goes on (about 5 of 32 lanes active).  Here the
-// warps of a grid of a few blocks per SM take leaves in chunks from a device counter (*work,
-// zero at launch), and a lane whose climb ended takes the warp's next leaf: one climb step
-// per lane and loop iteration.  The merges, boxes, records and heights are those of one climb
-// per leaf (min / max do not depend on the order of the arrivals).
-template <class T>
-__global__ void __launch_bounds__(256) refit_stream_kernel(int n, const int32_t *__restrict__ left,
-                                                           const int32_t *__restrict__ right,
-                                                           const int32_t *__restrict__ parent, T *mnx, T *mxx,
-                                                           T *mny, T *mxy, T *mnz, T *mxz, NodeRec<T> *recs,
-                                                           uint8_t *height, int32_t *counters,
-                                                           const int32_t *__restrict__ leaves, int32_t *work) {
-    T *const       soa[6] = {mnx, mxx, mny, mxy, mnz, mxz};
-    const unsigned FULL   = 0xffffffffu;
-    const int      lane   = threadIdx.x & 31;
-    constexpr int  kChunk = 256;
-    int            next = 0, end = 0; // the warp's chunk of leaves [next, end) (warp-uniform)
-    bool           more = true;       // the counter may still hold leaves (warp-uniform)
-    int            curr = -1, steps = 0;
-    for (;;) {
-        // lanes without a climb take the chunk's next leaves, in lane order
-        unsigned idle = __ballot_sync(FULL, curr < 0);
-        while (idle && more) {
-            if (next >= end) {
-                int b = 0;
-                if (lane == 0) b = atomicAdd(work, kChunk);
-                b = __shfl_sync(FULL, b, 0);
-                if (b >= n) {
-                    more = false;
-                    break;
-                }
-                next = b;
-                end  = min(b + kChunk, n);
-            }
-            const int take = min(__popc(idle), end - next);
-            const int rank = __popc(idle & ((1u << lane) - 1u));
-            if (curr < 0 && rank < take) {
-                curr  = next + rank + n - 1;
-                steps = 0;
-            }
-            next += take;
-            idle = __ballot_sync(FULL, curr < 0);
-        }
-        if (!__any_sync(FULL, curr >= 0)) break;
-        if (curr >= 0) curr = ++steps < n ? refit_step<T>(curr, n, left, right, parent, soa, recs, height, counters,
-                                                           leaves)
-                                          : -1;
-    }
-}
-
-// The fast walks' view of the tree (ft_qtree.cuh), after the refit: leaf j's position, and the
-// record of every internal node of more than kBucket leaves (and of the root), the only ones
-// a walk reaches.
-template <class T>
-__global__ void __launch_bounds__(256) qtree_kernel(int n, const NodeRec<T> *__restrict__ recs,
-                                                    const int32_t *__restrict__ leaves, const T *mnx, const T *mxx,
-                                                    const T *mny, const T *mxy, const T *mnz, const T *mxz,
-                                                    int periodic, QRec *qrec, QPoint *qpts, uint32_t *flag) {
-    const T   rb[6] = {mnx[0], mxx[0], mny[0], mxy[0], mnz[0], mxz[0]};
-    QFrame<T> f;
-    f.make(rb, n, periodic != 0);
-    if (!f.ok && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(flag, f.flag());
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const int s = j + n - 1;
-        qpts[j]     = qpoint<T>(mnx[s], mny[s], mnz[s], f, periodic != 0, flag);
-        if (j < n - 1 && (j == 0 || leaves[j] > kBucket)) qrec_node<T>(j, n, recs, leaves, f, qrec, flag);
     }
 }
 
@@ -553,7 +736,7 @@ template <class T> static void *alloc_dev(size_t count) {
 }
 
 void free_scratch(TreeImpl &s) {
-    void *ptrs[] = {s.recs, s.height, s.counters, s.leafcount, s.qrec, s.qpts, s.qflag, s.key_lo, s.key_hi, s.tmp_lo, s.tmp_hi,
+    void *ptrs[] = {s.recs, s.height, s.counters, s.leafcount, s.pack, s.pend, s.qrec, s.qpts, s.qflag, s.key_lo, s.key_hi, s.tmp_lo, s.tmp_hi,
                     s.perm, s.tmp_perm, s.bbox, s.bbox_partial, s.hist, s.lookback, s.tile_counter, s.status};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -562,9 +745,8 @@ void free_scratch(TreeImpl &s) {
     s.coord   = coord;
 }
 
-static size_t sort_tiles(size_t n, int W) { // the most tiles any tile size makes
-    (void)W;
-    const size_t tile = (size_t)kSortThreads * kSortItemsMin;
+static size_t sort_tiles(size_t n) { // the most tiles any tile size makes
+    const size_t tile = (size_t)kSortThreads * kSortItems;
     return (n + tile - 1) / tile;
 }
 
@@ -580,9 +762,11 @@ void ensure_scratch(TreeImpl &s, const ft_options &o, size_t n) {
     s.height   = (uint8_t *)alloc_dev<uint8_t>(cap);
     s.counters = (int32_t *)alloc_dev<int32_t>(cap);
     s.leafcount = (int32_t *)alloc_dev<int32_t>(cap);
+    s.pack      = alloc_dev<unsigned char>(cap * 4 * cb);
     s.qrec      = alloc_dev<QRec>(cap > 1 ? cap - 1 : 1);
     s.qpts      = alloc_dev<QPoint>(cap);
-    s.qflag     = (uint32_t *)alloc_dev<uint32_t>(1);
+    s.qflag     = (uint32_t *)alloc_dev<uint32_t>(4);
+    s.pend      = (uint32_t *)alloc_dev<uint32_t>(cap);
     s.key_lo   = (uint64_t *)alloc_dev<uint64_t>(cap);
     s.tmp_lo   = (uint64_t *)alloc_dev<uint64_t>(cap);
     if (W == 2) {
@@ -591,10 +775,10 @@ void ensure_scratch(TreeImpl &s, const ft_options &o, size_t n) {
     }
     s.perm         = (uint32_t *)alloc_dev<uint32_t>(cap);
     s.tmp_perm     = (uint32_t *)alloc_dev<uint32_t>(cap);
-    s.bbox         = alloc_dev<uint64_t>(6);
+    s.bbox         = alloc_dev<uint64_t>(12); // the keys' box, then the points' box
     s.bbox_partial = alloc_dev<uint64_t>((size_t)kBboxBlocks * 6);
     s.hist         = (uint32_t *)alloc_dev<uint32_t>(16 * 256 + 16);
-    s.lookback_words = 16 * sort_tiles(cap, W) * 256;
+    s.lookback_words = kSortDigits * sort_tiles(cap) * 256;
     s.lookback     = (uint32_t *)alloc_dev<uint32_t>(s.lookback_words);
     s.tile_counter = (uint32_t *)alloc_dev<uint32_t>(kTicketWords);
     s.status       = (uint32_t *)alloc_dev<uint32_t>(4 + sizeof(TreeSummary) / 4);
@@ -621,28 +805,23 @@ void compute_bbox(Context &ctx, TreeImpl *scratch, const void *x, const void *y,
     }
 }
 
-template <class T>
-static void encode_typed(const ft_options &o, const void *x, const void *y, const void *z, size_t n,
-                         const void *bbox, TreeImpl &s, cudaStream_t st) {
-    int blocks = grid_for(n, 256);
-    if (o.sfc_type == MORTON)
-        encode_kernel<T, MORTON><<<blocks, 256, 0, st>>>((const T *)x, (const T *)y, (const T *)z, n,
-                                                         (const T *)bbox, (unsigned long long *)s.key_lo,
-                                                         (unsigned long long *)s.key_hi, s.perm);
-    else
-        encode_kernel<T, PEANO_HILBERT><<<blocks, 256, 0, st>>>((const T *)x, (const T *)y, (const T *)z, n,
-                                                                (const T *)bbox, (unsigned long long *)s.key_lo,
-                                                                (unsigned long long *)s.key_hi, s.perm);
-    FT_CUDA(cudaGetLastError());
-}
-
-static void encode(const ft_options &o, const void *x, const void *y, const void *z, size_t n, const void *bbox,
-                   TreeImpl &s, cudaStream_t st) {
+// fn(value of the coordinate type's, std::integral_constant of the SFC) for the context's options.
+template <class F> static void for_type(const ft_options &o, F &&f) {
+    auto sfc = [&](auto zero) {
+        using T = decltype(zero);
+        if constexpr (Coord<T>::is_float) {
+            if (o.sfc_type == MORTON) {
+                f(zero, std::integral_constant<int, MORTON>{});
+                return;
+            }
+        }
+        f(zero, std::integral_constant<int, PEANO_HILBERT>{});
+    };
     switch (o.coord_type) {
-    case F32: encode_typed<float>(o, x, y, z, n, bbox, s, st); break;
-    case F64: encode_typed<double>(o, x, y, z, n, bbox, s, st); break;
-    case U32: encode_typed<uint32_t>(o, x, y, z, n, bbox, s, st); break;
-    case U64: encode_typed<unsigned long long>(o, x, y, z, n, bbox, s, st); break;
+    case F32: sfc(0.0f); break;
+    case F64: sfc(0.0); break;
+    case U32: sfc((uint32_t)0); break;
+    case U64: sfc((unsigned long long)0); break;
     }
 }
 
@@ -653,23 +832,32 @@ static int ref_key_mode(const ft_options &o) {
 
 void sfc_encode_ref_layout(Context &ctx, TreeImpl &s, const void *x, const void *y, const void *z, size_t n,
                            const void *bbox_dev, void *keys_ref_dev, cudaStream_t st) {
-    encode(ctx.opts, x, y, z, n, bbox_dev, s, st);
+    for_type(ctx.opts, [&](auto zero, auto sfc) {
+        using T = decltype(zero);
+        encode_kernel<T, decltype(sfc)::value><<<grid_for(n, 256), 256, 0, st>>>(
+            (const T *)x, (const T *)y, (const T *)z, n, (const T *)bbox_dev, (unsigned long long *)s.key_lo,
+            (unsigned long long *)s.key_hi, nullptr, nullptr, nullptr, nullptr);
+    });
+    FT_CUDA(cudaGetLastError());
     keys_to_ref_kernel<<<grid_for(n, 256), 256, 0, st>>>((const unsigned long long *)s.key_lo,
                                                           (const unsigned long long *)s.key_hi, n,
                                                           ref_key_mode(ctx.opts), keys_ref_dev);
     FT_CUDA(cudaGetLastError());
 }
 
-// Two-word keys, second stage: after the passes over the high word, runs of equal high
-// words are put in (low word, input index) order.  The thread at the start of each run
-// insertion-sorts it in place when it holds at most kRunCap keys (stable, so equal keys keep
-// the index order the high-word passes left); a longer run sets flag[0], which switches on
-// the low-word and high-word passes queued behind this kernel.
+// 126-bit keys, second stage: after the sort by the high word, runs of equal high words are put
+// in (low word, input index) order.  The thread at the start of each run insertion-sorts its
+// values in place when it holds at most kRunCap keys (stable, so equal keys keep the index
+// order of the sort); a longer run sets flag[0], and the host sorts by both words instead.
 static constexpr int kRunCap = 32;
 
-__global__ void __launch_bounds__(256) hi_run_fixup_kernel(unsigned long long *__restrict__ klo,
-                                                           const unsigned long long *__restrict__ khi,
-                                                           uint32_t *__restrict__ perm, size_t n, uint32_t *flag) {
+template <class T>
+__global__ void __launch_bounds__(256) hi_run_fixup_kernel(const SortPairs pairs, const uint32_t *__restrict__ skip,
+                                                           int passes, const PackedPoint<T> *__restrict__ pack,
+                                                           size_t n, uint32_t *flag) {
+    const int par = sort_parity(skip, passes);
+    const unsigned long long *__restrict__ khi = pairs.k[par];
+    uint32_t *__restrict__ perm                = pairs.v[par];
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i + 1 < n; i += (size_t)gridDim.x * blockDim.x) {
         const unsigned long long h = khi[i];
         if (khi[i + 1] != h || (i > 0 && khi[i - 1] == h)) continue; // not the start of a run
@@ -680,40 +868,66 @@ __global__ void __launch_bounds__(256) hi_run_fixup_kernel(unsigned long long *_
             continue;
         }
         for (size_t j = i + 1; j < e; ++j) {
-            const unsigned long long kl = klo[j];
-            const uint32_t           pv = perm[j];
-            size_t                   m  = j;
-            while (m > i && klo[m - 1] > kl) {
-                klo[m]  = klo[m - 1];
+            const uint32_t pv = perm[j];
+            const T        kl = pack[pv].pad; // the low key word
+            size_t         m  = j;
+            while (m > i && pack[perm[m - 1]].pad > kl) {
                 perm[m] = perm[m - 1];
                 --m;
             }
-            klo[m]  = kl;
             perm[m] = pv;
         }
     }
 }
 
-// Zeroes `words` words at p when *enable is set (the fallback's look-back status words).
-__global__ void __launch_bounds__(256) zero_if_kernel(uint32_t *p, size_t words, const uint32_t *enable) {
-    if (*enable == 0u) return;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x)
-        p[i] = 0u;
+// Full sort of 126-bit keys (a long run of equal high words): keys for the passes over the low
+// word, and, in the order those leave, for the passes over the high word (from the points, or
+// from the caller's keys).
+__global__ void __launch_bounds__(256) low_keys_kernel(const PackedPoint<unsigned long long> *__restrict__ pack, size_t n,
+                                                       unsigned long long *key, uint32_t *perm) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        key[i]  = pack[i].pad;
+        perm[i] = (uint32_t)i;
+    }
+}
+__global__ void __launch_bounds__(256) high_keys_kernel(const PackedPoint<unsigned long long> *__restrict__ pack,
+                                                        const unsigned long long *__restrict__ ref,
+                                                        const SortPairs pairs, const uint32_t *__restrict__ skip,
+                                                        size_t n) {
+    __shared__ uint8_t s_rot[48 * 8], s_sub[48 * 8];
+    for (int i = threadIdx.x; i < 48 * 8; i += blockDim.x) {
+        s_rot[i] = c_rot[i];
+        s_sub[i] = c_sub[i];
+    }
+    __syncthreads();
+    const int       par  = sort_parity(skip, kSortDigits);
+    const uint32_t *perm = pairs.v[par];
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t     src = perm[i];
+        unsigned long long hi, lo;
+        if (ref) {
+            hi = ref[3 * (size_t)src + 1];
+        } else {
+            const PackedPoint<unsigned long long> p = pack[src];
+            encode_point<unsigned long long, PEANO_HILBERT>(p.x, p.y, p.z, nullptr, s_rot, s_sub, hi, lo);
+        }
+        pairs.k[0][i] = hi;
+        pairs.v[0][i] = src; // (par 0: in place)
+    }
 }
 
-// Persistent grid of a onesweep pass: the CTAs resident at once (three per SM with the
-// tile's shared memory), never more than the tiles.
-template <int W, int IT = 0> static unsigned sort_grid(size_t tiles) {
+// Persistent grid of a onesweep pass: the CTAs resident at once, never more than the tiles.
+template <int ITEMS> static unsigned sort_grid(size_t tiles) {
     static int per_sm = 0, sms = 0;
     static std::once_flag once;
     std::call_once(once, [] {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaFuncSetAttribute(onesweep_kernel<W, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)SortCfg<W, IT>::smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, onesweep_kernel<W, IT>, kSortThreads,
-                                                          SortCfg<W, IT>::smem) != cudaSuccess) {
+            cudaFuncSetAttribute(onesweep_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)SortCfg<ITEMS>::smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, onesweep_kernel<ITEMS>, kSortThreads,
+                                                          SortCfg<ITEMS>::smem) != cudaSuccess) {
             cudaGetLastError();
             per_sm = 1;
             sms    = 148;
@@ -723,125 +937,76 @@ template <int W, int IT = 0> static unsigned sort_grid(size_t tiles) {
     return (unsigned)std::max<size_t>(1, std::min<size_t>(tiles, (size_t)per_sm * (size_t)sms));
 }
 
-// The key sort of build_bvh, with no host synchronisation.  One-word keys: histograms of the
-// eight digits, then eight passes (a constant digit's pass copies).  Two-word keys: the
-// high word's eight passes, then runs of equal high words of at most 32 keys are ordered by
-// (low word, input index) in place; a longer run switches on, on the device, the full
-// two-word sort from that order (histograms of the low word, then the eight low-word and the
-// eight high-word passes: an even number, so the host's ping-pong order is the same whether
-// they run or not).
-template <int W, int IT = 0> static void sort_impl(TreeImpl &s, size_t n, cudaStream_t st) {
-    using Cfg            = SortCfg<W, IT>;
-    const int      D     = 8 * W;
-    const size_t   tiles = (n + Cfg::tile - 1) / Cfg::tile;
-    const unsigned grid  = sort_grid<W, IT>(tiles);
-    FT_CUDA(cudaFuncSetAttribute(onesweep_kernel<W, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)Cfg::smem));
-    FT_CUDA(cudaMemsetAsync(s.hist, 0, (16 * 256 + 16) * sizeof(uint32_t), st));
-    FT_CUDA(cudaMemsetAsync(s.tile_counter, 0, kTicketWords * sizeof(uint32_t), st));
-    uint32_t *skip_dev = s.hist + 16 * 256;
-    uint32_t *fallback = s.tile_counter + 32;
-    // histograms of the digit positions [d0, d0 + 8) of one key word
-    auto histogram = [&](int d0, const uint32_t *enable) {
-        radix_hist_kernel<W, 8><<<grid_for(n, 256, 148 * 4), 256, 0, st>>>(
-            (const unsigned long long *)s.key_lo, (const unsigned long long *)s.key_hi, n, s.hist, d0, enable);
-        radix_scan_kernel<<<8, 256, 0, st>>>(s.hist + d0 * 256, n, skip_dev + d0, enable);
-        FT_CUDA(cudaGetLastError());
-    };
-    auto pass = [&](int d, uint32_t *ticket, const uint32_t *enable) {
-        onesweep_kernel<W, IT><<<grid, kSortThreads, Cfg::smem, st>>>(
-            (const unsigned long long *)s.key_lo, (const unsigned long long *)s.key_hi, s.perm,
-            (unsigned long long *)s.tmp_lo, (unsigned long long *)s.tmp_hi, s.tmp_perm, n, tiles, d >> 3,
-            8 * (d & 7), s.hist + d * 256, s.lookback + (size_t)d * tiles * 256, ticket, enable, skip_dev + d,
-            s.status);
-        FT_CUDA(cudaGetLastError());
-        std::swap(s.key_lo, s.tmp_lo);
-        std::swap(s.key_hi, s.tmp_hi);
-        std::swap(s.perm, s.tmp_perm);
-    };
-    histogram(W == 2 ? 8 : 0, nullptr);
-    FT_CUDA(cudaMemsetAsync(s.lookback, 0, (size_t)D * tiles * 256 * sizeof(uint32_t), st));
-    if constexpr (W == 1) {
-        for (int d = 0; d < 8; ++d) pass(d, s.tile_counter + d, nullptr);
-    } else {
-        // high-word passes first; equal high words are rare for data spread over the box (a
-        // 62-bit prefix of the curve), so a fix-up of their short runs replaces the low-word
-        // passes
-        for (int d = 8; d < 16; ++d) pass(d, s.tile_counter + d, nullptr);
-        hi_run_fixup_kernel<<<grid_for(n, 256), 256, 0, st>>>((unsigned long long *)s.key_lo,
-                                                              (const unsigned long long *)s.key_hi, s.perm, n,
-                                                              fallback);
-        FT_CUDA(cudaGetLastError());
-        // a long run of equal high words: the full two-word sort from the current order (it is
-        // stable, and within equal keys the current order is the input index order)
-        histogram(0, fallback);
-        zero_if_kernel<<<grid_for((size_t)D * tiles * 256, 256, 148 * 8), 256, 0, st>>>(
-            s.lookback, (size_t)D * tiles * 256, fallback);
-        FT_CUDA(cudaGetLastError());
-        for (int d = 0; d < 16; ++d) pass(d, s.tile_counter + 16 + d, fallback);
-    }
-}
-
-// The same sort over a fixed list of digit positions (every listed pass runs; no skips and no
-// fallback), used by the batched build and the query order.
-template <int W> static void sort_fixed_impl(TreeImpl &s, size_t n, int ndig, const int *digits, cudaStream_t st) {
-    using Cfg            = SortCfg<W>;
-    const int      D     = 8 * W;
-    const size_t   tiles = (n + Cfg::tile - 1) / Cfg::tile;
-    const unsigned grid  = sort_grid<W>(tiles);
-    FT_CUDA(cudaMemsetAsync(s.hist, 0, (16 * 256 + 16) * sizeof(uint32_t), st));
-    radix_hist_kernel<W><<<grid_for(n, 256, 148 * 4), 256, 0, st>>>((const unsigned long long *)s.key_lo,
-                                                                      (const unsigned long long *)s.key_hi, n,
-                                                                      s.hist);
-    radix_scan_kernel<<<D, 256, 0, st>>>(s.hist, n, s.hist + 16 * 256);
-    FT_CUDA(cudaGetLastError());
-    FT_CUDA(cudaMemsetAsync(s.lookback, 0, (size_t)D * tiles * 256 * sizeof(uint32_t), st));
-    FT_CUDA(cudaMemsetAsync(s.tile_counter, 0, 16 * sizeof(uint32_t), st));
-    FT_CUDA(cudaFuncSetAttribute(onesweep_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem));
+// The passes of `ndig` digit positions over pairs whose histograms (of all eight positions) are in
+// s.hist.  skip: null (every listed pass runs) or the skip words, indexed by position (then the
+// positions are 0 .. ndig - 1).
+template <int ITEMS>
+static void sort_passes(TreeImpl &s, const SortPairs &pairs, size_t n, int ndig, const int *digits,
+                        const uint32_t *skip, cudaStream_t st) {
+    const size_t   tiles = (n + SortCfg<ITEMS>::tile - 1) / SortCfg<ITEMS>::tile;
+    const unsigned grid  = sort_grid<ITEMS>(tiles);
+    FT_CUDA(cudaFuncSetAttribute(onesweep_kernel<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)SortCfg<ITEMS>::smem));
     for (int i = 0; i < ndig; ++i) {
         const int d = digits[i];
-        onesweep_kernel<W><<<grid, kSortThreads, Cfg::smem, st>>>(
-            (const unsigned long long *)s.key_lo, (const unsigned long long *)s.key_hi, s.perm,
-            (unsigned long long *)s.tmp_lo, (unsigned long long *)s.tmp_hi, s.tmp_perm, n, tiles, d >> 3, 8 * (d & 7),
-            s.hist + d * 256, s.lookback + (size_t)d * tiles * 256, s.tile_counter + d, nullptr, nullptr, s.status);
+        onesweep_kernel<ITEMS><<<grid, kSortThreads, SortCfg<ITEMS>::smem, st>>>(
+            pairs, n, tiles, i, 8 * d, s.hist + d * 256, s.lookback + (size_t)i * tiles * 256, s.tile_counter + i, skip,
+            s.status);
         FT_CUDA(cudaGetLastError());
+    }
+}
+static const int kAllDigits[kSortDigits] = {0, 1, 2, 3, 4, 5, 6, 7};
+
+// Scratch words a sort of n pairs starts from: histograms, look-back words and tickets.
+static void sort_clear(TreeImpl &s, size_t n, int ndig, int items, cudaStream_t st) {
+    const size_t tile  = (size_t)kSortThreads * items;
+    const size_t tiles = (n + tile - 1) / tile;
+    FT_CUDA(cudaMemsetAsync(s.hist, 0, (kSortDigits * 256 + 16) * sizeof(uint32_t), st));
+    FT_CUDA(cudaMemsetAsync(s.tile_counter, 0, kSortDigits * sizeof(uint32_t), st));
+    FT_CUDA(cudaMemsetAsync(s.lookback, 0, (size_t)ndig * tiles * 256 * sizeof(uint32_t), st));
+}
+
+// Sort of build_bvh's pairs after their histograms (constant digits are skipped on the device).
+static void sort_run(TreeImpl &s, const SortPairs &pairs, size_t n, int items, cudaStream_t st) {
+    uint32_t *skip = s.hist + kSortDigits * 256;
+    radix_scan_kernel<<<kSortDigits, 256, 0, st>>>(s.hist, n, skip);
+    FT_CUDA(cudaGetLastError());
+    switch (items) {
+    case 12: sort_passes<12>(s, pairs, n, kSortDigits, kAllDigits, skip, st); break;
+    case 16: sort_passes<16>(s, pairs, n, kSortDigits, kAllDigits, skip, st); break;
+    case 20: sort_passes<20>(s, pairs, n, kSortDigits, kAllDigits, skip, st); break;
+    default: sort_passes<kSortItems>(s, pairs, n, kSortDigits, kAllDigits, skip, st); break;
+    }
+}
+static int sort_tile_items(int items) { return items == 12 || items == 16 || items == 20 ? items : kSortItems; }
+
+// The same sort over a fixed list of digit positions of (key_lo, perm) (every listed pass runs),
+// used by the batched build and the query order.
+void sort_pairs_fixed(TreeImpl &s, size_t n, int words, int ndigits, const int *digits, cudaStream_t st) {
+    (void)words; // one-word keys
+    if (n < 2 || ndigits <= 0) return;
+    sort_clear(s, n, ndigits, kSortItems, st);
+    radix_hist_kernel<<<grid_for(n, 256, 148 * 4), 256, 0, st>>>((const unsigned long long *)s.key_lo, n, s.hist);
+    radix_scan_kernel<<<kSortDigits, 256, 0, st>>>(s.hist, n, s.hist + kSortDigits * 256);
+    FT_CUDA(cudaGetLastError());
+    const SortPairs pairs = {{(unsigned long long *)s.key_lo, (unsigned long long *)s.tmp_lo}, {s.perm, s.tmp_perm}};
+    sort_passes<kSortItems>(s, pairs, n, ndigits, digits, nullptr, st);
+    if (ndigits & 1) {
         std::swap(s.key_lo, s.tmp_lo);
-        std::swap(s.key_hi, s.tmp_hi);
         std::swap(s.perm, s.tmp_perm);
     }
 }
 
-void sort_pairs_fixed(TreeImpl &s, size_t n, int words, int ndigits, const int *digits, cudaStream_t st) {
-    if (n < 2 || ndigits <= 0) return;
-    if (words == 1) sort_fixed_impl<1>(s, n, ndigits, digits, st);
-    else sort_fixed_impl<2>(s, n, ndigits, digits, st);
-}
-
-size_t sort_lookback_words(size_t n, int words) { return 16 * sort_tiles(n, words) * 256; }
-
-// items: keys per thread of a onesweep tile (0: the default for the key width).
-static void sort_keys(const ft_options &o, TreeImpl &s, size_t n, cudaStream_t st, int items = 0) {
-    if (n < 2) return;
-    if (key_words(o) == 1) {
-        switch (items) {
-        case 12: sort_impl<1, 12>(s, n, st); break;
-        case 16: sort_impl<1, 16>(s, n, st); break;
-        case 20: sort_impl<1, 20>(s, n, st); break;
-        default: sort_impl<1>(s, n, st); break; // 8
-        }
-    } else {
-        switch (items) {
-        case 12: sort_impl<2, 12>(s, n, st); break;
-        case 16: sort_impl<2, 16>(s, n, st); break;
-        default: sort_impl<2>(s, n, st); break; // 8
-        }
-    }
+size_t sort_lookback_words(size_t n, int words) {
+    (void)words;
+    return kSortDigits * sort_tiles(n) * 256;
 }
 
 const int *sort_item_choices(int words, int *count) {
-    static const int one[4] = {8, 12, 16, 20}, two[3] = {8, 12, 16}; // the default first
-    *count = words == 1 ? 4 : 3;
-    return words == 1 ? one : two;
+    static const int items[4] = {8, 12, 16, 20}; // the default first
+    (void)words;                                 // (126-bit keys are sorted by their high word)
+    *count = 4;
+    return items;
 }
 
 template <class T> struct SoA {
@@ -851,110 +1016,180 @@ template <class T> struct SoA {
           mxz((T *)t.max_z) {}
 };
 
-template <class T>
-static void build_qtree(const ft_options &o, ft_tree &t, TreeImpl &s, size_t n, cudaStream_t st) {
-    SoA<T> a(t);
-    FT_CUDA(cudaMemsetAsync(s.qflag, 0, sizeof(uint32_t), st));
-    qtree_kernel<T><<<grid_for(n, 256, 148 * 32), 256, 0, st>>>((int)n, (const NodeRec<T> *)s.recs, s.leafcount, a.mnx,
-                                                                a.mxx, a.mny, a.mxy, a.mnz, a.mxz, o.periodic,
-                                                                (QRec *)s.qrec, (QPoint *)s.qpts, s.qflag);
+// Topology, boxes and records from sorted keys (ft_treelet.cuh): the treelets, then the walk
+// records of the nodes formed outside a block.
+template <class T, int SRC>
+static void build_treelets(const ft_options &o, ft_tree &t, TreeImpl &s, size_t n, const void *box, TreeletArgs<T> a,
+                           cudaStream_t st, Context *prof = nullptr) {
+    a.n        = (int)n;
+    a.periodic = o.periodic;
+    a.klo      = (const unsigned long long *)s.key_lo;
+    a.khi      = (const unsigned long long *)s.key_hi;
+    if (SRC != LEAVES_PACKED) s.sort_passes = 0;
+    a.box      = (const T *)box;
+    void *soa[6] = {t.min_x, t.max_x, t.min_y, t.max_y, t.min_z, t.max_z};
+    for (int d = 0; d < 6; ++d) a.soa[d] = (T *)soa[d];
+    a.left      = t.left_child;
+    a.right     = t.right_child;
+    a.parent    = t.parent;
+    a.orig      = t.orig_idx;
+    a.id_out    = t.id;
+    a.ghost_out = t.is_ghost;
+    a.recs      = (NodeRec<T> *)s.recs;
+    a.height    = s.height;
+    a.leaves    = s.leafcount;
+    a.qrec      = (QRec *)s.qrec;
+    a.qpts      = (QPoint *)s.qpts;
+    a.qflag     = s.qflag;
+    a.slot      = s.counters;
+    a.pend      = s.pend;
+    a.list      = (int32_t *)s.lookback; // (at least n words; the sort is done with them)
+    a.status    = s.status;
+    const bool many = n > (size_t)kTreeletLeaves;
+    FT_CUDA(cudaMemsetAsync(s.qflag, 0, 4 * sizeof(uint32_t), st));
+    if (many) FT_CUDA(cudaMemsetAsync(s.counters, 0xFF, n * sizeof(int32_t), st));
+    if (n == 1) FT_CUDA(cudaMemsetAsync(t.parent, 0xFF, sizeof(int32_t), st));
+    const unsigned blocks = (unsigned)((n + kTreeletLeaves - 1) / kTreeletLeaves);
+    auto           run    = [&](auto kind) {
+        auto fn = treelet_kernel<T, decltype(kind)::value, SRC>;
+        FT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TreeletShared<T>)));
+        fn<<<blocks, kTreeletThreads, sizeof(TreeletShared<T>), st>>>(a);
+        if (many) // (a warp per 32 entries of some 20 a block, at most a few per SM)
+            treelet_climb_kernel<T, decltype(kind)::value, SRC><<<grid_for(n / 16, 128, 148 * 8), 128, 0, st>>>(a);
+    };
+    if constexpr (Coord<T>::key_words == 2) run(std::integral_constant<int, 2>{});
+    else if (delta_kind(o) == 0) run(std::integral_constant<int, 0>{});
+    else run(std::integral_constant<int, 1>{});
     FT_CUDA(cudaGetLastError());
-}
-
-template <class T>
-static void topology_and_refit(const ft_options &o, ft_tree &t, TreeImpl &s, size_t n, cudaStream_t st,
-                               Context *prof = nullptr) {
-    if (n < 2) {
-        s.height_root = 0;
-        stage_mark(prof, BS_TOPOLOGY, st);
-        stage_mark(prof, BS_REFIT, st);
-        stage_mark(prof, BS_RECORDS, st);
-        return;
-    }
-    FT_CUDA(cudaMemsetAsync(t.parent, 0xFF, (2 * n - 1) * sizeof(int32_t), st)); // -1 (849)
-    int blocks = grid_for(n, 256, 148 * 32);
-    const unsigned long long *lo = (const unsigned long long *)s.key_lo, *hi = (const unsigned long long *)s.key_hi;
-    switch (delta_kind(o)) {
-    case 0: karras_kernel<0><<<blocks, 256, 0, st>>>(lo, hi, (int)n, t.left_child, t.right_child, t.parent, s.leafcount); break;
-    case 1: karras_kernel<1><<<blocks, 256, 0, st>>>(lo, hi, (int)n, t.left_child, t.right_child, t.parent, s.leafcount); break;
-    default: karras_kernel<2><<<blocks, 256, 0, st>>>(lo, hi, (int)n, t.left_child, t.right_child, t.parent, s.leafcount); break;
-    }
-    FT_CUDA(cudaGetLastError());
-    stage_mark(prof, BS_TOPOLOGY, st);
-    // arrival counters of the n - 1 internal nodes, then the streaming refit's leaf counter
-    FT_CUDA(cudaMemsetAsync(s.counters, 0, n * sizeof(int32_t), st));
-    SoA<T> a(t);
-    refit_stream_kernel<T><<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(
-        (int)n, t.left_child, t.right_child, t.parent, a.mnx, a.mxx, a.mny, a.mxy, a.mnz, a.mxz,
-        (NodeRec<T> *)s.recs, s.height, s.counters, s.leafcount, s.counters + (n - 1));
     stage_mark(prof, BS_REFIT, st);
+    if (many) treelet_qrec_kernel<T><<<grid_for(n / 64 + 1, 128, 148 * 8), 128, 0, st>>>(a);
     FT_CUDA(cudaGetLastError());
-    build_qtree<T>(o, t, s, n, st);
     stage_mark(prof, BS_RECORDS, st);
+    if (n < 2) s.height_root = 0;
 }
 
-template <class T>
+// The same from leaf slots that hold their points (caller arrays, an imported tree).
+template <class T> static void build_in_place(Context &ctx, ft_tree &t, TreeImpl &s, size_t n, cudaStream_t st) {
+    const size_t leaf = n - 1;
+    void        *box  = (T *)s.bbox + 6;
+    compute_bbox(ctx, &s, (const T *)t.min_x + leaf, (const T *)t.min_y + leaf, (const T *)t.min_z + leaf, n, box, st);
+    build_treelets<T, LEAVES_IN_PLACE>(ctx.opts, t, s, n, box, TreeletArgs<T>{}, st);
+}
+
+// The pairs build_bvh sorts: the sort word of each key and its input index.
+static SortPairs build_pairs(const ft_options &o, const TreeImpl &s) {
+    const bool two = key_words(o) == 2;
+    return SortPairs{{(unsigned long long *)(two ? s.key_hi : s.key_lo), (unsigned long long *)(two ? s.tmp_hi : s.tmp_lo)},
+                     {s.perm, s.tmp_perm}};
+}
+
+// full_sort: 126-bit keys by both words (the last build met a long run of equal high words).
+template <class T, int SFC>
 static void build_bvh_typed(Context &ctx, ft_tree &t, const void *x, const void *y, const void *z, size_t n,
-                            const uint32_t *id, const int8_t *ghost, const void *bbox_host, void *caller_keys,
-                            cudaStream_t st, int sort_items) {
-    TreeImpl &s = *(TreeImpl *)t.impl;
+                            const uint32_t *id, const int8_t *ghost, const void *bbox_host, const void *caller_keys,
+                            cudaStream_t st, int sort_items, bool full_sort) {
+    constexpr bool TWO = Coord<T>::key_words == 2;
+    TreeImpl      &s   = *(TreeImpl *)t.impl;
     ensure_scratch(s, ctx.opts, n);
-    stage_mark(&ctx, BS_START, st);
-    // 1. bounding box.  Only the float encode reads it; integer encoding ignores it, so an
-    // integer tree always keeps its true box (the query distance mode depends on it).
-    if (bbox_host && Coord<T>::is_float)
-        FT_CUDA(cudaMemcpyAsync(s.bbox, bbox_host, 6 * sizeof(T), cudaMemcpyHostToDevice, st));
-    else compute_bbox(ctx, &s, x, y, z, n, s.bbox, st);
-    stage_mark(&ctx, BS_BBOX, st);
-    // 2. keys + iota permutation
-    if (caller_keys) {
-        keys_from_ref_kernel<<<grid_for(n, 256), 256, 0, st>>>(caller_keys, n, ref_key_mode(ctx.opts),
-                                                               (unsigned long long *)s.key_lo,
-                                                               (unsigned long long *)s.key_hi, s.perm);
-        FT_CUDA(cudaGetLastError());
-    } else {
-        encode(ctx.opts, x, y, z, n, s.bbox, s, st);
-    }
-    stage_mark(&ctx, BS_ENCODE, st);
-    // 3. sort (key, perm), with the tile the autotuner chose for this shape
-    if (sort_items <= 0) {
+    if (sort_items <= 0) { // the tile the autotuner chose for this shape
         auto it = ctx.tuned.find(tune_key(TUNE_BUILD, key_words(ctx.opts), n));
         if (it != ctx.tuned.end()) sort_items = it->second.items;
     }
-    sort_keys(ctx.opts, s, n, st, sort_items);
-    stage_mark(&ctx, BS_SORT, st);
-    if (caller_keys) {
-        keys_to_ref_kernel<<<grid_for(n, 256), 256, 0, st>>>((const unsigned long long *)s.key_lo,
-                                                              (const unsigned long long *)s.key_hi, n,
-                                                              ref_key_mode(ctx.opts), caller_keys);
+    sort_items = sort_tile_items(sort_items);
+    stage_mark(&ctx, BS_START, st);
+    const T *px = (const T *)x, *py = (const T *)y, *pz = (const T *)z;
+    // 1. bounding box.  Only the float encode reads a caller's; integer encoding ignores it, so an
+    // integer tree always keeps its true box (the query distance mode depends on it).  The
+    // walks' frame follows from the points' own box.
+    const bool caller_box = bbox_host && Coord<T>::is_float;
+    T         *box        = (T *)s.bbox + (caller_box ? 6 : 0);
+    if (caller_box) FT_CUDA(cudaMemcpyAsync(s.bbox, bbox_host, 6 * sizeof(T), cudaMemcpyHostToDevice, st));
+    PackedPoint<T> *pack  = (PackedPoint<T> *)s.pack;
+    const SortPairs pairs = build_pairs(ctx.opts, s);
+    uint32_t       *skip  = s.hist + kSortDigits * 256;
+    uint32_t       *runs  = s.tile_counter + kLongRunWord;
+    const bool      front = n <= (size_t)kFrontMax && !caller_keys && !full_sort;
+    if (front) { // box, keys and sort in one block
+        auto fn = front_kernel<T, SFC>;
+        FT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FrontShared<T>)));
+        fn<<<1, kFrontThreads, sizeof(FrontShared<T>), st>>>(px, py, pz, (int)n, caller_box ? 1 : 0, (T *)s.bbox,
+                                                             pairs.k[0], pairs.v[0], pack);
+        FT_CUDA(cudaGetLastError());
+        s.sort_passes = 0;
+        stage_mark(&ctx, BS_BBOX, st);
+        stage_mark(&ctx, BS_ENCODE, st);
+    } else {
+        compute_bbox(ctx, &s, x, y, z, n, box, st);
+        stage_mark(&ctx, BS_BBOX, st);
+        // 2. keys, input indices, packed points, digit histograms
+        sort_clear(s, n, kSortDigits, sort_items, st);
+        const int grid = grid_for(n, 256, 148 * 8);
+        if (caller_keys)
+            pack_ref_kernel<T><<<grid, 256, 0, st>>>(px, py, pz, n, caller_keys, ref_key_mode(ctx.opts), pairs.k[0],
+                                                     pairs.v[0], pack, s.hist);
+        else
+            encode_kernel<T, SFC><<<grid, 256, 0, st>>>(px, py, pz, n, (const T *)s.bbox, nullptr, nullptr, pairs.k[0],
+                                                        pairs.v[0], pack, s.hist);
+        FT_CUDA(cudaGetLastError());
+        stage_mark(&ctx, BS_ENCODE, st);
+        // 3. sort
+        if constexpr (TWO) {
+            if (full_sort) { // by the low word first
+                low_keys_kernel<<<grid_for(n, 256), 256, 0, st>>>(pack, n, pairs.k[0], pairs.v[0]);
+                FT_CUDA(cudaMemsetAsync(s.hist, 0, kSortDigits * 256 * sizeof(uint32_t), st));
+                radix_hist_kernel<<<grid_for(n, 256, 148 * 4), 256, 0, st>>>(pairs.k[0], n, s.hist);
+                sort_run(s, pairs, n, sort_items, st);
+                high_keys_kernel<<<grid_for(n, 256), 256, 0, st>>>(pack, (const unsigned long long *)caller_keys, pairs,
+                                                                   skip, n);
+                sort_clear(s, n, kSortDigits, sort_items, st);
+                radix_hist_kernel<<<grid_for(n, 256, 148 * 4), 256, 0, st>>>(pairs.k[0], n, s.hist);
+                FT_CUDA(cudaGetLastError());
+            }
+        }
+        sort_run(s, pairs, n, sort_items, st);
+        s.sort_passes = kSortDigits;
+    }
+    if constexpr (TWO) {
+        FT_CUDA(cudaMemsetAsync(runs, 0, sizeof(uint32_t), st));
+        if (!full_sort)
+            hi_run_fixup_kernel<T><<<grid_for(n, 256), 256, 0, st>>>(pairs, skip, s.sort_passes, pack, n, runs);
         FT_CUDA(cudaGetLastError());
     }
-    // 4. gather into leaf slots; internal slots of id / is_ghost / orig_idx are zeroed
-    SoA<T> a(t);
-    if (n > 1) {
-        FT_CUDA(cudaMemsetAsync(t.id, 0, (n - 1) * sizeof(uint32_t), st));
-        FT_CUDA(cudaMemsetAsync(t.is_ghost, 0, (n - 1) * sizeof(int8_t), st));
-        FT_CUDA(cudaMemsetAsync(t.orig_idx, 0, (n - 1) * sizeof(int32_t), st));
-    }
-    gather_kernel<T><<<grid_for(n, 256), 256, 0, st>>>((const T *)x, (const T *)y, (const T *)z, s.perm, n, id, ghost,
-                                                       a.mnx, a.mxx, a.mny, a.mxy, a.mnz, a.mxz, t.id, t.is_ghost,
-                                                       t.orig_idx);
-    FT_CUDA(cudaGetLastError());
-    if (n == 1) FT_CUDA(cudaMemsetAsync(t.parent, 0xFF, sizeof(int32_t), st));
+    stage_mark(&ctx, BS_SORT, st);
+    // 4. leaves, topology, boxes and records
     stage_mark(&ctx, BS_GATHER, st);
-    // 5. topology + refit
-    topology_and_refit<T>(ctx.opts, t, s, n, st, &ctx);
+    stage_mark(&ctx, BS_TOPOLOGY, st);
+    TreeletArgs<T> a{};
+    for (int b = 0; b < 2; ++b) {
+        a.key[b]  = pairs.k[b];
+        a.perm[b] = pairs.v[b];
+    }
+    a.skip    = skip;
+    a.passes  = s.sort_passes;
+    a.stop    = TWO ? runs : nullptr;
+    a.klo_out = TWO ? (unsigned long long *)s.key_lo : nullptr;
+    a.pack    = pack;
+    a.id      = id;
+    a.ghost   = ghost;
+    build_treelets<T, LEAVES_PACKED>(ctx.opts, t, s, n, box, a, st, &ctx);
     ctx.bprof.recorded = ctx.bprof.on;
 }
 
 void build_bvh(Context &ctx, ft_tree &t, const void *x, const void *y, const void *z, size_t n, const uint32_t *id,
-               const int8_t *ghost, const void *bbox_host, void *caller_keys, cudaStream_t st, int sort_items) {
-    switch (ctx.opts.coord_type) {
-    case F32: build_bvh_typed<float>(ctx, t, x, y, z, n, id, ghost, bbox_host, caller_keys, st, sort_items); break;
-    case F64: build_bvh_typed<double>(ctx, t, x, y, z, n, id, ghost, bbox_host, caller_keys, st, sort_items); break;
-    case U32: build_bvh_typed<uint32_t>(ctx, t, x, y, z, n, id, ghost, bbox_host, caller_keys, st, sort_items); break;
-    case U64: build_bvh_typed<unsigned long long>(ctx, t, x, y, z, n, id, ghost, bbox_host, caller_keys, st, sort_items); break;
-    }
+               const int8_t *ghost, const void *bbox_host, const void *caller_keys, cudaStream_t st, int sort_items,
+               bool full_sort) {
+    for_type(ctx.opts, [&](auto zero, auto sfc) {
+        build_bvh_typed<decltype(zero), decltype(sfc)::value>(ctx, t, x, y, z, n, id, ghost, bbox_host, caller_keys, st,
+                                                              sort_items, full_sort);
+    });
+}
+
+// The sorted keys of a finished build in the reference's layout.
+void sorted_keys_to_ref(const ft_options &o, const TreeImpl &s, size_t n, void *keys_ref, cudaStream_t st) {
+    keys_to_ref_kernel<<<grid_for(n, 256), 256, 0, st>>>((const unsigned long long *)s.key_lo,
+                                                          (const unsigned long long *)s.key_hi, n, ref_key_mode(o),
+                                                          keys_ref);
+    FT_CUDA(cudaGetLastError());
 }
 
 int key_words_of(const ft_options &o) { return key_words(o); }
@@ -968,7 +1203,7 @@ static void build_tree_typed(Context &ctx, ft_tree &t, const void *keys_ref, con
     ensure_scratch(s, ctx.opts, n);
     keys_from_ref_kernel<<<grid_for(n, 256), 256, 0, st>>>(keys_ref, n, ref_key_mode(ctx.opts),
                                                            (unsigned long long *)s.key_lo,
-                                                           (unsigned long long *)s.key_hi, nullptr);
+                                                           (unsigned long long *)s.key_hi);
     FT_CUDA(cudaGetLastError());
     SoA<T> a(t);
     if (sx && sy && sz)
@@ -976,8 +1211,7 @@ static void build_tree_typed(Context &ctx, ft_tree &t, const void *keys_ref, con
                                                               sghost, sorig, a.mnx, a.mxx, a.mny, a.mxy, a.mnz,
                                                               a.mxz, t.id, t.is_ghost, t.orig_idx);
     FT_CUDA(cudaGetLastError());
-    if (n == 1) FT_CUDA(cudaMemsetAsync(t.parent, 0xFF, sizeof(int32_t), st));
-    topology_and_refit<T>(ctx.opts, t, s, n, st);
+    build_in_place<T>(ctx, t, s, n, st);
 }
 
 // Refit-only update of a built tree (no reference counterpart: the reference rebuilds).  The
@@ -986,30 +1220,26 @@ static void build_tree_typed(Context &ctx, ft_tree &t, const void *keys_ref, con
 // result is the tree build_tree (src/hlbvh.hpp:773-982) makes from the same sorted keys with
 // the new positions as its leaf arrays.
 template <class T>
-static void refit_typed(const ft_options &o, ft_tree &t, const void *x, const void *y, const void *z, size_t n, bool leaf_order,
-                        cudaStream_t st) {
-    TreeImpl &s = *(TreeImpl *)t.impl;
-    SoA<T>    a(t);
-    refit_gather_kernel<T><<<grid_for(n, 256), 256, 0, st>>>((const T *)x, (const T *)y, (const T *)z,
-                                                             leaf_order ? nullptr : t.orig_idx, n, a.mnx, a.mxx,
-                                                             a.mny, a.mxy, a.mnz, a.mxz, s.status);
-    FT_CUDA(cudaGetLastError());
-    if (n < 2) return;
-    FT_CUDA(cudaMemsetAsync(s.counters, 0, n * sizeof(int32_t), st));
-    refit_stream_kernel<T><<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(
-        (int)n, t.left_child, t.right_child, t.parent, a.mnx, a.mxx, a.mny, a.mxy, a.mnz, a.mxz,
-        (NodeRec<T> *)s.recs, s.height, s.counters, s.leafcount, s.counters + (n - 1));
-    FT_CUDA(cudaGetLastError());
-    build_qtree<T>(o, t, s, n, st);
+static void refit_typed(Context &ctx, ft_tree &t, const void *x, const void *y, const void *z, size_t n,
+                        bool leaf_order, cudaStream_t st) {
+    TreeImpl &s   = *(TreeImpl *)t.impl;
+    void     *box = (T *)s.bbox + 6; // (the build's box stays: it encoded the keys)
+    compute_bbox(ctx, &s, x, y, z, n, box, st);
+    TreeletArgs<T> a{};
+    a.x          = (const T *)x;
+    a.y          = (const T *)y;
+    a.z          = (const T *)z;
+    a.leaf_order = leaf_order ? 1 : 0;
+    build_treelets<T, LEAVES_MOVED>(ctx.opts, t, s, n, box, a, st);
 }
 
 void refit_bvh(Context &ctx, ft_tree &t, const void *x, const void *y, const void *z, size_t n, bool leaf_order,
                cudaStream_t st) {
     switch (ctx.opts.coord_type) {
-    case F32: refit_typed<float>(ctx.opts, t, x, y, z, n, leaf_order, st); break;
-    case F64: refit_typed<double>(ctx.opts, t, x, y, z, n, leaf_order, st); break;
-    case U32: refit_typed<uint32_t>(ctx.opts, t, x, y, z, n, leaf_order, st); break;
-    case U64: refit_typed<unsigned long long>(ctx.opts, t, x, y, z, n, leaf_order, st); break;
+    case F32: refit_typed<float>(ctx, t, x, y, z, n, leaf_order, st); break;
+    case F64: refit_typed<double>(ctx, t, x, y, z, n, leaf_order, st); break;
+    case U32: refit_typed<uint32_t>(ctx, t, x, y, z, n, leaf_order, st); break;
+    case U64: refit_typed<unsigned long long>(ctx, t, x, y, z, n, leaf_order, st); break;
     }
 }
 
@@ -1019,16 +1249,17 @@ void recompute_from_keys(Context &ctx, ft_tree &t, cudaStream_t st) {
     TreeImpl &s = *(TreeImpl *)t.impl;
     size_t    n = t.num_leaves;
     switch (ctx.opts.coord_type) {
-    case F32: topology_and_refit<float>(ctx.opts, t, s, n, st); break;
-    case F64: topology_and_refit<double>(ctx.opts, t, s, n, st); break;
-    case U32: topology_and_refit<uint32_t>(ctx.opts, t, s, n, st); break;
-    case U64: topology_and_refit<unsigned long long>(ctx.opts, t, s, n, st); break;
+    case F32: build_in_place<float>(ctx, t, s, n, st); break;
+    case F64: build_in_place<double>(ctx, t, s, n, st); break;
+    case U32: build_in_place<uint32_t>(ctx, t, s, n, st); break;
+    case U64: build_in_place<unsigned long long>(ctx, t, s, n, st); break;
     }
 }
 
 template <class T>
 __global__ void tree_summary_kernel(int n, const T *mxx, const T *mxy, const T *mxz, const uint8_t *height,
-                                    const uint32_t *status, const uint32_t *qflag, TreeSummary *out) {
+                                    const uint32_t *status, const uint32_t *qflag, const uint32_t *skip, int passes,
+                                    const uint32_t *runs, TreeSummary *out) {
     TreeSummary m;
     m.mx[0]  = Coord<T>::is_float ? 0ull : (unsigned long long)mxx[0];
     m.mx[1]  = Coord<T>::is_float ? 0ull : (unsigned long long)mxy[0];
@@ -1036,17 +1267,20 @@ __global__ void tree_summary_kernel(int n, const T *mxx, const T *mxy, const T *
     m.status = *status;
     m.height = n > 1 ? height[0] : 0u;
     m.qflag  = n > 1 ? *qflag : 0u;
-    m.pad    = 0u;
-    *out     = m;
+    m.parity    = (uint32_t)sort_parity(skip, passes);
+    m.long_runs = runs ? *runs : 0u;
+    *out        = m;
 }
 
-void tree_summary(const ft_options &o, const ft_tree &t, TreeSummary &out, cudaStream_t st) {
-    const TreeImpl &s   = *(const TreeImpl *)t.impl;
+void tree_summary(const ft_options &o, ft_tree &t, bool sorted, TreeSummary &out, cudaStream_t st) {
+    TreeImpl       &s   = *(TreeImpl *)t.impl;
+    const uint32_t *runs = sorted && key_words(o) == 2 ? s.tile_counter + kLongRunWord : nullptr;
     TreeSummary    *dev = reinterpret_cast<TreeSummary *>(s.status + 4);
     auto            run = [&](auto *p) {
         using T = std::remove_pointer_t<decltype(p)>;
         tree_summary_kernel<T><<<1, 1, 0, st>>>((int)t.num_leaves, (const T *)t.max_x, (const T *)t.max_y,
-                                                (const T *)t.max_z, s.height, s.status, s.qflag, dev);
+                                                (const T *)t.max_z, s.height, s.status, s.qflag,
+                                                s.hist + kSortDigits * 256, sorted ? s.sort_passes : 0, runs, dev);
     };
     switch (o.coord_type) {
     case F32: run((float *)nullptr); break;
@@ -1057,6 +1291,12 @@ void tree_summary(const ft_options &o, const ft_tree &t, TreeSummary &out, cudaS
     FT_CUDA(cudaGetLastError());
     FT_CUDA(cudaMemcpyAsync(&out, dev, sizeof(out), cudaMemcpyDeviceToHost, st));
     FT_CUDA(cudaStreamSynchronize(st));
+    if (out.parity) { // the sort left its pairs in the second buffers
+        if (key_words(o) == 2) std::swap(s.key_hi, s.tmp_hi);
+        else std::swap(s.key_lo, s.tmp_lo);
+        std::swap(s.perm, s.tmp_perm);
+    }
+    s.sort_passes = 0;
 }
 
 void build_tree_from_keys(Context &ctx, ft_tree &t, const void *keys_ref, const void *sx, const void *sy,

@@ -169,6 +169,18 @@ template <class T> FT_D void sfc_axis_params(T lo, T hi, T &p_lo, T &p_inv) {
     p_lo = lo;
 }
 
+// Cells of a floating-point position on the 21-bit grid (389-403): nx = clamp((p - min) * inv, 0,
+// nextafter(1, 0)) in T.
+template <class T, int SFC> FT_D void sfc_cells(T x, T y, T z, const T *par, unsigned long long c[3]) {
+    const T upper = (sizeof(T) == 4) ? (T)0x1.fffffep-1f : (T)0x1.fffffffffffffp-1;
+    const T p[3]  = {x, y, z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const T nx = c_fmin(c_fmax(mul_rn(sub_rn(p[d], par[2 * d]), par[2 * d + 1]), T(0)), upper);
+        c[d]       = (SFC == 0) ? morton_cell(nx) : ph_cell(nx);
+    }
+}
+
 // SFC key of one point (sfc_encode, src/hlbvh.hpp:357-423).  par = {lo, inv} per axis (float
 // coordinates only); integer coordinates are masked to their position bits (375-387).
 template <class T, int SFC>
@@ -182,15 +194,8 @@ FT_D void encode_point(T x, T y, T z, const T *par, const uint8_t *s_rot, const 
         ph_key<C::bits>((unsigned long long)x & mask, (unsigned long long)y & mask, (unsigned long long)z & mask,
                         s_rot, s_sub, hi, lo);
     } else {
-        // nx = clamp((p - min) * inv, 0, nextafter(1, 0)) in T (389-403)
-        const T upper = (sizeof(T) == 4) ? (T)0x1.fffffep-1f : (T)0x1.fffffffffffffp-1;
-        T       p[3]  = {x, y, z};
         unsigned long long c[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            T nx = c_fmin(c_fmax(mul_rn(sub_rn(p[d], par[2 * d]), par[2 * d + 1]), T(0)), upper);
-            c[d] = (SFC == MORTON) ? morton_cell(nx) : ph_cell(nx);
-        }
+        sfc_cells<T, SFC>(x, y, z, par, c);
         if (SFC == MORTON) lo = spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2);
         else ph_key<21>(c[0], c[1], c[2], s_rot, s_sub, hi, lo);
     }

@@ -444,10 +444,12 @@ ft_status ft_sfc_encode(ft_context *ctx, const void *x, const void *y, const voi
 // What the host keeps of a finished build: one small launch, one copy, one wait.  Throws what
 // the kernels recorded; sets the height, the frame and whether every coordinate of an integer
 // tree lies below the period 2^42 (64-bit) / 2^21 (32-bit), i.e. the root box maxima do.
-static void finish_build(const ft_context *ctx, ft_tree *tree, cudaStream_t st) {
+// sorted: the build sorted its keys itself (build_bvh).  Returns false when it has to be repeated
+// with the full sort.
+static bool finish_build(const ft_context *ctx, ft_tree *tree, cudaStream_t st, bool sorted = false) {
     TreeImpl    &impl = *(TreeImpl *)tree->impl;
     TreeSummary  m;
-    tree_summary(ctx->opts, *tree, m, st);
+    tree_summary(ctx->opts, *tree, sorted, m, st);
     if (m.status) check_device_status(impl.status, st);
     const int      ct = ctx->opts.coord_type;
     const uint64_t P  = ct == FT_COORD_U64 ? 1ull << 42 : 1ull << 21;
@@ -456,6 +458,7 @@ static void finish_build(const ft_context *ctx, ft_tree *tree, cudaStream_t st) 
     impl.plain_only   = (m.qflag & kQFlagPlain) != 0u;
     impl.in_period    = ct == FT_COORD_F32 || ct == FT_COORD_F64 || (m.mx[0] < P && m.mx[1] < P && m.mx[2] < P);
     impl.clean42      = impl.clean42_ok && ct == FT_COORD_U64 && impl.in_period;
+    return m.long_runs == 0u;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -648,10 +651,18 @@ ft_status ft_build_bvh(ft_context *ctx, const void *x, const void *y, const void
     impl.own_keys      = false;
     ft::build_bvh(*ctx, *tree, sx.dev, sy.dev, sz.dev, n, (const uint32_t *)sid.dev, (const int8_t *)sgh.dev, bbox6,
                   sk.dev, st);
-    impl.own_keys = keys == nullptr; // the sorted keys are this library's encoding of bbox
-    if (keys) sk.copy_back();
+    impl.own_keys   = keys == nullptr; // the sorted keys are this library's encoding of bbox
     impl.clean42_ok = true;
-    finish_build(ctx, tree, st);
+    if (!finish_build(ctx, tree, st, true)) {
+        ft::build_bvh(*ctx, *tree, sx.dev, sy.dev, sz.dev, n, (const uint32_t *)sid.dev, (const int8_t *)sgh.dev, bbox6,
+                      sk.dev, st, 0, true);
+        finish_build(ctx, tree, st, true);
+    }
+    if (keys) { // sorted in place, as in the reference
+        sorted_keys_to_ref(ctx->opts, impl, n, sk.dev, st);
+        sk.copy_back();
+        FT_CUDA(cudaStreamSynchronize(st));
+    }
     FT_API_END
 }
 

@@ -33,11 +33,13 @@ struct TreeImpl {
     int       coord        = 0;
     void     *recs         = nullptr; // NodeRec<T>[cap-1]
     uint8_t  *height       = nullptr; // subtree height of internal nodes
-    int32_t  *counters     = nullptr; // refit arrival counters
+    int32_t  *counters     = nullptr; // arrivals at the splits between blocks of leaves
     int32_t  *leafcount    = nullptr; // leaves under each internal node (Karras range size)
+    void     *pack         = nullptr; // PackedPoint[cap]: the build's points in input order
     void     *qrec         = nullptr; // QRec[cap-1]: the fast walks' records (ft_qtree.cuh)
     void     *qpts         = nullptr; // QPoint[cap]: leaf positions in the walks' frame
-    uint32_t *qflag        = nullptr; // device word, not 0: the frame does not serve the tree
+    uint32_t *pend         = nullptr; // climbs between blocks of leaves (ft_treelet.cuh)
+    uint32_t *qflag        = nullptr; // device word (single trees: four), not 0: the frame does not serve the tree
     uint64_t *key_lo       = nullptr; // sorted keys (low word)
     uint64_t *key_hi       = nullptr; // sorted keys (high word, 126-bit keys only)
     uint64_t *tmp_lo       = nullptr; // sort ping-pong
@@ -46,7 +48,8 @@ struct TreeImpl {
     uint32_t *tmp_perm     = nullptr;
     void     *bbox         = nullptr; // 6 coords on the device
     void     *bbox_partial = nullptr; // per-block partial boxes
-    uint32_t *hist         = nullptr; // [digit position][256] counts, then offsets
+    int       sort_passes  = 0;       // passes (run or skipped) since the pairs were in the first buffers
+    uint32_t *hist         = nullptr; // [digit position][256] counts, then offsets; then the skip words
     uint32_t *lookback     = nullptr; // onesweep tile status
     size_t    lookback_words = 0;
     uint32_t *tile_counter = nullptr; // per-pass tile ticket
@@ -224,9 +227,13 @@ const uint32_t *sfc_query_order(Context &ctx, const ft_tree &tree, const void *q
 // root's height and the frame's flag (ft_build.cu).  Waits for the stream.
 struct TreeSummary {
     uint64_t mx[3];
-    uint32_t status, height, qflag, pad;
+    uint32_t status, height, qflag;
+    uint32_t parity;    // build_bvh: the sorted pairs lie in the second buffers (swapped by the call)
+    uint32_t long_runs; // build_bvh of 126-bit keys: sort by both words (nothing was built)
+    uint32_t pad;
 };
-void tree_summary(const ft_options &o, const ft_tree &tree, TreeSummary &out, cudaStream_t st);
+void tree_summary(const ft_options &o, ft_tree &tree, bool sorted, TreeSummary &out, cudaStream_t st);
+void sorted_keys_to_ref(const ft_options &o, const TreeImpl &s, size_t n, void *keys_ref, cudaStream_t st);
 void recompute_from_keys(Context &ctx, ft_tree &tree, cudaStream_t st);
 void refit_bvh(Context &ctx, ft_tree &tree, const void *x, const void *y, const void *z, size_t n, bool leaf_order,
                cudaStream_t st);
@@ -262,8 +269,8 @@ inline void stage_mark(Context *ctx, int i, cudaStream_t st) {
 // sort_items: keys per thread of the sort's tiles (0: the autotuner's choice for the shape,
 // else the default).
 void build_bvh(Context &ctx, ft_tree &tree, const void *x, const void *y, const void *z, size_t n,
-               const uint32_t *id, const int8_t *ghost, const void *bbox_host, void *caller_keys_dev,
-               cudaStream_t st, int sort_items = 0);
+               const uint32_t *id, const int8_t *ghost, const void *bbox_host, const void *caller_keys_dev,
+               cudaStream_t st, int sort_items = 0, bool full_sort = false);
 // Tile sizes the build's sort offers for one- or two-word keys (the default first).
 const int *sort_item_choices(int words, int *count);
 int        key_words_of(const ft_options &o);

@@ -1,0 +1,543 @@
+// ft_treelet.cuh -- topology, boxes and records of a radix tree over sorted keys, built bottom up
+// in blocks of consecutive leaves (src/hlbvh.hpp:852-969: Karras topology and refit).
+//
+// A node that covers leaves [l, r] joins the neighbour it shares the longer key prefix with: its
+// parent's split is the pair (r, r + 1) when delta(r) > delta(l - 1), else (l - 1, l), with
+// delta(x) the common prefix of the sorted keys x and x + 1 (the agglomerative form of the binary
+// radix tree, Apetrei 2014).  It is therefore the Karras tree of the same keys, and every node
+// takes its Karras number: a left child the last leaf it covers, a right child the first, the
+// root 0.
+//
+// A block takes kTreeletLeaves consecutive leaves.  Climbs meet in shared memory as long as both
+// sides of a split lie in the block; one whose split or sibling reaches beyond the block's edge
+// is left for the end.  Then the
+// block writes every node it formed -- boxes, children, counts and heights as coalesced arrays,
+// node records, and the fast walks' records -- all of whose descendants are in shared memory.
+// The climbs that left their blocks (about one leaf in 25) go on in global memory in a second
+// launch, where the second arrival at a split (one acquire-release exchange) forms the node, and a
+// third makes the walk records of the nodes formed there.
+//
+// Bound: with one climb step per level in global memory the refit alone was bound by the
+// latency of its atomics (1.27 ms for 10M uint64 points, after 0.34 ms of binary searches for the
+// topology, 0.60 ms of gather and 0.78 ms for the walk records).  In shared memory a step is some
+// tens of cycles, about one climb in 25 leaves the block, and the kernel moves each array once.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "ft_build_dev.cuh"
+#include "ft_common.cuh"
+#include "ft_qtree.cuh"
+
+namespace ft {
+
+// Which of a sort's two buffers holds its pairs: the passes that ran (skip: null, or a word per
+// pass, set when it moved nothing).
+FT_D int sort_parity(const uint32_t *skip, int passes) {
+    int p = 0;
+    for (int d = 0; d < passes; ++d) p ^= (skip && skip[d]) ? 0 : 1;
+    return p;
+}
+
+static constexpr int kTreeletLeaves = 512, kTreeletThreads = 256;
+
+// A point of the sort's input order in one 16- or 32-byte sector: the gather by permutation reads
+// one sector a leaf, not three.
+template <class T> struct alignas(sizeof(T) * 4) PackedPoint {
+    T x, y, z, pad; // pad: the low key word of 64-bit integer positions
+};
+
+// Where the leaves come from.
+enum TreeletSource {
+    LEAVES_PACKED = 0, // pack[perm[i]]: the build; also writes id, ghost, orig
+    LEAVES_IN_PLACE = 1, // the leaf slots hold them
+    LEAVES_MOVED = 2   // new positions x / y / z of the points in the leaves (refit)
+};
+
+template <class T> struct TreeletArgs {
+    int                       n, periodic;
+    const unsigned long long *klo, *khi; // sorted keys (LEAVES_PACKED: key / perm instead)
+    const unsigned long long *key[2];    // LEAVES_PACKED: the sort's buffers; those that hold the
+    const uint32_t           *perm[2];   // pairs follow from the passes that ran
+    const uint32_t           *skip;
+    int                       passes;
+    const uint32_t           *stop;      // null, or a word that is set when nothing is to be built
+    unsigned long long       *klo_out;   // LEAVES_PACKED, 126-bit keys: the sorted low words
+    const PackedPoint<T>     *pack;
+    const T                  *x, *y, *z; // LEAVES_MOVED
+    int                       leaf_order;
+    const uint32_t           *id;
+    const int8_t             *ghost;
+    const T                  *box; // the points' box (6 coordinates), from which the frame follows
+    T                        *soa[6];
+    int32_t                  *left, *right, *parent, *orig;
+    uint32_t                 *id_out;
+    int8_t                   *ghost_out;
+    NodeRec<T>               *recs;
+    uint8_t                  *height;
+    int32_t                  *leaves;
+    QRec                     *qrec;
+    QPoint                   *qpts;
+    uint32_t                 *qflag; // four words, zero: the tree's flag, nodes in `list`, entries of
+                                     // `pend` taken, entries of `pend`
+    int32_t                  *slot;       // n words, -1
+    uint32_t                 *pend;       // climbs that left their blocks
+    int32_t                  *list;       // nodes formed outside a block
+    uint32_t                 *status;
+};
+
+// A child of a node by its leaf range; `right`: a right child (which numbers it).
+struct TreeletChild {
+    int  l, r;
+    bool right;
+    FT_D int count() const { return r - l + 1; }
+    FT_D int node() const { return right ? l : r; } // internal number (l < r)
+};
+
+// The walk record of a node covering [l, r] with split s: its two children, then twice the child
+// with the most leaves (more than kBucket) replaced by its own two.  split(c): the split of
+// internal child c; box(c, b): its box.
+template <class T, class Split, class Box>
+FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, uint32_t *flag, Split split, Box box) {
+    TreeletChild ch[4] = {{l, s, false}, {s + 1, r, true}, {0, -1, false}, {0, -1, false}};
+    int          c     = 2;
+#pragma unroll
+    for (int step = 0; step < 2; ++step) {
+        int b = -1, most = kBucket;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if (i < c && ch[i].count() > most) {
+                b    = i;
+                most = ch[i].count();
+            }
+        if (b < 0) break;
+        const TreeletChild o  = b == 0 ? ch[0] : b == 1 ? ch[1] : ch[2];
+        const int          os = split(o);
+#pragma unroll
+        for (int i = 3; i > 0; --i)
+            if (i > b + 1) ch[i] = ch[i - 1]; // make room behind the opened child
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i == b) ch[i] = {o.l, os, false};
+            else if (i == b + 1) ch[i] = {os + 1, o.r, true};
+        }
+        ++c;
+    }
+    uint4     *dst = reinterpret_cast<uint4 *>(out);
+    uint32_t   w[32];
+    bool       dense = false;
+    const bool lossy = Coord<T>::is_float || f.shift > 0; // exact frames lose nothing
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        T b[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+        if (i < c) box(ch[i], b);
+        uint32_t hm   = 0;
+        bool     flat = true; // copies of one point: no frame tells them apart
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const uint32_t lo = (uint32_t)f.pos(b[2 * a], a), hi = (uint32_t)f.pos(b[2 * a + 1], a);
+            const uint32_t ce = lo + ((hi - lo) >> 1);
+            w[6 * i + a]      = ce;
+            w[6 * i + 3 + a]  = (hi - ce) + f.m;
+            hm                = max(hm, hi - ce);
+            flat              = flat && !(b[2 * a] < b[2 * a + 1]);
+        }
+        const int cnt = ch[i].count();
+        w[24 + i]     = i >= c ? kQEmpty : cnt <= kBucket ? qref_bucket(ch[i].l, cnt) : (uint32_t)ch[i].node();
+        w[28 + i]     = i >= c ? 0u : (uint32_t)cnt;
+        dense         = dense || (lossy && !flat && i < c && cnt > kDenseLeaves && hm <= kDenseUnits);
+    }
+    if (dense) atomicOr(flag, QFLAG_DENSE);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+}
+
+// A node's record for the exact traversals.
+template <class T>
+FT_D void treelet_noderec(NodeRec<T> *out, const T lb[6], const T rb[6], int lc, int rc, int nl, int nr, int hl, int hr) {
+    NodeRec<T> rec;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+        rec.lb[d] = lb[d];
+        rec.rb[d] = rb[d];
+    }
+    rec.l = lc;
+    rec.r = rc;
+#pragma unroll
+    for (int d = 0; d < (int)(sizeof(rec.pad) / 4); ++d) rec.pad[d] = 0;
+    rec.pad[0] = (int32_t)rec_child_info((uint32_t)nl, (uint32_t)hl);
+    rec.pad[1] = (int32_t)rec_child_info((uint32_t)nr, (uint32_t)hr);
+    const uint4 *src = reinterpret_cast<const uint4 *>(&rec);
+    uint4       *dst = reinterpret_cast<uint4 *>(out);
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(rec) / 16); ++i) dst[i] = src[i];
+}
+
+// delta of the adjacent sorted keys x and x + 1 (0 <= x < n - 1), plus one (0 is the border's).
+// (not below one: keys wider than the reference's would differ above its prefix)
+// lo: the sorted low words, or null (LEAVES_PACKED of 126-bit keys): they are in the packed points.
+template <class T> struct TreeletKeys {
+    const unsigned long long *lo, *hi;
+    const uint32_t           *perm;
+};
+template <class T, int KIND> FT_D int treelet_delta(const TreeletArgs<T> &a, const TreeletKeys<T> &key, int x) {
+    if constexpr (KIND == 2) {
+        const unsigned long long p = key.hi[x], q = key.hi[x + 1];
+        if (p != q) return max(clz64(p ^ q) - 1, 1);
+        const unsigned long long u = key.lo ? key.lo[x] : (unsigned long long)a.pack[key.perm[x]].pad,
+                                 v = key.lo ? key.lo[x + 1] : (unsigned long long)a.pack[key.perm[x + 1]].pad;
+        if (u != v) return 63 + clz64(u ^ v);
+        return 127 + clz64((unsigned long long)x ^ (unsigned long long)(x + 1));
+    } else {
+        const unsigned long long u = key.lo[x], v = key.lo[x + 1];
+        if (u != v) return max(clz64(u ^ v) - (KIND == 1 ? 1 : 0) + 1, 1);
+        return 64 + clz64((unsigned long long)x ^ (unsigned long long)(x + 1));
+    }
+}
+
+template <class T> struct TreeletShared {
+    T        lx[3][kTreeletLeaves];    // leaf positions
+    T        bx[6][kTreeletLeaves];    // boxes of the nodes formed here, by their number in the block
+    int32_t  slot[kTreeletLeaves];     // first arrival's far end at each split
+    uint16_t nl[kTreeletLeaves], nr[kTreeletLeaves], ns[kTreeletLeaves]; // a node's leaves and split
+    uint8_t  nh[kTreeletLeaves];       // height; 0: no node of this number here
+    uint8_t  delta[kTreeletLeaves + 1]; // pairs (j - 1, j)
+    uint16_t out[kTreeletLeaves];      // nodes (kTreeletLeaves +: leaves) that climb on outside
+    int      outs, base; // their number, and their place in the list
+};
+
+template <class T, int KIND, int SRC>
+__global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TreeletShared<T> &s  = *reinterpret_cast<TreeletShared<T> *>(smem_raw);
+    const int         n = a.n, tid = threadIdx.x;
+    const int         b0 = blockIdx.x * kTreeletLeaves, m = min(kTreeletLeaves, n - b0);
+    if (SRC == LEAVES_PACKED && a.stop && *a.stop) return; // grid-uniform
+    TreeletKeys<T> key = {a.klo, a.khi, nullptr};
+    if constexpr (SRC == LEAVES_PACKED) {
+        const int par = sort_parity(a.skip, a.passes);
+        key.perm      = a.perm[par];
+        if (KIND == 2) key = {nullptr, a.key[par], a.perm[par]};
+        else key.lo = a.key[par];
+    }
+    QFrame<T>         f;
+    f.make(a.box, n, a.periodic != 0);
+    if (!f.ok && blockIdx.x == 0 && tid == 0) atomicOr(a.qflag, f.flag());
+
+    // ---- leaves and deltas ----
+    if (tid == 0) s.outs = 0;
+    for (int j = tid; j < m; j += kTreeletThreads) {
+        const int i = b0 + j;
+        const int leaf = i + n - 1;
+        T         p[3];
+        if constexpr (SRC == LEAVES_PACKED) {
+            const uint32_t       src = key.perm[i];
+            const uint4         *q   = reinterpret_cast<const uint4 *>(a.pack + src);
+            uint4                v[sizeof(T) / 4];
+#pragma unroll
+            for (int c = 0; c < (int)sizeof(T) / 4; ++c) v[c] = __ldg(q + c);
+            const PackedPoint<T> &pt = *reinterpret_cast<const PackedPoint<T> *>(v);
+            p[0] = pt.x;
+            p[1] = pt.y;
+            p[2] = pt.z;
+            if constexpr (KIND == 2) a.klo_out[i] = (unsigned long long)pt.pad;
+            a.id_out[leaf]    = a.id ? a.id[src] : src;
+            a.ghost_out[leaf] = a.ghost ? a.ghost[src] : (int8_t)0;
+            a.orig[leaf]      = (int32_t)src;
+            if (i < n - 1) { // internal slots
+                a.id_out[i]    = 0u;
+                a.ghost_out[i] = (int8_t)0;
+                a.orig[i]      = 0;
+            }
+        } else if constexpr (SRC == LEAVES_MOVED) {
+            int64_t src = a.leaf_order ? (int64_t)i : (int64_t)a.orig[leaf];
+            if (src < 0 || src >= (int64_t)n) { // (the slot keeps its position)
+                atomicOr(a.status, STATUS_BAD_INPUT);
+                atomicOr(a.qflag, QFLAG_FRAME); // (it may lie outside the new positions' box)
+                p[0] = a.soa[0][leaf];
+                p[1] = a.soa[2][leaf];
+                p[2] = a.soa[4][leaf];
+            } else {
+                p[0] = a.x[src];
+                p[1] = a.y[src];
+                p[2] = a.z[src];
+            }
+        } else {
+            p[0] = a.soa[0][leaf];
+            p[1] = a.soa[2][leaf];
+            p[2] = a.soa[4][leaf];
+        }
+        if constexpr (SRC != LEAVES_IN_PLACE) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                a.soa[2 * d][leaf]     = p[d];
+                a.soa[2 * d + 1][leaf] = p[d];
+            }
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s.lx[d][j] = p[d];
+        a.qpts[i] = qpoint<T>(p[0], p[1], p[2], f, a.periodic != 0, a.qflag);
+        s.slot[j] = -1;
+        s.nh[j]   = 0;
+    }
+    for (int j = tid; j <= m; j += kTreeletThreads) {
+        const int x = b0 + j - 1;
+        s.delta[j]  = (x < 0 || x >= n - 1) ? 0 : (uint8_t)treelet_delta<T, KIND>(a, key, x);
+    }
+    __syncthreads();
+
+    // ---- climbs inside the block ----
+    for (int j = tid; j < m; j += kTreeletThreads) {
+        int l = j, r = j, sp = 0, h = 0;
+        T   box[6];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) box[2 * d] = box[2 * d + 1] = s.lx[d][j];
+        for (;;) {
+            const int  dl = s.delta[l], dr = s.delta[r + 1];
+            const bool root     = b0 + l == 0 && b0 + r == n - 1;
+            const bool up_right = dr > dl;
+            const int  ci       = root ? 0 : (up_right ? r : l);
+            if (l < r) { // a node formed by this thread
+#pragma unroll
+                for (int d = 0; d < 6; ++d) s.bx[d][ci] = box[d];
+                s.nl[ci] = (uint16_t)l;
+                s.nr[ci] = (uint16_t)r;
+                s.ns[ci] = (uint16_t)sp;
+                s.nh[ci] = (uint8_t)min(h, 255);
+            }
+            if (root) break;
+            const int split = up_right ? r : l - 1;
+            if (split < 0 || split + 1 >= m) { // the split lies on the block's edge
+                const int o = atomicAdd(&s.outs, 1);
+                s.out[o]    = (uint16_t)(l == r ? kTreeletLeaves + l : ci);
+                break;
+            }
+            __threadfence_block();
+            const int prev = atomicExch(&s.slot[split], up_right ? l : r);
+            if (prev < 0) break; // first arrival: the sibling forms the parent
+            s.slot[split] = -2;  // both have arrived
+            __threadfence_block();
+            const int sl = up_right ? split + 1 : prev, sr = up_right ? prev : split;
+            const int si = up_right ? sl : sr; // the sibling's number
+            T         sb[6];
+            int       sh = 0;
+            if (sl == sr) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) sb[2 * d] = sb[2 * d + 1] = s.lx[d][sl];
+            } else {
+                const volatile T *q = &s.bx[0][si];
+#pragma unroll
+                for (int d = 0; d < 6; ++d) sb[d] = q[d * kTreeletLeaves];
+                sh = *(const volatile uint8_t *)&s.nh[si];
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) { // (left, right) order, as the refit merges
+                box[2 * d]     = up_right ? box_min(box[2 * d], sb[2 * d]) : box_min(sb[2 * d], box[2 * d]);
+                box[2 * d + 1] = up_right ? box_max(box[2 * d + 1], sb[2 * d + 1]) : box_max(sb[2 * d + 1], box[2 * d + 1]);
+            }
+            h  = 1 + max(h, sh);
+            sp = split;
+            l  = min(l, sl);
+            r  = max(r, sr);
+        }
+    }
+    __syncthreads();
+    // splits where only one side arrived: the other reaches beyond the block's edge
+    for (int j = tid; j < m - 1; j += kTreeletThreads) {
+        const int far = s.slot[j];
+        if (far < 0) continue;
+        const int o  = atomicAdd(&s.outs, 1);
+        const int at = far <= j ? j : j + 1; // [far, j] or [j + 1, far]
+        s.out[o]     = (uint16_t)(far == at ? kTreeletLeaves + at : at);
+    }
+
+    // ---- the nodes formed here ----
+    auto child_box = [&](const TreeletChild &c, T b[6]) {
+        if (c.l == c.r) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) b[2 * d] = b[2 * d + 1] = s.lx[d][c.l - b0];
+        } else {
+#pragma unroll
+            for (int d = 0; d < 6; ++d) b[d] = s.bx[d][c.node() - b0];
+        }
+    };
+    for (int j = tid; j < m; j += kTreeletThreads) {
+        const int h = s.nh[j];
+        if (h == 0) continue;
+        const int          v = b0 + j, l = b0 + s.nl[j], r = b0 + s.nr[j], sp = b0 + s.ns[j];
+        const TreeletChild cl = {l, sp, false}, cr = {sp + 1, r, true};
+        const int          lc = l == sp ? l + n - 1 : sp, rc = sp + 1 == r ? r + n - 1 : sp + 1;
+        T                  lb[6], rb[6];
+        child_box(cl, lb);
+        child_box(cr, rb);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) a.soa[d][v] = s.bx[d][j];
+        a.left[v]   = lc;
+        a.right[v]  = rc;
+        a.parent[lc] = v;
+        a.parent[rc] = v;
+        a.leaves[v] = r - l + 1;
+        a.height[v] = (uint8_t)h;
+        if (v == 0) a.parent[0] = -1; // (number 0 is the root's)
+        treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, cl.count(), cr.count(), l == sp ? 0 : s.nh[sp - b0],
+                           sp + 1 == r ? 0 : s.nh[sp + 1 - b0]);
+        if (v == 0 || r - l + 1 > kBucket)
+            treelet_qrec<T>(l, r, sp, f, a.qrec + v, a.qflag,
+                            [&](const TreeletChild &c) { return b0 + (int)s.ns[c.node() - b0]; }, child_box);
+    }
+    __syncthreads();
+
+    // ---- climbs that leave the block ----
+    const int outs = s.outs;
+    if (tid == 0 && outs > 0) s.base = (int)atomicAdd(a.qflag + 3, (uint32_t)outs);
+    __syncthreads();
+    for (int o = tid; o < outs; o += kTreeletThreads) {
+        const int code = s.out[o];
+        uint32_t  w;
+        if (code >= kTreeletLeaves) w = ((uint32_t)(b0 + code - kTreeletLeaves) << 2) | 2u;
+        else w = ((uint32_t)(b0 + code) << 2) | (code == (int)s.nr[code] ? 1u : 0u);
+        a.pend[s.base + o] = w;
+    }
+}
+
+// The climbs that left their blocks: entries number << 2 | leaf << 1 | (number is the last leaf it
+// covers).  Warps take entries from a device counter (qflag[2]) and a lane whose climb ended
+// takes the next one: one step a lane and round, as many lanes as possible.
+template <class T, int KIND, int SRC>
+__global__ void __launch_bounds__(128) treelet_climb_kernel(const TreeletArgs<T> a) {
+    if (SRC == LEAVES_PACKED && a.stop && *a.stop) return;
+    TreeletKeys<T> key = {a.klo, a.khi, nullptr};
+    if constexpr (SRC == LEAVES_PACKED) {
+        const int par = sort_parity(a.skip, a.passes);
+        if (KIND == 2) key.hi = a.key[par]; // (the low words are written out by now)
+        else key.lo = a.key[par];
+        if (KIND == 2) key.lo = a.klo_out;
+    }
+    const unsigned FULL = 0xffffffffu;
+    const int      lane = threadIdx.x & 31, n = a.n, total = (int)a.qflag[3];
+    constexpr int  kChunk = 32;
+    int            next = 0, end = 0; // the warp's chunk of entries (warp-uniform)
+    bool           more = true, on = false;
+    int            l = 0, r = 0, h = 0, dl = 0, dr = 0;
+    T              box[6];
+    for (;;) {
+        unsigned idle = __ballot_sync(FULL, !on);
+        while (idle && more) {
+            if (next >= end) {
+                int b = 0;
+                if (lane == 0) b = (int)atomicAdd(a.qflag + 2, (uint32_t)kChunk);
+                b = __shfl_sync(FULL, b, 0);
+                if (b >= total) {
+                    more = false;
+                    break;
+                }
+                next = b;
+                end  = min(b + kChunk, total);
+            }
+            const int take = min(__popc(idle), end - next);
+            const int rank = __popc(idle & ((1u << lane) - 1u));
+            if (!on && rank < take) {
+                const uint32_t w = a.pend[next + rank];
+                const int      v = (int)(w >> 2);
+                const bool     leaf = (w & 2u) != 0u;
+                const int      c = leaf ? 1 : a.leaves[v], id = leaf ? v + n - 1 : v;
+                l = (leaf || !(w & 1u)) ? v : v - c + 1;
+                r = l + c - 1;
+                h = leaf ? 0 : (int)a.height[v];
+#pragma unroll
+                for (int d = 0; d < 6; ++d) box[d] = a.soa[d][id];
+                dl = l > 0 ? treelet_delta<T, KIND>(a, key, l - 1) : 0;
+                dr = r < n - 1 ? treelet_delta<T, KIND>(a, key, r) : 0;
+                on = true;
+            }
+            next += take;
+            idle = __ballot_sync(FULL, !on);
+        }
+        if (!__any_sync(FULL, on)) break;
+        if (on) {
+            // the node [l, r] -- box, height and everything below it -- is in global memory
+            const bool up_right = dr > dl;
+            const int  ci       = l == r ? l + n - 1 : (up_right ? r : l);
+            const int  split    = up_right ? r : l - 1;
+            int        prev;
+            asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;"
+                         : "=r"(prev)
+                         : "l"(a.slot + split), "r"(up_right ? l : r)
+                         : "memory");
+            if (prev < 0) {
+                on = false; // first arrival
+            } else {
+                const int sl = up_right ? split + 1 : prev, sr = up_right ? prev : split;
+                const int si = sl == sr ? sl + n - 1 : (up_right ? sl : sr);
+                const int L  = min(l, sl), R = max(r, sr);
+                T         sb[6], lb[6], rb[6];
+#pragma unroll
+                for (int d = 0; d < 6; ++d) sb[d] = __ldcg(a.soa[d] + si);
+                const int sh = sl == sr ? 0 : (int)__ldcg(a.height + si);
+                // only the far end's delta is new
+                if (up_right) dr = R < n - 1 ? treelet_delta<T, KIND>(a, key, R) : 0;
+                else dl = L > 0 ? treelet_delta<T, KIND>(a, key, L - 1) : 0;
+                const bool root = L == 0 && R == n - 1;
+                const int  v    = root ? 0 : (dr > dl ? R : L);
+                const int  lc = up_right ? ci : si, rc = up_right ? si : ci;
+                const int  hl = up_right ? h : sh, hr = up_right ? sh : h;
+#pragma unroll
+                for (int d = 0; d < 6; ++d) {
+                    lb[d] = up_right ? box[d] : sb[d];
+                    rb[d] = up_right ? sb[d] : box[d];
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    box[2 * d]     = box_min(lb[2 * d], rb[2 * d]);
+                    box[2 * d + 1] = box_max(lb[2 * d + 1], rb[2 * d + 1]);
+                }
+                h = min(255, 1 + max(hl, hr));
+#pragma unroll
+                for (int d = 0; d < 6; ++d) __stcg(a.soa[d] + v, box[d]);
+                __stcg(a.height + v, (uint8_t)h);
+                a.left[v]    = lc;
+                a.right[v]   = rc;
+                a.parent[lc] = v;
+                a.parent[rc] = v;
+                a.leaves[v]  = R - L + 1;
+                if (root) a.parent[0] = -1;
+                treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, split - L + 1, R - split, hl, hr);
+                if (root || R - L + 1 > kBucket) a.list[atomicAdd(a.qflag + 1, 1u)] = v;
+                l  = L;
+                r  = R;
+                on = !root;
+            }
+        }
+    }
+}
+
+// The walk records of the nodes formed outside a block (the list), from the finished arrays.
+template <class T>
+__global__ void __launch_bounds__(128) treelet_qrec_kernel(const TreeletArgs<T> a) {
+    if (a.stop && *a.stop) return;
+    const int n = a.n, cnt = (int)a.qflag[1];
+    QFrame<T> f;
+    f.make(a.box, n, a.periodic != 0);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
+        const int v = a.list[i];
+        // the node's leaves follow from its side: a left child's last leaf is its number
+        const int  c  = a.leaves[v];
+        const int  p  = v == 0 ? -1 : a.parent[v];
+        const bool lf = p >= 0 && a.left[p] == v;
+        const int  l  = v == 0 ? 0 : lf ? v - c + 1 : v, r = l + c - 1;
+        auto       split_of = [&](int node) {
+            const int x = a.left[node];
+            return x >= n - 1 ? x - (n - 1) : x;
+        };
+        treelet_qrec<T>(l, r, split_of(v), f, a.qrec + v, a.qflag,
+                        [&](const TreeletChild &ch) { return split_of(ch.node()); },
+                        [&](const TreeletChild &ch, T b[6]) {
+                            const int id = ch.l == ch.r ? ch.l + n - 1 : ch.node();
+#pragma unroll
+                            for (int d = 0; d < 6; ++d) b[d] = a.soa[d][id];
+                        });
+    }
+}
+
+} // namespace ft
