@@ -72,6 +72,19 @@ template <class T> FT_D typename Coord<T>::dist_t heap_key_ub(float key) {
     }
 }
 
+// Four 8-byte values to a 32-byte aligned address, streaming.
+template <class V> FT_D void st_sector(V *p, const V v[4]) {
+    static_assert(sizeof(V) == 8, "one sector");
+    unsigned long long w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if constexpr (std::is_floating_point<V>::value) w[i] = (unsigned long long)__double_as_longlong(v[i]);
+        else w[i] = v[i];
+    }
+    asm volatile("st.global.cs.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(w[0]), "l"(w[1]), "l"(w[2]), "l"(w[3])
+                 : "memory");
+}
+
 // A distance rounded up to a float (non-negative values): the key threshold of a bound for
 // float coordinates, whose keys are the distances themselves.
 template <class D> FT_D float key_up(D d) {
@@ -385,6 +398,11 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
             }
         }
     };
+    // whether a leaf may lie within the k-th distance (or the bound)
+    auto near_leaf = [&](const uint4 &v) -> bool {
+        if constexpr (std::is_same<T, float>::value) return !((float)exact_of(v) > kthr);
+        else return !(qdist(u, (int32_t)v.x, (int32_t)v.y, (int32_t)v.z, fr.m, fr.m, fr.m) > qlim);
+    };
     auto offer = [&](int32_t leaf) {
         const D     d  = exact(leaf);
         const float kd = heap_key<T>(d);
@@ -437,19 +455,21 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
         int      sp   = 0;
         bool     have = framed && active && n > 1;
         int      qc   = 0; // queued candidates
+        bool     room = true; // every lane's queue has room for a bucket (warp-uniform)
         // a bucket whose leaves all lie in the seeding window: first leaf in [w0, w1 - kBucket + 1]
         const uint32_t wref = kQBucket + (uint32_t)w0, wlen = (uint32_t)max(0, w1 - w0 + 2 - kBucket);
         for (;;) {
             const bool     inner = have && !(cur & kQBucket);
             const unsigned mi    = __ballot_sync(FULL, inner);
             const unsigned mb    = __ballot_sync(FULL, have && !inner);
-            if (!(mi | mb) || __any_sync(FULL, qc > kQueue - kBucket)) {
+            if (!(mi | mb) || !room) {
                 // rounds go on while many lanes have candidates or one has no room for a bucket
                 const int keep = (mi | mb) ? kOfferLanes : 1;
                 while (__popc(__ballot_sync(FULL, qc > 0)) >= keep || __any_sync(FULL, qc > kQueue - kBucket)) {
                     if (qc > 0) offer(queue[--qc * kThreads]);
                 }
                 if (!(mi | mb)) break;
+                room = true;
             }
             bool pop = false;
             if (mb == 0u || 2 * __popc(mi) >= __popc(mb)) {
@@ -514,13 +534,12 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                     for (int j = 0; j < kBucket; ++j) {
                         const uint4 v    = ld_rec16<COH>(p + min(j, cnt - 1));
                         const int   leaf = first + j; // (the query's own leaf lies in the window)
-                        bool        near;
-                        if constexpr (std::is_same<T, float>::value) near = !((float)exact_of(v) > kthr);
-                        else near = !(qdist(u, (int32_t)v.x, (int32_t)v.y, (int32_t)v.z, fr.m, fr.m, fr.m) > qlim);
+                        const bool  near = near_leaf(v); // (before the test: all loads in flight at once)
                         if (j < cnt && near && (leaf < w0 || leaf > w1)) queue[qc++ * kThreads] = leaf;
                     }
                     pop = true;
                 }
+                room = !__any_sync(FULL, qc > kQueue - kBucket);
             }
             __syncwarp();
             if (pop) {
@@ -647,19 +666,36 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                 if (HD(i) == HD(i - 1)) flag = true;
         }
         const size_t off = (size_t)q * (size_t)k;
-        for (int i = 0; i < k; ++i) {
+        auto         row = [&](int i, unsigned long long &id, D &dd) {
             if (i < count) {
-                const HeapEntry e    = HE(i);
-                const int32_t   leaf = e.leaf;
-                D               dd;
-                if constexpr (heap_keyed<T>()) dd = exact(leaf);
+                const HeapEntry e = HE(i);
+                if constexpr (heap_keyed<T>()) dd = exact(e.leaf);
                 else dd = (D)e.key;
-                __stcs(out_idx + off + i, (unsigned long long)(long long)(ret_orig ? t.orig_idx[leaf + n - 1] : leaf));
-                __stcs(out_dist + off + i, dd);
+                id = (unsigned long long)(long long)(ret_orig ? t.orig_idx[e.leaf + n - 1] : e.leaf);
             } else {
-                __stcs(out_idx + off + i, ~0ull);
-                __stcs(out_dist + off + i, dist_missing<D>());
+                id = ~0ull;
+                dd = dist_missing<D>();
             }
+        };
+        // four entries a store where the rows allow it: whole 32-byte sectors
+        const bool vec = (k & 3) == 0 && (((uintptr_t)out_idx | (uintptr_t)out_dist) & 31) == 0;
+        int        i   = 0;
+        if (vec) {
+            for (; i < k; i += 4) {
+                unsigned long long id[4];
+                D                  dd[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) row(i + j, id[j], dd[j]);
+                st_sector(out_idx + off + i, id);
+                st_sector(out_dist + off + i, dd);
+            }
+        }
+        for (; i < k; ++i) {
+            unsigned long long id;
+            D                  dd;
+            row(i, id, dd);
+            __stcs(out_idx + off + i, id);
+            __stcs(out_dist + off + i, dd);
         }
     }
     const bool to_replay = (active && flag) || force_replay;
