@@ -14,16 +14,16 @@
 
 namespace ft {
 
-// Resident two-warp blocks the walk is compiled for (86 registers, no spills; 8 / 10 / 11 blocks
-// 6.20 / 6.12 / 6.66 ms on 2M clustered uint64 points, k = 32: the 11th needs shorter queues).
+// Resident two-warp blocks the walk is compiled for (90 registers, no spills; 9 / 10 / 11 blocks
+// 5.80 / 5.81 / 5.89 ms on 2M clustered uint64 points, k = 32).
 #ifndef FT_FAST_MINB
 #define FT_FAST_MINB 10
 #endif
 // The walk's schedule, measured on the same points (with it 2.2 times the lanes of a walk that
 // lets each lane branch on its own run together, 14.4 -> 6.1 ms; the walk with exact 64-bit boxes
 // down to single leaves took 9.4 ms):
-//  * a warp expands while at least half as many lanes want to as wait for a bucket (as many:
-//    6.77, eight lanes 6.82, sixteen 7.23 against 6.69 ms);
+//  * a warp expands while as many lanes want to as wait with a bucket (half / a quarter as many:
+//    5.77 / 5.95 against 5.69 ms; every lane waiting at its first bucket: 5.82 ms);
 //  * queues of 16 candidates a lane (12 / 24: 6.97 / 7.28 ms, the longer ones cost a block), offered
 //    while kOfferLanes lanes have one (6 / 12 / 18 lanes: 6.91 / 6.82 / 6.82 ms).
 static constexpr int kQueue = 16, kOfferLanes = 12;
@@ -446,12 +446,13 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
     // the k-th distance; leaves at exactly that distance reach insert_k and raise the tie flag.
     const bool binary_walk = active && !framed && n > 1;
     {
-        // Warp-synchronous: lanes whose next node is an internal one expand it, lanes whose next
-        // is a bucket wait until few lanes are left to expand, then all waiting lanes test their
-        // buckets together.  Leaves within reach are queued and offered to the heaps when several
+        // Warp-synchronous: lanes whose next node is an internal one expand it; a lane that meets a
+        // bucket puts it aside and goes on, and waits at its second one, until more lanes wait
+        // than expand.  Then every lane with a bucket aside tests it.  Leaves within reach are queued and offered to the heaps when several
         // lanes have some (one a lane and round: the exact distances and the heaps' sifts run
         // with most lanes).
-        uint32_t cur  = 0; // node or bucket
+        uint32_t cur  = 0; // next: a node or a bucket
+        uint32_t pb   = kQEmpty; // a bucket put aside
         int      sp   = 0;
         bool     have = framed && active && n > 1;
         int      qc   = 0; // queued candidates
@@ -461,7 +462,7 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
         for (;;) {
             const bool     inner = have && !(cur & kQBucket);
             const unsigned mi    = __ballot_sync(FULL, inner);
-            const unsigned mb    = __ballot_sync(FULL, have && !inner);
+            const unsigned mb    = __ballot_sync(FULL, !inner && pb != kQEmpty);
             if (!(mi | mb) || !room) {
                 // rounds go on while many lanes have candidates or one has no room for a bucket
                 const int keep = (mi | mb) ? kOfferLanes : 1;
@@ -472,7 +473,7 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                 room = true;
             }
             bool pop = false;
-            if (mb == 0u || 2 * __popc(mi) >= __popc(mb)) {
+            if (mb == 0u || __popc(mi) >= __popc(mb)) {
                 if (inner) {
                     --budget;
                     ++visits;
@@ -515,6 +516,7 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                         if (budget < 0) atomicOr(status, STATUS_TRAVERSAL_LIMIT);
                         flag = true;
                         have = false;
+                        pb   = kQEmpty;
                     } else {
 #pragma unroll
                         for (int i = 0; i < 3; ++i)
@@ -522,13 +524,17 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                         sp += max(nv - 1, 0);
                         cur = nv == 1 ? oc[0] : nv == 2 ? oc[1] : nv == 3 ? oc[2] : oc[3];
                         pop = nv == 0;
+                        if (!pop && (cur & kQBucket) && pb == kQEmpty) {
+                            pb  = cur;
+                            pop = true;
+                        }
                     }
                 }
             } else {
                 // buckets: leaves whose bound is within reach join the lane's queue
-                if (have && !inner) {
+                if (pb != kQEmpty) {
                     ++visits;
-                    const int    first = qref_first(cur), cnt = qref_count(cur);
+                    const int    first = qref_first(pb), cnt = qref_count(pb);
                     const uint4 *p     = pts + first;
 #pragma unroll
                     for (int j = 0; j < kBucket; ++j) {
@@ -537,7 +543,8 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                         const bool  near = near_leaf(v); // (before the test: all loads in flight at once)
                         if (j < cnt && near && (leaf < w0 || leaf > w1)) queue[qc++ * kThreads] = leaf;
                     }
-                    pop = true;
+                    pb  = (have && !inner) ? cur : kQEmpty;
+                    pop = have && !inner;
                 }
                 room = !__any_sync(FULL, qc > kQueue - kBucket);
             }
@@ -547,7 +554,11 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                 while (sp > 0) {
                     const unsigned long long e = lane_stack[--sp];
                     if (!(__uint_as_float((uint32_t)(e >> 32)) > qlim)) {
-                        cur  = (uint32_t)e;
+                        cur = (uint32_t)e;
+                        if ((cur & kQBucket) && pb == kQEmpty) {
+                            pb = cur;
+                            continue;
+                        }
                         have = true;
                         break;
                     }
