@@ -227,6 +227,12 @@ template <bool COH> FT_D uint4 ld_rec16(const uint4 *p) {
     }
 }
 
+// Four 8-byte words to a 32-byte aligned address: one whole sector a store.
+FT_D void st_words32(void *p, const unsigned long long w[4]) {
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(w[0]), "l"(w[1]), "l"(w[2]), "l"(w[3])
+                 : "memory");
+}
+
 // load_rec plus the two children's info words (rec_child_info).
 template <class T, bool COH = false>
 FT_D void load_rec_info(const NodeRec<T> *recs, int node, T lb[6], T rb[6], int &l, int &r, uint32_t &il,

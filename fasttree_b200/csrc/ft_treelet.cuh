@@ -124,7 +124,6 @@ FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, uint3
         }
         ++c;
     }
-    uint4     *dst = reinterpret_cast<uint4 *>(out);
     uint32_t   w[32];
     bool       dense = false;
     const bool lossy = Coord<T>::is_float || f.shift > 0; // exact frames lose nothing
@@ -150,7 +149,12 @@ FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, uint3
     }
     if (dense) atomicOr(flag, QFLAG_DENSE);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+    for (int i = 0; i < 4; ++i) {
+        unsigned long long v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = (unsigned long long)w[8 * i + 2 * j + 1] << 32 | w[8 * i + 2 * j];
+        st_words32(reinterpret_cast<unsigned char *>(out) + 32 * i, v);
+    }
 }
 
 // A node's record for the exact traversals.
@@ -168,10 +172,12 @@ FT_D void treelet_noderec(NodeRec<T> *out, const T lb[6], const T rb[6], int lc,
     for (int d = 0; d < (int)(sizeof(rec.pad) / 4); ++d) rec.pad[d] = 0;
     rec.pad[0] = (int32_t)rec_child_info((uint32_t)nl, (uint32_t)hl);
     rec.pad[1] = (int32_t)rec_child_info((uint32_t)nr, (uint32_t)hr);
-    const uint4 *src = reinterpret_cast<const uint4 *>(&rec);
-    uint4       *dst = reinterpret_cast<uint4 *>(out);
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&rec);
 #pragma unroll
-    for (int i = 0; i < (int)(sizeof(rec) / 16); ++i) dst[i] = src[i];
+    for (int i = 0; i < (int)(sizeof(rec) / 32); ++i) {
+        const unsigned long long v[4] = {src[4 * i], src[4 * i + 1], src[4 * i + 2], src[4 * i + 3]};
+        st_words32(reinterpret_cast<unsigned char *>(out) + 32 * i, v);
+    }
 }
 
 // delta of the adjacent sorted keys x and x + 1 (0 <= x < n - 1), plus one (0 is the border's).
