@@ -766,7 +766,7 @@ void ensure_scratch(TreeImpl &s, const ft_options &o, size_t n) {
     s.qrec      = alloc_dev<QRec>(cap > 1 ? cap - 1 : 1);
     s.qpts      = alloc_dev<QPoint>(cap);
     s.qflag     = (uint32_t *)alloc_dev<uint32_t>(4);
-    s.pend      = (uint32_t *)alloc_dev<uint32_t>(cap);
+    s.pend      = (uint32_t *)alloc_dev<uint32_t>(2 * cap + 2 * (cap / kTreeletLeaves + 1));
     s.key_lo   = (uint64_t *)alloc_dev<uint64_t>(cap);
     s.tmp_lo   = (uint64_t *)alloc_dev<uint64_t>(cap);
     if (W == 2) {
@@ -1042,7 +1042,10 @@ static void build_treelets(const ft_options &o, ft_tree &t, TreeImpl &s, size_t 
     a.qpts      = (QPoint *)s.qpts;
     a.qflag     = s.qflag;
     a.slot      = s.counters;
-    a.pend      = s.pend;
+    uint32_t *list[2]  = {s.pend, s.pend + s.cap}; // (the four lie in one allocation)
+    uint32_t *count[2] = {s.pend + 2 * s.cap, s.pend + 2 * s.cap + s.cap / kTreeletLeaves + 1};
+    a.pend             = list[0];
+    a.pend_count       = count[0];
     a.list      = (int32_t *)s.lookback; // (at least n words; the sort is done with them)
     a.status    = s.status;
     const bool many = n > (size_t)kTreeletLeaves;
@@ -1054,8 +1057,20 @@ static void build_treelets(const ft_options &o, ft_tree &t, TreeImpl &s, size_t 
         auto fn = treelet_kernel<T, decltype(kind)::value, SRC>;
         FT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TreeletShared<T>)));
         fn<<<blocks, kTreeletThreads, sizeof(TreeletShared<T>), st>>>(a);
-        if (many) // (a warp per 32 entries of some 20 a block, at most a few per SM)
-            treelet_climb_kernel<T, decltype(kind)::value, SRC><<<grid_for(n / 16, 128, 148 * 8), 128, 0, st>>>(a);
+        if (!many) return;
+        auto join = treelet_join_kernel<T, decltype(kind)::value, SRC>;
+        FT_CUDA(cudaFuncSetAttribute(join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JoinShared<T>)));
+        JoinLevel lv{list[0], count[0], (int)blocks, (size_t)kTreeletLeaves, list[1], count[1]};
+        for (;;) {
+            const int groups = (lv.segs + kJoinBlocks - 1) / kJoinBlocks;
+            if (groups == 1) lv.out_count = nullptr;
+            join<<<groups, kJoinThreads, sizeof(JoinShared<T>), st>>>(a, lv);
+            if (groups == 1) break;
+            uint32_t *const from = const_cast<uint32_t *>(lv.in), *const from_count = const_cast<uint32_t *>(lv.in_count);
+            lv = JoinLevel{lv.out, lv.out_count, groups, lv.stride * kJoinBlocks, from, from_count};
+        }
+        a.left_over = lv.out;
+        treelet_climb_kernel<T, decltype(kind)::value, SRC><<<grid_for(n / 64, 128, 148 * 4), 128, 0, st>>>(a);
     };
     if constexpr (Coord<T>::key_words == 2) run(std::integral_constant<int, 2>{});
     else if (delta_kind(o) == 0) run(std::integral_constant<int, 0>{});

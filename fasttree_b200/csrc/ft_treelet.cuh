@@ -13,14 +13,20 @@
 // is left for the end.  Then the
 // block writes every node it formed -- boxes, children, counts and heights as coalesced arrays,
 // node records, and the fast walks' records -- all of whose descendants are in shared memory.
-// The climbs that left their blocks (about one leaf in 25) go on in global memory in a second
-// launch, where the second arrival at a split (one acquire-release exchange) forms the node, and a
-// third makes the walk records of the nodes formed there.
+// The climbs that left their blocks (about one leaf in 25) meet again the same way, the climbs of
+// 16 blocks in one block, level by level (treelet_join_kernel).  Climbs that too large groups pass
+// on end in global memory, where the second arrival at a split (one acquire-release exchange)
+// forms the node; a last launch makes the walk records of the nodes formed outside a block of
+// leaves.
 //
 // Bound: with one climb step per level in global memory the refit alone was bound by the
 // latency of its atomics (1.27 ms for 10M uint64 points, after 0.34 ms of binary searches for the
-// topology, 0.60 ms of gather and 0.78 ms for the walk records).  In shared memory a step is some
-// tens of cycles, about one climb in 25 leaves the block, and the kernel moves each array once.
+// topology, 0.60 ms of gather and 0.78 ms for the walk records: 3.0 ms).  In shared memory a step
+// is some tens of cycles and each array moves once: treelets 1.31, joins 0.19, walk records of the
+// nodes outside 0.05 ms.  The treelets move 3.0 TB/s; what holds them back is the L1's share of the
+// scattered record stores (32-byte stores: 3.09 -> 2.96 ms for the build) and the barriers between
+// their phases.  Leaves / threads of a block: 512 / 256 2.96, 1024 / 512 2.95 (refit of 3M float64
+// points 764 against 742 us), 256 / 128 3.09, 512 / 512 3.13 ms.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -80,9 +86,11 @@ template <class T> struct TreeletArgs {
     QRec                     *qrec;
     QPoint                   *qpts;
     uint32_t                 *qflag; // four words, zero: the tree's flag, nodes in `list`, entries of
-                                     // `pend` taken, entries of `pend`
+                                     // `left_over` taken, entries of `left_over`
     int32_t                  *slot;       // n words, -1
-    uint32_t                 *pend;       // climbs that left their blocks
+    uint32_t                 *pend, *pend_count; // climbs that left a block of leaves: from its first
+                                                 // leaf's place on, and their number (null: one block)
+    uint32_t                 *left_over;  // climbs that left the joins too
     int32_t                  *list;       // nodes formed outside a block
     uint32_t                 *status;
 };
@@ -210,7 +218,7 @@ template <class T> struct TreeletShared {
     uint8_t  nh[kTreeletLeaves];       // height; 0: no node of this number here
     uint8_t  delta[kTreeletLeaves + 1]; // pairs (j - 1, j)
     uint16_t out[kTreeletLeaves];      // nodes (kTreeletLeaves +: leaves) that climb on outside
-    int      outs, base; // their number, and their place in the list
+    int      outs; // their number
 };
 
 template <class T, int KIND, int SRC>
@@ -396,19 +404,222 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
 
     // ---- climbs that leave the block ----
     const int outs = s.outs;
-    if (tid == 0 && outs > 0) s.base = (int)atomicAdd(a.qflag + 3, (uint32_t)outs);
-    __syncthreads();
-    for (int o = tid; o < outs; o += kTreeletThreads) {
+    if (tid == 0 && a.pend_count) a.pend_count[blockIdx.x] = (uint32_t)outs;
+    for (int o = tid; o < outs; o += kTreeletThreads) { // (into this block's part of the array)
         const int code = s.out[o];
         uint32_t  w;
         if (code >= kTreeletLeaves) w = ((uint32_t)(b0 + code - kTreeletLeaves) << 2) | 2u;
         else w = ((uint32_t)(b0 + code) << 2) | (code == (int)s.nr[code] ? 1u : 0u);
-        a.pend[s.base + o] = w;
+        a.pend[b0 + o] = w;
     }
 }
 
-// The climbs that left their blocks: entries number << 2 | leaf << 1 | (number is the last leaf it
-// covers).  Warps take entries from a device counter (qflag[2]) and a lane whose climb ended
+// Leaf range of a climb that left its block (number << 2 | leaf << 1 | (number is the last leaf)).
+template <class T> FT_D void treelet_range(const TreeletArgs<T> &a, uint32_t w, int &l, int &r) {
+    const int  v    = (int)(w >> 2);
+    const bool leaf = (w & 2u) != 0u;
+    const int  c    = leaf ? 1 : a.leaves[v];
+    l               = (leaf || !(w & 1u)) ? v : v - c + 1;
+    r               = l + c - 1;
+}
+
+// The climbs that left kJoinBlocks consecutive blocks, in one block: the same as treelet_kernel's
+// with those subtrees in the leaves' place (some 20 a block).  Launched level by level, the blocks
+// of one level being the next one's groups, until one block is left; a group of more than
+// kJoinItems passes its climbs on as they are.  What the last level leaves goes to
+// treelet_climb_kernel (a level takes 12 to 16 us, the climbs of 100K points one by one 44 us).
+struct JoinLevel {
+    const uint32_t *in, *in_count; // segment b: in_count[b] entries from in + b * stride on
+    int             segs;
+    size_t          stride;
+    uint32_t       *out, *out_count; // this level's segments; out_count null: one list, its length
+};                                   // in qflag[3]
+static constexpr int kJoinBlocks = 16, kJoinItems = 512, kJoinThreads = 256;
+template <class T> struct JoinShared {
+    T        ib[6][kJoinItems]; // the items' boxes
+    T        bx[6][kJoinItems]; // boxes of the nodes formed here
+    int32_t  il[kJoinItems], ir[kJoinItems], slot[kJoinItems];
+    uint32_t code[kJoinItems]; // unsorted entries
+    uint32_t out[kJoinItems];
+    uint16_t nl[kJoinItems], nr[kJoinItems], ns[kJoinItems];
+    uint8_t  ih[kJoinItems], nh[kJoinItems], delta[kJoinItems + 1];
+    int      start[kJoinBlocks + 1];
+    int      outs, base;
+};
+template <class T, int KIND, int SRC>
+__global__ void __launch_bounds__(kJoinThreads) treelet_join_kernel(const TreeletArgs<T> a, const JoinLevel lv) {
+    if (SRC == LEAVES_PACKED && a.stop && *a.stop) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    JoinShared<T> &s   = *reinterpret_cast<JoinShared<T> *>(smem_raw);
+    const int      tid = threadIdx.x, n = a.n;
+    const int      t0 = blockIdx.x * kJoinBlocks, nb = min(kJoinBlocks, lv.segs - t0);
+    uint32_t      *out = lv.out + (lv.out_count ? (size_t)t0 * lv.stride : 0);
+    TreeletKeys<T> key = {a.klo, a.khi, nullptr};
+    if constexpr (SRC == LEAVES_PACKED) {
+        const int par = sort_parity(a.skip, a.passes);
+        if (KIND == 2) key = {a.klo_out, a.key[par], nullptr}; // (the low words are written out by now)
+        else key.lo = a.key[par];
+    }
+    if (tid == 0) {
+        int c = 0;
+        for (int b = 0; b < nb; ++b) {
+            s.start[b] = c;
+            c += (int)lv.in_count[t0 + b];
+        }
+        s.start[nb] = c;
+        s.outs      = 0;
+    }
+    __syncthreads();
+    const int m = s.start[nb];
+    auto place = [&](int count) { // where this block's entries go (every thread calls it)
+        if (tid == 0) {
+            if (lv.out_count) lv.out_count[blockIdx.x] = (uint32_t)count;
+            s.base = lv.out_count ? 0 : (int)atomicAdd(a.qflag + 3, (uint32_t)count);
+        }
+        __syncthreads();
+        return out + s.base;
+    };
+    if (m > kJoinItems) { // block-uniform: passed on as they are
+        uint32_t *to = place(m);
+        for (int b = 0; b < nb; ++b) {
+            const int c = s.start[b + 1] - s.start[b];
+            for (int o = tid; o < c; o += kJoinThreads) to[s.start[b] + o] = lv.in[(size_t)(t0 + b) * lv.stride + o];
+        }
+        return;
+    }
+    // ---- items in leaf order: by block, and inside a block by rank among its own ----
+    for (int i = tid; i < m; i += kJoinThreads) {
+        int b = 0;
+        while (i >= s.start[b + 1]) ++b;
+        const uint32_t w = lv.in[(size_t)(t0 + b) * lv.stride + (i - s.start[b])];
+        s.code[i]        = w;
+        int l, r;
+        treelet_range<T>(a, w, l, r);
+        s.slot[i] = l; // (for the ranks)
+    }
+    __syncthreads();
+    for (int i = tid; i < m; i += kJoinThreads) {
+        int b = 0;
+        while (i >= s.start[b + 1]) ++b;
+        const int mine = s.slot[i];
+        int       at   = s.start[b];
+        for (int o = s.start[b]; o < s.start[b + 1]; ++o) at += s.slot[o] < mine ? 1 : 0;
+        const uint32_t w = s.code[i];
+        int            l, r;
+        treelet_range<T>(a, w, l, r);
+        const int id = l == r ? l + n - 1 : (int)(w >> 2);
+        s.il[at]     = l;
+        s.ir[at]     = r;
+        s.ih[at]     = l == r ? (uint8_t)0 : a.height[id];
+        s.nh[at]     = 0;
+#pragma unroll
+        for (int d = 0; d < 6; ++d) s.ib[d][at] = a.soa[d][id];
+    }
+    __syncthreads();
+    for (int i = tid; i <= m && m > 0; i += kJoinThreads) {
+        const int x = i == 0 ? s.il[0] - 1 : s.ir[i - 1]; // the pair between items i - 1 and i
+        s.delta[i]  = (x < 0 || x >= n - 1) ? 0 : (uint8_t)treelet_delta<T, KIND>(a, key, x);
+        if (i < m) s.slot[i] = -1;
+    }
+    __syncthreads();
+    // ---- climbs ----
+    for (int j = tid; j < m; j += kJoinThreads) {
+        int l = j, r = j, sp = 0, h = s.ih[j];
+        T   box[6];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) box[d] = s.ib[d][j];
+        for (;;) {
+            const int  dl = s.delta[l], dr = s.delta[r + 1];
+            const bool root     = s.il[l] == 0 && s.ir[r] == n - 1;
+            const bool up_right = dr > dl;
+            const int  ci       = root ? 0 : (up_right ? r : l);
+            if (l < r) {
+#pragma unroll
+                for (int d = 0; d < 6; ++d) s.bx[d][ci] = box[d];
+                s.nl[ci] = (uint16_t)l;
+                s.nr[ci] = (uint16_t)r;
+                s.ns[ci] = (uint16_t)sp;
+                s.nh[ci] = (uint8_t)min(h, 255);
+            }
+            if (root) break;
+            const int split = up_right ? r : l - 1;
+            if (split < 0 || split + 1 >= m) {
+                s.out[atomicAdd(&s.outs, 1)] = (uint32_t)ci | (l == r ? 0x80000000u : 0u) | (up_right ? 0x40000000u : 0u);
+                break;
+            }
+            __threadfence_block();
+            const int prev = atomicExch(&s.slot[split], up_right ? l : r);
+            if (prev < 0) break; // first arrival
+            s.slot[split] = -2;
+            __threadfence_block();
+            const int sl = up_right ? split + 1 : prev, sr = up_right ? prev : split;
+            const int si = up_right ? sl : sr;
+            T         sb[6];
+            const volatile T *q = sl == sr ? &s.ib[0][si] : &s.bx[0][si];
+#pragma unroll
+            for (int d = 0; d < 6; ++d) sb[d] = q[d * kJoinItems];
+            const int sh = sl == sr ? s.ih[si] : *(const volatile uint8_t *)&s.nh[si];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) { // (left, right) order
+                box[2 * d]     = up_right ? box_min(box[2 * d], sb[2 * d]) : box_min(sb[2 * d], box[2 * d]);
+                box[2 * d + 1] = up_right ? box_max(box[2 * d + 1], sb[2 * d + 1]) : box_max(sb[2 * d + 1], box[2 * d + 1]);
+            }
+            h  = 1 + max(h, sh);
+            sp = split;
+            l  = min(l, sl);
+            r  = max(r, sr);
+        }
+    }
+    __syncthreads();
+    for (int j = tid; j < m - 1; j += kJoinThreads) { // splits where only one side arrived
+        const int far = s.slot[j];
+        if (far < 0) continue;
+        const bool up = far <= j;
+        const int  at = up ? j : j + 1;
+        s.out[atomicAdd(&s.outs, 1)] = (uint32_t)at | (far == at ? 0x80000000u : 0u) | (up ? 0x40000000u : 0u);
+    }
+    // ---- the nodes formed here ----
+    for (int j = tid; j < m; j += kJoinThreads) {
+        const int h = s.nh[j];
+        if (h == 0) continue;
+        const int  x = s.nl[j], y = s.nr[j], sp = s.ns[j];
+        const int  l = s.il[x], r = s.ir[y], sl = s.ir[sp]; // the split's last leaf
+        const bool root = l == 0 && r == n - 1;
+        const int  v    = root ? 0 : (j == y ? r : l);
+        const int  lc = l == sl ? l + n - 1 : sl, rc = sl + 1 == r ? r + n - 1 : sl + 1;
+        T          lb[6], rb[6];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+            lb[d] = x == sp ? s.ib[d][x] : s.bx[d][sp];
+            rb[d] = sp + 1 == y ? s.ib[d][y] : s.bx[d][sp + 1];
+            a.soa[d][v] = s.bx[d][j];
+        }
+        a.left[v]    = lc;
+        a.right[v]   = rc;
+        a.parent[lc] = v;
+        a.parent[rc] = v;
+        a.leaves[v]  = r - l + 1;
+        a.height[v]  = (uint8_t)h;
+        if (root) a.parent[0] = -1;
+        treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, sl - l + 1, r - sl, x == sp ? s.ih[x] : s.nh[sp],
+                           sp + 1 == y ? s.ih[y] : s.nh[sp + 1]);
+        if (root || r - l + 1 > kBucket) a.list[atomicAdd(a.qflag + 1, 1u)] = v;
+    }
+    __syncthreads();
+    // ---- climbs that leave this block too ----
+    const int outs = s.outs;
+    uint32_t *to   = place(outs);
+    for (int o = tid; o < outs; o += kJoinThreads) {
+        const uint32_t w  = s.out[o];
+        const int      at = (int)(w & 0xffffu);
+        const bool     up = (w & 0x40000000u) != 0u;
+        const int      x = (w & 0x80000000u) ? at : (int)s.nl[at], y = (w & 0x80000000u) ? at : (int)s.nr[at];
+        const int      l = s.il[x], r = s.ir[y];
+        to[o] = l == r ? ((uint32_t)l << 2) | 2u : up ? ((uint32_t)r << 2) | 1u : (uint32_t)l << 2;
+    }
+}
+
+// The climbs that are left (a.left_over).  Warps take entries from a device counter (qflag[2]) and a lane whose climb ended
 // takes the next one: one step a lane and round, as many lanes as possible.
 template <class T, int KIND, int SRC>
 __global__ void __launch_bounds__(128) treelet_climb_kernel(const TreeletArgs<T> a) {
@@ -444,13 +655,10 @@ __global__ void __launch_bounds__(128) treelet_climb_kernel(const TreeletArgs<T>
             const int take = min(__popc(idle), end - next);
             const int rank = __popc(idle & ((1u << lane) - 1u));
             if (!on && rank < take) {
-                const uint32_t w = a.pend[next + rank];
-                const int      v = (int)(w >> 2);
-                const bool     leaf = (w & 2u) != 0u;
-                const int      c = leaf ? 1 : a.leaves[v], id = leaf ? v + n - 1 : v;
-                l = (leaf || !(w & 1u)) ? v : v - c + 1;
-                r = l + c - 1;
-                h = leaf ? 0 : (int)a.height[v];
+                const uint32_t w = a.left_over[next + rank];
+                treelet_range<T>(a, w, l, r);
+                const int id = l == r ? l + n - 1 : (int)(w >> 2);
+                h = l == r ? 0 : (int)a.height[id];
 #pragma unroll
                 for (int d = 0; d < 6; ++d) box[d] = a.soa[d][id];
                 dl = l > 0 ? treelet_delta<T, KIND>(a, key, l - 1) : 0;
