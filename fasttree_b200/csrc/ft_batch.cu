@@ -237,7 +237,8 @@ __global__ void __launch_bounds__(256)
 // 7. refit of every set with >= 2 leaves (climbs from its leaves), then the root height of
 //    each set
 // =========================================================================================
-// The same refit with every lane kept busy (as refit_stream_kernel for one tree): warps take
+// A climb ends at its first arrival at a node, so one thread per leaf would leave most lanes of a
+// warp idle while its longest climb goes on.  Here warps take
 // leaves in chunks from a device counter (*work, zero at launch) and a lane whose climb ended
 // takes the next leaf, finding its set by binary search over the offsets.
 template <class T>

@@ -305,14 +305,4 @@ FT_D int refit_step(int curr, int n, const int32_t *__restrict__ left, const int
     return p;
 }
 
-template <class T>
-FT_D void refit_leaf(int leaf, int n, const int32_t *__restrict__ left, const int32_t *__restrict__ right,
-                     const int32_t *__restrict__ parent, T *const *soa, NodeRec<T> *recs, uint8_t *height,
-                     int32_t *counters, const int32_t *__restrict__ leaves) {
-    int curr  = leaf + n - 1;
-    int steps = 0;
-    while (curr >= 0 && ++steps < n)
-        curr = refit_step<T>(curr, n, left, right, parent, soa, recs, height, counters, leaves);
-}
-
 } // namespace ft

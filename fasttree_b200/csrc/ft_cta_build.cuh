@@ -5,7 +5,7 @@
 // 2165-2290): the set's bounding box (462-572), its SFC keys (357-423), the keys sorted with
 // their input indices (2202-2232; equal keys in input order), the leaf gather (2266-2279),
 // the Karras topology (861-903) and the bottom-up refit (925-969) -- here one agglomerative
-// climb that yields the same tree, numbering and boxes -- then this library's 4-wide
+// climb that yields the same tree, numbering and boxes -- then this library's walk
 // records.  Only the schedule differs: every step runs inside the block, with block barriers
 // between them, over the set's slice of the batch's arrays.  The key sort is a stable LSD
 // radix sort over 8-bit digits whose tiles the block takes in order, so a tile's place in

@@ -253,7 +253,7 @@ ft_status ft_range(ft_context *ctx, const ft_tree *tree, const void *qx, const v
 
 /* How ft_range walks trees of height <= 62 on this context: 0 (default), where the box
  * distance is monotone over nested boxes, each query writes its row with a walk over the
- * 4-wide records and stops once the row is full, then the full rows of a warp's 32 queries
+ * 32-bit 4-wide records and stops once the row is full, then the full rows of a warp's 32 queries
  * (neighbours in SFC order) are counted together when their points lie close against the
  * radius (nodes inside every query's shell counted whole, nodes beyond every ball skipped,
  * the leaves between tested per query), else per query; elsewhere one walk per query over the
@@ -471,13 +471,13 @@ ft_status ft_tune_reset(ft_context *ctx);
 /* ft_get_build_profile returns the last profiled build's stage times (synchronises).       */
 /* ---------------------------------------------------------------------------------- */
 typedef struct ft_build_profile {
-    float   bbox_ms;      /* compute_bbox                                                  */
-    float   encode_ms;    /* SFC keys + permutation                                        */
+    float   bbox_ms;      /* compute_bbox (up to 8192 points: box, keys and sort in one)   */
+    float   encode_ms;    /* SFC keys, packed points, digit histograms                     */
     float   sort_ms;      /* key + permutation sort                                        */
-    float   gather_ms;    /* leaf gather                                                   */
-    float   topology_ms;  /* Karras topology                                               */
-    float   refit_ms;     /* bottom-up refit (boxes, node records, heights)                */
-    float   records_ms;   /* 4-wide records of the fast walk                               */
+    float   gather_ms;    /* 0: part of refit_ms                                           */
+    float   topology_ms;  /* 0: part of refit_ms                                           */
+    float   refit_ms;     /* leaf gather, topology, boxes, records, heights (treelets)     */
+    float   records_ms;   /* walk records of the nodes formed outside the treelets         */
     float   total_ms;
     int32_t reserved[8];
 } ft_build_profile;
