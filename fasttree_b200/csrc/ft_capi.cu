@@ -254,8 +254,6 @@ ft_status ft_context_destroy(ft_context *ctx) {
     if (ctx) {
         if (ctx->status) cudaFree(ctx->status);
         if (ctx->replay_ranks) cudaFree(ctx->replay_ranks);
-        if (ctx->replay_rows) cudaFree(ctx->replay_rows);
-        if (ctx->seed_ranks) cudaFree(ctx->seed_ranks);
         if (ctx->miss_ranks) cudaFree(ctx->miss_ranks);
         if (ctx->miss_rows) cudaFree(ctx->miss_rows);
         for (int b = 0; b < 2; ++b) {

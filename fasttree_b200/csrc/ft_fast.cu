@@ -296,18 +296,19 @@ void batch_self_knn(Context &ctx, const ft_tree &all, const BatchDev &bt, size_t
     replay_exact(ctx, all, rr, rw, counters, k, excl, idx, dist, st, bt);
 }
 
+// The three lists lie in one allocation.
 void ensure_replay(Context &ctx, size_t num) {
     if (num <= ctx.replay_cap && ctx.replay_ranks) return;
     if (ctx.replay_ranks) cudaFree(ctx.replay_ranks);
-    if (ctx.replay_rows) cudaFree(ctx.replay_rows);
-    if (ctx.seed_ranks) cudaFree(ctx.seed_ranks);
     ctx.replay_ranks = ctx.replay_rows = ctx.seed_ranks = nullptr;
     ctx.replay_cap                                       = 0;
-    size_t cap = num + num / 4 + 1024;
-    FT_CUDA(cudaMalloc(&ctx.replay_ranks, cap * sizeof(int32_t)));
-    FT_CUDA(cudaMalloc(&ctx.replay_rows, cap * sizeof(int32_t)));
-    FT_CUDA(cudaMalloc(&ctx.seed_ranks, cap * sizeof(int32_t)));
-    ctx.replay_cap = cap;
+    const size_t cap = (num + num / 4 + 1024 + 63) / 64 * 64;
+    int32_t     *p   = nullptr;
+    FT_CUDA(cudaMalloc(&p, 3 * cap * sizeof(int32_t)));
+    ctx.replay_ranks = p;
+    ctx.replay_rows  = p + cap;
+    ctx.seed_ranks   = p + 2 * cap;
+    ctx.replay_cap   = cap;
 }
 
 // =========================================================================================

@@ -30,6 +30,7 @@ enum : uint32_t { STATUS_SPIN_LIMIT = 1u, STATUS_TRAVERSAL_LIMIT = 2u, STATUS_BA
 // the role of the reference's BvhScratch, src/hlbvh.hpp:720-745).
 struct TreeImpl {
     size_t    cap          = 0; // leaf capacity
+    void     *arena        = nullptr; // single trees: the allocation that holds the arrays below
     int       coord        = 0;
     void     *recs         = nullptr; // NodeRec<T>[cap-1]
     uint8_t  *height       = nullptr; // subtree height of internal nodes
@@ -129,7 +130,7 @@ struct Context {
     ft_query_stats stats{};
     uint32_t      *status = nullptr; // [0] status word of query kernels, [1] replay count,
                                      // [2..3] visits, [4] bound misses (8 words)
-    int32_t       *replay_ranks = nullptr; // queries the fast traversal hands to the exact one
+    int32_t       *replay_ranks = nullptr; // queries the fast traversal hands to the exact one (holds the next two)
     int32_t       *replay_rows  = nullptr;
     int32_t       *seed_ranks   = nullptr; // SFC rank of each external query (fast knn)
     size_t         replay_cap   = 0;
