@@ -138,10 +138,10 @@ def run_batched(args, dev, stream, timed_steps, warmup):
     seq_ms = timed(lambda: b.build_knn(off, x, y, z, k, idx, dst, method="fast"), timed_steps)  # launch sequence
     b.check()
     stats = b.query_stats()
-    # the same build + query as one persistent launch (the default method), in its own graph
+    # the same build + query as one persistent launch, in its own graph
     bp = ft.BatchedSets(ctx, N, S)
     pidx, pdst = torch.empty_like(idx), torch.empty_like(dst)
-    persist_ms = timed(lambda: bp.build_knn(off, x, y, z, k, pidx, pdst, method="default"), timed_steps)
+    persist_ms = timed(lambda: bp.build_knn(off, x, y, z, k, pidx, pdst, method="persistent"), timed_steps)
     bp.check()
     pstats = bp.query_stats()
     bp.set_build_method("persistent")  # its builds alone (the same kernel without the queries)
@@ -160,11 +160,11 @@ def run_batched(args, dev, stream, timed_steps, warmup):
     del fi, fd, pidx, pdst
     persistent = {"ms_per_step": persist_ms, "value": N / (persist_ms / 1e3), "unit": "queries/s",
                   "replayed": pstats["replayed"], "build_only_ms": persist_build_ms,
-                  "note": "ft_batch_build_knn, default method: prep + order + one persistent kernel (per-set "
+                  "note": "ft_batch_build_knn, method persistent: prep + order + one persistent kernel (per-set "
                           "builds, then 32-query chunks of finished sets) + replay, one CUDA graph; build_only_ms: "
                           "the same kernel without the queries (ft_batch_build, per-set method)"}
     sequence = {"ms_per_step": seq_ms, "value": N / (seq_ms / 1e3), "unit": "queries/s", "replayed": stats["replayed"],
-                "note": "ft_batch_build_knn, method fast: the launch sequence (build kernels over all points, then "
+                "note": "ft_batch_build_knn, method fast (the default): the launch sequence (build kernels over all points, then "
                         "the fast walk) in one CUDA graph"}
     learned = run_batched_learned(args, ctx, b, off, x, y, z, k, idx, dst, (pi, pd), timed, timed_steps, plain_ms)
     del pi, pd
@@ -173,7 +173,7 @@ def run_batched(args, dev, stream, timed_steps, warmup):
     if getattr(args, "no_per_set_loop", False):
         del b
         return {"workload": w["name"], "n_sets": S, "n_points": N, "k": k,
-                "graph_build_plus_query_ms": persist_ms, "value": N / (persist_ms / 1e3), "unit": "queries/s",
+                "graph_build_plus_query_ms": seq_ms, "value": N / (seq_ms / 1e3), "unit": "queries/s",
                 "persistent": persistent, "launch_sequence": sequence, "build_ms": build_ms, "query_fast_ms": fast_ms, "query_plain_ms": plain_ms,
                 "replayed": stats["replayed"], "bit_exact": bit_exact, "learned": learned, "tuning": tuning}
     tree = ft.TreeSoA(ctx, int(np.diff(offs).max()))
@@ -191,13 +191,13 @@ def run_batched(args, dev, stream, timed_steps, warmup):
     loop_ms = (time.perf_counter() - t0) * 1e3
     del b, tree
     return {"workload": w["name"], "n_sets": S, "n_points": N, "k": k,
-            "graph_build_plus_query_ms": persist_ms, "value": N / (persist_ms / 1e3), "unit": "queries/s",
+            "graph_build_plus_query_ms": seq_ms, "value": N / (seq_ms / 1e3), "unit": "queries/s",
             "persistent": persistent, "launch_sequence": sequence, "build_ms": build_ms, "query_fast_ms": fast_ms,
             "query_plain_ms": plain_ms,
             "query_fast_qps": N / (fast_ms / 1e3), "query_plain_qps": N / (plain_ms / 1e3),
             "per_set_loop_ms": loop_ms, "per_set_loop_qps": N / (loop_ms / 1e3),
             "replayed": stats["replayed"], "bit_exact": bit_exact, "learned": learned, "tuning": tuning,
-            "note": "graph_build_plus_query_ms = ft_batch_build_knn's default (the persistent launch); build_ms / "
+            "note": "graph_build_plus_query_ms = ft_batch_build_knn's default (the launch sequence); build_ms / "
                     "query_*_ms: ft_batch_build (launch sequence) and ft_batch_self_knn alone; per-set loop = "
                     "build_bvh + self_knn_query(method='fast') per set through the single-tree API (wall clock)"}
 
@@ -409,7 +409,7 @@ def run_cfg2_extra(args, ctx, tree, x, y, z, n, stream):
     out["range_query"] = {"ms_per_step": ms, "value": n / (ms / 1e3), "unit": "queries/s",
                           "mean_count": float(c.mean()), "max_count": int(cnt.max()),
                           "truncated_queries": int((cnt > max_per).sum()), "max_results_per_query": max_per,
-                          "walk": "default: rows by a 4-wide walk per query that stops once the row is full, "
+                          "walk": "default: rows by a walk over the 32-bit records per query that stops once the row is full, "
                                   "then the full rows' counts by a warp's 32 SFC-neighbour queries together "
                                   "when their points lie close against the radius, else per query",
                           "queries": "the N particle positions in input order (the library walks them in SFC "
@@ -650,10 +650,11 @@ def run_profile(args, stream):
 
 def build_stage_roofline(ctx, p, tree, n, sc, stream):
     """One more build with stage events (ft_set_build_profiling): each stage's time, its
-    as-designed bytes (every byte once: bbox 3 s_c N; keys N(3 s_c + s_k + 4); sort 8 passes
-    of 2N(s_k + 4) plus the N s_k histogram read; gather N(4 + 9 s_c + 9); topology
-    2N s_k + 12(N-1); refit (N-1)(18 s_c + 8); 4-wide records (N-1)(48 s_c + 16)) and the GB/s
-    and fraction of the measured HBM bandwidth they imply; and the whole build against the
+    as-designed bytes (every byte once: bbox 3 s_c N; keys N(3 s_c + 12 + 4 s_c), packed points
+    included; sort 8 passes of 24 N over the sort word and the index; refit, which is the
+    treelets' gather, topology, boxes and records in one, N(10 s_c + s_k + 38) for the leaves and
+    (N-1)(22 s_c + 21) for the nodes; records, the walk records made outside the treelets, not
+    counted) and the GB/s and fraction of the measured HBM bandwidth they imply; and the whole build against the
     compulsory bytes 3 s_c N + (2N-1)(6 s_c + 4) + 8(N-1) + 9N."""
     import torch
 
@@ -665,13 +666,12 @@ def build_stage_roofline(ctx, p, tree, n, sc, stream):
     ctx.profile_builds(False)
     torch.cuda.synchronize()
     peak, kind = measured_peaks()
-    designed = {"bbox_ms": 3 * sc * n, "encode_ms": n * (3 * sc + sk + 4), "sort_ms": 8 * 2 * n * (sk + 4) + n * sk,
-                "gather_ms": n * (4 + 9 * sc + 9), "topology_ms": 2 * n * sk + 12 * (n - 1),
-                "refit_ms": (n - 1) * (18 * sc + 8), "records_ms": (n - 1) * (48 * sc + 16)}
+    designed = {"bbox_ms": 3 * sc * n, "encode_ms": n * (7 * sc + 12), "sort_ms": 8 * 24 * n, "gather_ms": 0,
+                "topology_ms": 0, "refit_ms": n * (10 * sc + sk + 38) + (n - 1) * (22 * sc + 21), "records_ms": 0}
     stages = {}
     for key, b in designed.items():
         ms = prof[key]
-        gbs = b / (ms / 1e3) / 1e9 if ms > 0 else None
+        gbs = b / (ms / 1e3) / 1e9 if ms > 0 and b else None
         stages[key[:-3]] = {"ms": ms, "bytes": b, "gbs": gbs, "frac": gbs / peak if gbs else None}
     compulsory = 3 * sc * n + (2 * n - 1) * (6 * sc + 4) + 8 * (n - 1) + 9 * n
     tot = prof["total_ms"]
