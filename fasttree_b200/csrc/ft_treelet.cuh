@@ -188,6 +188,17 @@ FT_D void treelet_noderec(NodeRec<T> *out, const T lb[6], const T rb[6], int lc,
     }
 }
 
+// The root is formed.  The records are in the frame of a.box and a query takes the root box's: the
+// two differ when the box was folded over points that are not the leaves (a refit whose original
+// indices leave rows of its input out), and the frame does not serve the tree then.
+template <class T> FT_D void treelet_root(const TreeletArgs<T> &a, const T box[6]) {
+    a.parent[0] = -1;
+    bool same   = true;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) same = same && box[d] == a.box[d];
+    if (!same) atomicOr(a.qflag, QFLAG_FRAME);
+}
+
 // delta of the adjacent sorted keys x and x + 1 (0 <= x < n - 1), plus one (0 is the border's).
 // (not below one: keys wider than the reference's would differ above its prefix)
 // lo: the sorted low words, or null (LEAVES_PACKED of 126-bit keys): they are in the packed points.
@@ -393,7 +404,10 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
         a.parent[rc] = v;
         a.leaves[v] = r - l + 1;
         a.height[v] = (uint8_t)h;
-        if (v == 0) a.parent[0] = -1; // (number 0 is the root's)
+        if (v == 0) { // (number 0 is the root's)
+            const T rb0[6] = {s.bx[0][0], s.bx[1][0], s.bx[2][0], s.bx[3][0], s.bx[4][0], s.bx[5][0]};
+            treelet_root<T>(a, rb0);
+        }
         treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, cl.count(), cr.count(), l == sp ? 0 : s.nh[sp - b0],
                            sp + 1 == r ? 0 : s.nh[sp + 1 - b0]);
         if (v == 0 || r - l + 1 > kBucket)
@@ -600,7 +614,10 @@ __global__ void __launch_bounds__(kJoinThreads) treelet_join_kernel(const Treele
         a.parent[rc] = v;
         a.leaves[v]  = r - l + 1;
         a.height[v]  = (uint8_t)h;
-        if (root) a.parent[0] = -1;
+        if (root) {
+            const T rb0[6] = {s.bx[0][j], s.bx[1][j], s.bx[2][j], s.bx[3][j], s.bx[4][j], s.bx[5][j]};
+            treelet_root<T>(a, rb0);
+        }
         treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, sl - l + 1, r - sl, x == sp ? s.ih[x] : s.nh[sp],
                            sp + 1 == y ? s.ih[y] : s.nh[sp + 1]);
         if (root || r - l + 1 > kBucket) a.list[atomicAdd(a.qflag + 1, 1u)] = v;
@@ -715,7 +732,7 @@ __global__ void __launch_bounds__(128) treelet_climb_kernel(const TreeletArgs<T>
                 a.parent[lc] = v;
                 a.parent[rc] = v;
                 a.leaves[v]  = R - L + 1;
-                if (root) a.parent[0] = -1;
+                if (root) treelet_root<T>(a, box);
                 treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, split - L + 1, R - split, hl, hr);
                 if (root || R - L + 1 > kBucket) a.list[atomicAdd(a.qflag + 1, 1u)] = v;
                 l  = L;

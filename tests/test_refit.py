@@ -139,3 +139,58 @@ def test_refit_errors_and_small_trees():
         nx = x[:n][::-1].copy()
         ft.refit_bvh(ctx, ft.particles(nx, y[:n], z[:n]), t2)
         assert_tree_equal(t2.to_numpy(), _oracle_refit(opts, ot, n, nx, y[:n], z[:n]), n)
+
+
+def _against_exact_walks(ctx, tree, k, radius, qn=300):
+    """Default kNN rows against the reference traversal's, range rows against the binary walk's."""
+    a = ft.self_knn_query(ctx, tree, k, method="plain")
+    a = (a[0].clone(), a[1].clone())
+    b = ft.self_knn_query(ctx, tree, k)
+    torch.cuda.synchronize()
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    q = [c[:qn].contiguous() for c in tree.leaf_coords()]
+    lo, hi = (torch.from_numpy(np.full(qn, r, O.NP_COORD[ctx.coord])).cuda() for r in (0, radius))
+    want = None
+    for walk in (1, 0, 3):
+        ctx.set_range_walk(walk)
+        res = torch.full((qn * 12,), -1, dtype=torch.int32, device="cuda")
+        cnt = torch.zeros(qn, dtype=torch.int32, device="cuda")
+        ft.range_query(ctx, tree, *q, lo, hi, 12, res, cnt)
+        torch.cuda.synchronize()
+        want = want or (res, cnt)
+        assert torch.equal(cnt, want[1]) and torch.equal(res, want[0]), walk
+    ctx.set_range_walk(0)
+
+
+def _tree_with_orig(ctx, opts, x, y, z, change):
+    """build_tree from the build's sorted keys and points, with changed original indices."""
+    n = len(x)
+    ot = O.build_bvh(opts, x, y, z)
+    orig = ot.orig_idx[n - 1:2 * n - 1].astype(np.int64)
+    if opts.coord == O.U64:
+        keys = np.zeros((n, 3), np.uint64)
+        keys[:, 1], keys[:, 2] = ot.sorted_hi[:n], ot.sorted_lo[:n]
+    else:
+        keys = ot.sorted_lo[:n]
+    tree = ft.TreeSoA(ctx, n)
+    ft.build_tree(ctx, tree, keys, x[orig], y[orig], z[orig], sorted_orig_idx=change(orig).astype(np.int32))
+    return tree
+
+
+@pytest.mark.parametrize("n", [400, 3000, 20_000])  # the root formed in a block, in a join, in a later one
+@pytest.mark.parametrize("coord,sfc,per", [(O.F64, O.MORTON, False), (O.U64, O.PEANO_HILBERT, False),
+                                           (O.F32, O.MORTON, False)], ids=["f64", "u64", "f32"])
+def test_refit_of_repeated_points(coord, sfc, per, n):
+    """Original indices that leave out half of the input rows: those rows' positions are no part of
+    the tree, so neither of the box its walks work in."""
+    ctx = ft.Context(NAMES[coord], sfc, periodic=per)
+    x, y, z = gen("uniform", n, coord, 5)
+    tree = _tree_with_orig(ctx, O.Options(coord, sfc, per), x, y, z, lambda o: o // 2)
+    moved = [a.copy() for a in gen("uniform", n, coord, 6)]
+    unit = 100.0
+    if coord == O.U64:
+        moved, unit = [a >> np.uint64(12) for a in moved], float(1 << 30)
+    for a in moved:  # rows no leaf takes lie far away
+        a[(n + 1) // 2:] = a[(n + 1) // 2:] * a.dtype.type(500)
+    ft.refit_bvh(ctx, ft.particles(*moved), tree)
+    _against_exact_walks(ctx, tree, 9, 0.1 * unit)
