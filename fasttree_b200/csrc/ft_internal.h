@@ -63,7 +63,7 @@ struct TreeImpl {
                                     // for 32-bit): the periodic distance is then monotone over
                                     // nested boxes, which the fast walks rely on
     bool      framed       = false; // the 32-bit frame serves the tree (qflag was 0 after the build)
-    bool      plain_only   = false; // box distances are not monotone (kQFlagPlain)
+    bool      plain_only   = false; // only the reference traversal gives its rows (kQFlagPlain)
     bool      view         = false; // one set of a batch: arrays owned by the batch, no builds
     bool      own_keys     = false; // key_lo / key_hi hold keys this library encoded (build_bvh
                                     // without caller keys), with the box in bbox
@@ -87,7 +87,7 @@ struct BatchDev {
 // integer one on coordinates at or above the period (2^42 / 2^21), whose unmasked box bounds
 // break it; such trees keep the reference traversal.
 inline bool fast_walk_applies(const ft_options &o, const TreeImpl &t) {
-    if (t.plain_only) return false; // a coordinate that is not finite, or squares beyond 64 bits
+    if (t.plain_only) return false; // a coordinate not finite, squares beyond 64 bits, leaves that are boxes
     return !o.periodic || o.coord_type == FT_COORD_F32 || o.coord_type == FT_COORD_F64 || t.in_period;
 }
 

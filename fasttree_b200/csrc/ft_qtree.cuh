@@ -52,9 +52,10 @@ FT_HD int qref_count(uint32_t r) { return (int)((r >> 28) & 7u) + 1; }
 // Bits of the per-tree flag (0: the frame serves the walks).  DENSE, FRAME (no frame for the root
 // box): the exact binary walk serves the tree.  NONFINITE (a coordinate is not finite), OVERFLOW
 // (integer gaps whose squares may leave 64 bits): box distances are not monotone, so only the
-// reference traversal gives its rows.
-enum : uint32_t { QFLAG_NONFINITE = 1u, QFLAG_DENSE = 2u, QFLAG_FRAME = 4u, QFLAG_OVERFLOW = 8u };
-static constexpr uint32_t kQFlagPlain = QFLAG_NONFINITE | QFLAG_OVERFLOW;
+// reference traversal gives its rows.  BOXES (a leaf slot of the caller's whose minimum is not its
+// maximum): the walks take leaves for points, the reference traversal measures to their boxes.
+enum : uint32_t { QFLAG_NONFINITE = 1u, QFLAG_DENSE = 2u, QFLAG_FRAME = 4u, QFLAG_OVERFLOW = 8u, QFLAG_BOXES = 16u };
+static constexpr uint32_t kQFlagPlain = QFLAG_NONFINITE | QFLAG_OVERFLOW | QFLAG_BOXES;
 // A node of more than kDenseLeaves leaves whose box spans at most 2 kDenseUnits units on every
 // axis: the frame no longer tells its leaves apart (QFLAG_DENSE; the exact walk serves the tree).
 static constexpr int      kDenseLeaves = 256;

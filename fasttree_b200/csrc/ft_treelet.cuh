@@ -57,7 +57,7 @@ template <class T> struct alignas(sizeof(T) * 4) PackedPoint {
 // Where the leaves come from.
 enum TreeletSource {
     LEAVES_PACKED = 0, // pack[perm[i]]: the build; also writes id, ghost, orig
-    LEAVES_IN_PLACE = 1, // the leaf slots hold them
+    LEAVES_IN_PLACE = 1, // the leaf slots hold them: points, or boxes of the caller's (QFLAG_BOXES)
     LEAVES_MOVED = 2   // new positions x / y / z of the points in the leaves (refit)
 };
 
@@ -292,6 +292,8 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
             p[0] = a.soa[0][leaf];
             p[1] = a.soa[2][leaf];
             p[2] = a.soa[4][leaf];
+            if (!(a.soa[1][leaf] == p[0] && a.soa[3][leaf] == p[1] && a.soa[5][leaf] == p[2]))
+                atomicOr(a.qflag, QFLAG_BOXES);
         }
         if constexpr (SRC != LEAVES_IN_PLACE) {
 #pragma unroll
@@ -312,12 +314,21 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
     }
     __syncthreads();
 
+    // a leaf's box: its point, or what the caller left in its slot
+    auto leaf_box = [&](int j, T b[6]) {
+        if constexpr (SRC == LEAVES_IN_PLACE) {
+#pragma unroll
+            for (int d = 0; d < 6; ++d) b[d] = a.soa[d][b0 + j + n - 1];
+        } else {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) b[2 * d] = b[2 * d + 1] = s.lx[d][j];
+        }
+    };
     // ---- climbs inside the block ----
     for (int j = tid; j < m; j += kTreeletThreads) {
         int l = j, r = j, sp = 0, h = 0;
         T   box[6];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) box[2 * d] = box[2 * d + 1] = s.lx[d][j];
+        leaf_box(j, box);
         for (;;) {
             const int  dl = s.delta[l], dr = s.delta[r + 1];
             const bool root     = b0 + l == 0 && b0 + r == n - 1;
@@ -348,8 +359,7 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
             T         sb[6];
             int       sh = 0;
             if (sl == sr) {
-#pragma unroll
-                for (int d = 0; d < 3; ++d) sb[2 * d] = sb[2 * d + 1] = s.lx[d][sl];
+                leaf_box(sl, sb);
             } else {
                 const volatile T *q = &s.bx[0][si];
 #pragma unroll
@@ -380,8 +390,7 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
     // ---- the nodes formed here ----
     auto child_box = [&](const TreeletChild &c, T b[6]) {
         if (c.l == c.r) {
-#pragma unroll
-            for (int d = 0; d < 3; ++d) b[2 * d] = b[2 * d + 1] = s.lx[d][c.l - b0];
+            leaf_box(c.l - b0, b);
         } else {
 #pragma unroll
             for (int d = 0; d < 6; ++d) b[d] = s.bx[d][c.node() - b0];

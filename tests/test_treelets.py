@@ -105,3 +105,59 @@ def test_refit_equals_build_tree_of_the_moved_points(cfg, n):
         assert np.array_equal(a[k], getattr(ot, k)[:n - 1])
     ft.refit_bvh(ctx, ft.particles(*gen("uniform", n, cfg[0], seed=n)), tree)
     assert_tree_equal(tree.to_numpy(), ot, n)
+
+
+@pytest.mark.parametrize("n", [2, 9, 300, 1500, 9001])
+@pytest.mark.parametrize("coord", ["f64", "u64"])
+def test_build_tree_of_boxes_in_the_leaf_slots(coord, n):
+    """build_tree without coordinate arrays takes what the leaf slots hold, boxes too: internal boxes
+    cover them and queries measure the distance to them (src/hlbvh.hpp:941-969, 998-1055)."""
+    rng = np.random.default_rng(n)
+    ctx = ft.Context(coord, "morton" if coord == "f64" else "ph")
+    dt = np.float64 if coord == "f64" else np.uint64
+    scale = 1.0 if coord == "f64" else 2.0**40
+    order = np.argsort(rng.random(n))
+    base = np.sort(rng.random(n))  # along x, so that keys and places agree
+    lo = [(base if a == 0 else rng.random(n)) * scale for a in range(3)]
+    hi = [v + rng.random(n) * 0.01 * scale for v in lo]
+    lo, hi = [v.astype(dt) for v in lo], [v.astype(dt) for v in hi]
+    kv = (base * 2.0**60).astype(np.uint64)
+    keys = kv if coord == "f64" else np.stack([np.zeros(n, np.uint64), kv, order.astype(np.uint64)], axis=1)
+    tree = ft.TreeSoA(ctx, n)
+    for a, v, w in zip("xyz", lo, hi):
+        getattr(tree, "min_" + a)[n - 1:] = torch.from_numpy(v).cuda()
+        getattr(tree, "max_" + a)[n - 1:] = torch.from_numpy(w).cuda()
+    ft.build_tree(ctx, tree, keys)
+    t = tree.to_numpy()
+    for a, v, w in zip("xyz", lo, hi):
+        assert np.array_equal(t["min_" + a][n - 1:], v) and np.array_equal(t["max_" + a][n - 1:], w)
+        for v2, f, nm in ((v, np.minimum, "min_"), (w, np.maximum, "max_")):
+            b = t[nm + a]
+            assert np.array_equal(b[:n - 1], f(b[t["left_child"]], b[t["right_child"]])) and b[0] == f.reduce(v2)
+    t2 = ft.import_tree(ctx, tree.export())
+    for k, v in t2.to_numpy().items():
+        assert k in ("id", "is_ghost", "orig_idx") or np.array_equal(v, t[k]), k
+    # every query kind against distances to the boxes
+    q = [(rng.random(200) * scale).astype(dt) for _ in range(3)]
+    k = min(n, 6)
+
+    def gap(p, v, w):
+        if coord == "f64":
+            return np.maximum(np.maximum(v - p, p - w), 0.0)
+        return np.where(p < v, (v - p) >> np.uint64(11), np.where(p > w, (p - w) >> np.uint64(11), np.uint64(0)))
+
+    g = [gap(p[:, None], v[None], w[None]) for p, v, w in zip(q, lo, hi)]
+    d = g[0] * g[0] + g[1] * g[1] + g[2] * g[2]
+    want = np.sort(d, axis=1)[:, :k]
+    for method in ("plain", "fast"):
+        _, gd = ft.knn_query(ctx, tree, *q, k, method=method)
+        torch.cuda.synchronize()
+        assert np.array_equal(gd.cpu().numpy(), want), method
+    r = 0.2 * scale
+    r2 = np.float64(r) * np.float64(r) if coord == "f64" else np.uint64(int(r) >> 11) ** 2
+    cnt = torch.zeros(200, dtype=torch.int32, device="cuda")
+    res = torch.zeros(200 * 4, dtype=torch.int32, device="cuda")
+    one = np.ones(200)
+    ft.range_query(ctx, tree, *q, (0 * one).astype(dt), (r * one).astype(dt), 4, res, cnt)
+    torch.cuda.synchronize()
+    assert np.array_equal(cnt.cpu().numpy(), (d <= r2).sum(axis=1))
