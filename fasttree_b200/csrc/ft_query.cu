@@ -686,9 +686,9 @@ template <class T, class D> FT_D RangeLimits range_limits(const QFrame<T> &f, D 
         else return __ull2float_rd(d);
     };
     RangeLimits l;
-    l.out = f.limit(up(RM2));
+    l.out = RM2 >= D(0) ? f.limit(up(RM2)) : -1.0f; // (a radius that is not a number reaches nothing)
     l.in  = down(RM2) * f.k2 * (1.0f - 0x1p-15f) - f.slack;
-    l.ge  = rm2 > D(0) ? f.limit(up(rm2)) : 0.0f;
+    l.ge  = rm2 <= D(0) ? 0.0f : f.limit(up(rm2)); // (not a number: no box lies beyond it)
     l.lt  = down(rm2) * f.k2 * (1.0f - 0x1p-15f) - f.slack;
     return l;
 }
@@ -742,7 +742,7 @@ FT_D int range_rows(const TreeDev<T> &t, bool go, const RangePoint<T, PER> &pt, 
     uint32_t       st[kRows];
     uint32_t       cur = 0;
     int            sp = 0, count = 0;
-    bool           have = go;
+    bool           have = go && lim.out >= 0.0f;
     if constexpr (STOP) {
         *filled = false;
         if (max_per <= 0 && have) { // no row: only the count is wanted

@@ -187,3 +187,31 @@ def test_query_counts_spread_over_warps(n):
     a = ft.self_knn_query_subset(ctx, tree, ids, 12, method="plain")
     a = (a[0].clone(), a[1].clone())
     assert same(a, ft.self_knn_query_subset(ctx, tree, ids, 12))
+
+
+@pytest.mark.parametrize("coord", ["f32", "f64"])
+def test_radii_that_are_not_numbers(coord):
+    """A shell with a NaN on either side holds nothing; the other queries of the warp are not
+    touched."""
+    rng = np.random.default_rng(12)
+    n = 6000
+    xyz = [rng.random(n).astype(NP[coord]) for _ in range(3)]
+    ctx, tree = build(coord, "ph", False, xyz)
+    q = [dev(a[:640]) for a in xyz]
+    lo = np.where(rng.random(640) < 0.3, 0.05, 0.0)
+    hi = np.full(640, 0.3)
+    lo[rng.random(640) < 0.2] = np.nan
+    hi[rng.random(640) < 0.2] = np.nan
+    bad = np.isnan(lo) | np.isnan(hi)
+    lo, hi = dev(lo.astype(NP[coord])), dev(hi.astype(NP[coord]))
+    for rows in (0, 1, 8):
+        want = None
+        for walk in (1, 0, 3, 4):
+            ctx.set_range_walk(walk)
+            res = torch.full((640 * max(rows, 1),), -1, dtype=torch.int32, device="cuda")
+            cnt = torch.zeros(640, dtype=torch.int32, device="cuda")
+            ft.range_query(ctx, tree, *q, lo, hi, rows, res, cnt)
+            torch.cuda.synchronize()
+            want = want or (res, cnt)
+            assert (cnt.cpu().numpy()[bad] == 0).all(), (walk, rows)
+            assert torch.equal(cnt, want[1]) and torch.equal(res, want[0]), (walk, rows)
