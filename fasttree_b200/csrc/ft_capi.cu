@@ -439,23 +439,24 @@ ft_status ft_sfc_encode(ft_context *ctx, const void *x, const void *y, const voi
     FT_API_END
 }
 
-// What the host keeps of a finished build: one small launch, one copy, one wait.  Throws what
-// the kernels recorded; sets the height, the frame and whether every coordinate of an integer
-// tree lies below the period 2^42 (64-bit) / 2^21 (32-bit), i.e. the root box maxima do.
+// What the host keeps of a finished build: one small launch, one copy, one wait.  Sets the frame
+// and whether every coordinate of an integer tree lies below the period 2^42 (64-bit) / 2^21
+// (32-bit), i.e. the root box maxima do; then throws what the kernels recorded (a refit that fails
+// has moved the other leaves: the walks must not go by the frame of before); then the height.
 // sorted: the build sorted its keys itself (build_bvh).  Returns false when it has to be repeated
 // with the full sort.
 static bool finish_build(const ft_context *ctx, ft_tree *tree, cudaStream_t st, bool sorted = false) {
     TreeImpl    &impl = *(TreeImpl *)tree->impl;
     TreeSummary  m;
     tree_summary(ctx->opts, *tree, sorted, m, st);
-    if (m.status) check_device_status(impl.status, st);
     const int      ct = ctx->opts.coord_type;
     const uint64_t P  = ct == FT_COORD_U64 ? 1ull << 42 : 1ull << 21;
-    impl.height_root  = (int)m.height;
     impl.framed       = m.qflag == 0u;
     impl.plain_only   = (m.qflag & kQFlagPlain) != 0u;
     impl.in_period    = ct == FT_COORD_F32 || ct == FT_COORD_F64 || (m.mx[0] < P && m.mx[1] < P && m.mx[2] < P);
     impl.clean42      = impl.clean42_ok && ct == FT_COORD_U64 && impl.in_period;
+    if (m.status) check_device_status(impl.status, st);
+    impl.height_root = (int)m.height;
     return m.long_runs == 0u;
 }
 

@@ -194,3 +194,22 @@ def test_refit_of_repeated_points(coord, sfc, per, n):
         a[(n + 1) // 2:] = a[(n + 1) // 2:] * a.dtype.type(500)
     ft.refit_bvh(ctx, ft.particles(*moved), tree)
     _against_exact_walks(ctx, tree, 9, 0.1 * unit)
+
+
+def test_refit_that_fails_leaves_a_tree_its_walks_agree_on():
+    """A refit that reports an original index out of range has moved the other leaves: range
+    queries must not go on in the box of before."""
+    ctx = ft.Context("f64", "morton")
+    n = 3000
+    x, y, z = gen("uniform", n, O.F64, 7)
+
+    def change(o):
+        o = o.copy()
+        o[n // 3] = n + 5
+        return o
+
+    tree = _tree_with_orig(ctx, O.Options(O.F64, O.MORTON, False), x, y, z, change)
+    _against_exact_walks(ctx, tree, 9, 10.0)
+    with pytest.raises(Exception):
+        ft.refit_bvh(ctx, ft.particles(*(a + 5000.0 for a in (x, y, z))), tree)
+    _against_exact_walks(ctx, tree, 9, 10.0)
