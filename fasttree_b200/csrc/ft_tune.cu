@@ -6,8 +6,8 @@
 // bit, so the choice is free to follow speed: the tuner times each candidate on the caller's
 // own data and keeps the fastest for the shape, keyed by (kind, k, floor(log2 n)) in the
 // context.  Later calls with default options take the kept choice.
-//  * build: keys per thread of a onesweep tile (8 / 12 / 16 / 20 for one-word keys, 8 / 12 /
-//    16 for two-word keys), timed over whole builds of the caller's points;
+//  * build: keys per thread of a onesweep tile (8 / 12 / 16 / 20), timed over whole builds of the
+//    caller's points (by both words where 126-bit keys share their high word in long runs);
 //  * self-kNN (single tree and batched sets): the walk variant (4-wide walk, exact binary
 //    walk), the SFC seeding half-window (k/2, k, 2k) and the block shape
 //    (two-warp blocks with 32-entry heaps, or one-warp blocks), timed on up to 2^18 queries
@@ -220,9 +220,14 @@ void tune_build(Context &ctx, ft_tree &tree, const void *x, const void *y, const
     FT_CUDA(cudaMemsetAsync(cur.p, 0, words8 * 8, st));
     float      best_ms = 0.0f, default_ms = 0.0f;
     int        best = 0;
+    // points that need the full sort (ft_build_bvh repeats the build then): nothing is built without it
+    TreeSummary m;
+    build_bvh(ctx, tree, x, y, z, n, nullptr, nullptr, nullptr, nullptr, st);
+    tree_summary(ctx.opts, tree, true, m, st);
+    const bool full = m.long_runs != 0u;
     for (int c = 0; c < count; ++c) {
         const float ms = time_median(st, 3, [&] {
-            build_bvh(ctx, tree, x, y, z, n, nullptr, nullptr, nullptr, nullptr, st, items[c]);
+            build_bvh(ctx, tree, x, y, z, n, nullptr, nullptr, nullptr, nullptr, st, items[c], full);
         });
         // the leaf order (original index of every leaf slot) must not depend on the tile
         const int32_t *perm = tree.orig_idx + (n - 1);

@@ -108,3 +108,21 @@ def test_build_stage_profile():
     assert all(v >= 0.0 for v in stages) and prof["total_ms"] > 0.0
     assert abs(sum(stages) - prof["total_ms"]) < 0.05 * prof["total_ms"] + 0.01
     ctx.profile_builds(False)
+
+
+def test_tuned_build_of_long_runs_times_whole_builds():
+    """Points whose 126-bit keys share high words in long runs are sorted by both words; the tuner's
+    candidates have to do that too (a candidate that builds nothing takes a third of the time)."""
+    n = 2_000_000
+    rng = np.random.default_rng(31)
+    base = rng.integers(0, 1 << 41, (3, n // 100), dtype=np.uint64)
+    p = np.ascontiguousarray(base[:, np.arange(n) // 100])
+    ctx = ft.Context("u64", "ph", periodic=True)
+    xyz = [torch.from_numpy(a).cuda() for a in p]
+    tree = ft.TreeSoA(ctx, n)
+    ctx.profile_builds(True)
+    ft.build_bvh(ctx, ft.particles(*xyz), tree)
+    ft.build_bvh(ctx, ft.particles(*xyz), tree)
+    whole = ctx.build_profile()["total_ms"]  # the repeated build, by both words
+    ctx.profile_builds(False)
+    assert ft.tune_build(ctx, ft.particles(*xyz), tree)["default_ms"] > 0.7 * whole
