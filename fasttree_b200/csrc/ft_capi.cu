@@ -568,7 +568,7 @@ ft_status ft_tree_import(ft_context *ctx, const void *buf, size_t bytes, ft_tree
     const size_t n = (size_t)h.n;
     need(tree->capacity >= n, "tree import: tree capacity is smaller than the stored leaf count");
     TreeImpl &impl = *(TreeImpl *)tree->impl;
-    if (n) ensure_scratch(impl, ctx->opts, n);
+    if (n) ensure_scratch(*ctx, impl, n, tree->capacity, st);
     tree->num_leaves   = n;
     tree->num_internal = n ? n - 1 : 0;
     auto secs          = tree_sections(*ctx, *tree, n);

@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <map>
+#include <memory>
 #include <string>
 #include <type_traits>
 
@@ -26,11 +27,24 @@ void              check_cuda(cudaError_t e, const char *what);
 // Device status word bits (written by kernels instead of trapping).
 enum : uint32_t { STATUS_SPIN_LIMIT = 1u, STATUS_TRAVERSAL_LIMIT = 2u, STATUS_BAD_INPUT = 4u };
 
+// Device memory for the scratch of small trees: a context's, held by its trees too, so that it goes
+// when the last of them has (ensure_scratch).
+struct ScratchPool {
+    cudaMemPool_t pool = nullptr;
+    int           device = 0;
+    ScratchPool() = default;
+    ScratchPool(const ScratchPool &) = delete;
+    ~ScratchPool() {
+        if (pool) cudaMemPoolDestroy(pool);
+    }
+};
+
 // Library-owned per-tree acceleration data and build scratch (the persistent part plays
 // the role of the reference's BvhScratch, src/hlbvh.hpp:720-745).
 struct TreeImpl {
     size_t    cap          = 0; // leaf capacity
     void     *arena        = nullptr; // single trees: the allocation that holds the arrays below
+    std::shared_ptr<ScratchPool> pool; // where it comes from (null: cudaMalloc)
     int       coord        = 0;
     void     *recs         = nullptr; // NodeRec<T>[cap-1]
     uint8_t  *height       = nullptr; // subtree height of internal nodes
@@ -128,6 +142,7 @@ struct Context {
     int            device = 0;
     int            num_sms = 148;
     ft_query_stats stats{};
+    std::shared_ptr<ScratchPool> pool; // scratch of small trees
     uint32_t      *status = nullptr; // [0] status word of query kernels, [1] replay count,
                                      // [2..3] visits, [4] bound misses (8 words)
     int32_t       *replay_ranks = nullptr; // queries the fast traversal hands to the exact one (holds the next two)
@@ -287,7 +302,9 @@ size_t ref_key_bytes(const ft_options &o);
 // d < 8: low word, 8 <= d < 16: high word); no host synchronisation.
 void   sort_pairs_fixed(TreeImpl &s, size_t n, int words, int ndigits, const int *digits, cudaStream_t st);
 size_t sort_lookback_words(size_t n, int words);
-void   ensure_scratch(TreeImpl &impl, const ft_options &o, size_t n);
+// Build scratch for n leaves with room to grow, but never for more than `most` (the leaves the
+// tree's node arrays hold).
+void   ensure_scratch(Context &ctx, TreeImpl &impl, size_t n, size_t most, cudaStream_t st);
 void   free_scratch(TreeImpl &impl);
 
 // ---- queries (ft_query.cu) ----

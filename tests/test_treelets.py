@@ -161,3 +161,71 @@ def test_build_tree_of_boxes_in_the_leaf_slots(coord, n):
     ft.range_query(ctx, tree, *q, (0 * one).astype(dt), (r * one).astype(dt), 4, res, cnt)
     torch.cuda.synchronize()
     assert np.array_equal(cnt.cpu().numpy(), (d <= r2).sum(axis=1))
+
+
+def test_scratch_of_small_trees_from_a_shared_pool():
+    """Small trees take their scratch from a pool of their context: it is handed on only when the
+    queries of the tree before have ended, it outlives the context with its trees, and several
+    threads may build at once."""
+    import threading
+
+    n = 3000
+    sets = [[torch.from_numpy(a).cuda() for a in gen("uniform", n, O.F32, seed=s)] for s in range(8)]
+    want = []
+    for s in sets:
+        c = ft.Context("f32", "morton")
+        t = ft.TreeSoA(c, n)
+        ft.build_bvh(c, ft.particles(*s), t)
+        want.append([a.clone() for a in ft.self_knn_query(c, t, 16)])
+    torch.cuda.synchronize()
+    # a tree goes while its query runs on another stream; the next is built at once
+    ctx, streams, got = ft.Context("f32", "morton"), [torch.cuda.Stream() for _ in range(2)], []
+    for i, s in enumerate(sets * 3):
+        st = streams[i % 2]
+        t = ft.TreeSoA(ctx, n)
+        ft.build_bvh(ctx, ft.particles(*s), t, stream=st)
+        idx = torch.empty(n * 16, dtype=torch.uint64, device="cuda")
+        dist = torch.empty(n * 16, dtype=torch.float64, device="cuda")
+        ft.self_knn_query(ctx, t, 16, idx, dist, stream=st)
+        t.free()
+        got.append((idx, dist))
+    torch.cuda.synchronize()
+    for i, (idx, dist) in enumerate(got):
+        assert torch.equal(idx, want[i % 8][0].reshape(-1)) and torch.equal(dist, want[i % 8][1].reshape(-1)), i
+    # the context goes before its tree
+    t = ft.TreeSoA(ctx, n)
+    ft.build_bvh(ctx, ft.particles(*sets[0]), t)
+    other = ft.Context("f32", "morton")
+    t.ctx = other
+    del ctx
+    t2 = ft.TreeSoA(other, n)
+    ft.build_bvh(other, ft.particles(*sets[1]), t2)
+    for tree, w in ((t, want[0]), (t2, want[1])):
+        r = ft.self_knn_query(other, tree, 16)
+        torch.cuda.synchronize()
+        assert torch.equal(r[0], w[0]) and torch.equal(r[1], w[1])
+    t.free()
+    # four threads build trees of one context
+    trees = [[None] * 6 for _ in range(4)]
+
+    def work(k):
+        st = torch.cuda.Stream()
+        for j in range(6):
+            tr = ft.TreeSoA(other, n)
+            ft.build_bvh(other, ft.particles(*sets[(k + j) % 8]), tr, stream=st)
+            if j % 2:
+                trees[k][j] = tr
+            else:
+                tr.free()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    for k in range(4):
+        for j in (1, 3, 5):
+            r = ft.self_knn_query(other, trees[k][j], 16)
+            torch.cuda.synchronize()
+            w = want[(k + j) % 8]
+            assert torch.equal(r[0], w[0]) and torch.equal(r[1], w[1])
