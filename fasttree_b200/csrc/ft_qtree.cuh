@@ -67,7 +67,7 @@ template <class T> struct QFrame {
     double   s;     // units per coordinate (floating point)
     int      shift; // integers: right shift, negative: left
     uint32_t m;     // margin in units
-    float    k2, slack; // distance -> units^2: limit(d) = d * k2 + slack
+    float    ka, kb, slack; // distance -> units^2: limit(d) = d * ka * kb + slack
     bool     ok, overflow;
 
     // box: the root box (minx, maxx, miny, maxy, minz, maxz); n: leaves
@@ -78,7 +78,7 @@ template <class T> struct QFrame {
         shift = 0;
         m     = 1u;
         slack = 0.0f;
-        k2    = 1.0f;
+        ka = kb = 1.0f;
 #pragma unroll
         for (int a = 0; a < 3; ++a) o[a] = box[2 * a];
         if constexpr (C::is_float) {
@@ -89,15 +89,15 @@ template <class T> struct QFrame {
                 if (!(e >= 0.0) || !(fabs((double)box[2 * a]) <= 1e300)) ok = false; // NaN or an empty box
                 span = fmax(span, e);
             }
-            // units^2 and their inverses stay normal floats, and distances keyable ones
-            if (!(span > 1e-9 && span < 1e18)) ok = false;
-            if (!ok) return;
-            // span < 2^(x + 1): span * 2^(29 - x) < 2^30, and 2^(29 - x) is exact
+            // span < 2^(x + 1): span * 2^(29 - x) < 2^30, and 2^(29 - x) is exact, a normal float for
+            // -97 <= x <= 126 (spans of 1e-29 to 1e38: distances beyond have no float keys)
             const int x = (int)((__double_as_longlong(span) >> 52) & 2047) - 1023;
-            s           = __longlong_as_double((long long)(1023 + 29 - x) << 52);
-            const double s2 = s * s;
-            k2    = __double2float_ru(s2 * (1.0 + 0x1p-17));
-            slack = __double2float_ru(s2 * 0x1p-140); // distances that underflow
+            if (x < -97 || x > 126) ok = false;
+            if (!ok) return;
+            s     = __longlong_as_double((long long)(1023 + 29 - x) << 52);
+            ka    = (float)s; // (in two steps: s^2 may be no float, and d * s is one where d * s^2 is)
+            kb    = (float)s * (1.0f + 0x1p-17f);
+            slack = __double2float_ru(s * s * 0x1p-140); // distances that underflow
         } else {
             int sh; // right shift from coordinate units to frame units
             if (periodic) {
@@ -124,12 +124,16 @@ template <class T> struct QFrame {
             const int du = C::dist_shift - sh;
             m            = 1u + (C::dist_shift > 0 ? (du > 0 ? 1u << min(du, 31) : 1u) : 0u); // du <= 31
             // distance units are 2^dist_shift coordinate units: factor 4^(dist_shift - sh)
-            k2 = __int_as_float((127 + 2 * du) << 23) * (1.0f + 0x1p-17f);
+            kb = __int_as_float((127 + 2 * du) << 23) * (1.0f + 0x1p-17f);
         }
     }
     // the flag's part that follows from the root box
     FT_D uint32_t flag() const { return (ok ? 0u : QFLAG_FRAME) | (overflow ? QFLAG_OVERFLOW : 0u); }
-    FT_D float limit(float key) const { return fmaf(key, k2, slack); }
+    FT_D float limit(float key) const {
+        const float l = fmaf(key * ka, kb, slack);
+        // (FLT_MAX keys every finite distance from there up)
+        return C::is_float && key >= FLT_MAX ? __int_as_float(0x7f800000) : l;
+    }
 
     // position in units; in the tree (or a periodic query): always representable
     FT_D int32_t pos(T v, int a) const {

@@ -687,9 +687,9 @@ template <class T, class D> FT_D RangeLimits range_limits(const QFrame<T> &f, D 
     };
     RangeLimits l;
     l.out = RM2 >= D(0) ? f.limit(up(RM2)) : -1.0f; // (a radius that is not a number reaches nothing)
-    l.in  = down(RM2) * f.k2 * (1.0f - 0x1p-15f) - f.slack;
+    l.in  = down(RM2) * f.ka * f.kb * (1.0f - 0x1p-15f) - f.slack;
     l.ge  = rm2 <= D(0) ? 0.0f : f.limit(up(rm2)); // (not a number: no box lies beyond it)
-    l.lt  = down(rm2) * f.k2 * (1.0f - 0x1p-15f) - f.slack;
+    l.lt  = down(rm2) * f.ka * f.kb * (1.0f - 0x1p-15f) - f.slack;
     return l;
 }
 

@@ -131,7 +131,10 @@ def test_shapes_of_the_box(coord, sfc, per, kind):
 
 
 @pytest.mark.parametrize("coord,span,lo", [("f64", 1e-10, 0.0), ("f64", 3e-9, 1.0), ("f64", 1e-3, 1e6), ("f64", 1e20, 0.0),
-                                           ("f64", 1e26, -5e25), ("f32", 1e-12, 0.0), ("f32", 1e-4, 0.0),
+                                           ("f64", 1e26, -5e25), ("f64", 1e-28, 0.0),
+                                           ("f64", 1e-31, 0.0), ("f64", 1e37, 0.0), ("f64", 1e40, 1e39),
+                                           ("f32", 1e-28, 0.0), ("f32", 1e-32, 0.0), ("f32", 1e37, -5e36),
+                                           ("f32", 1e-12, 0.0), ("f32", 1e-4, 0.0),
                                            ("f32", 4.0, 1000.0), ("f32", 1e18, 0.0), ("u64", 100.0, 5.0),
                                            ("u64", 2.0**13, 2.0**50), ("u64", 2.0**42, 0.0), ("u64", 2.0**45, 7.0),
                                            ("u32", 50.0, 3.0), ("u32", 2.0**31, 9.0)])
@@ -215,3 +218,20 @@ def test_radii_that_are_not_numbers(coord):
             want = want or (res, cnt)
             assert (cnt.cpu().numpy()[bad] == 0).all(), (walk, rows)
             assert torch.equal(cnt, want[1]) and torch.equal(res, want[0]), (walk, rows)
+
+
+@pytest.mark.parametrize("coord,powers", [("f64", (-40, -90, 40, 61)), ("f32", (-20, -40, 40, 58))], ids=["f64", "f32"])
+def test_walks_do_not_depend_on_the_unit(coord, powers):
+    """Points scaled by a power of two: the same rows, and after the same walk (visits counted) as long
+    as squared distances are normal floats: whether positions are given in metres or in megaparsecs."""
+    p = np.random.default_rng(6).random((3, 20_000))
+    want = None
+    for e in (0,) + powers:
+        xyz = [(a.astype(NP[coord]) * NP[coord](2.0**e)) for a in p]
+        ctx, tree = build(coord, "morton", False, xyz)
+        i, d = ft.self_knn_query(ctx, tree, 16)
+        torch.cuda.synchronize()
+        got = (i.cpu().numpy(), d.cpu().numpy() * 2.0 ** (-2 * e), ctx.query_stats()["visits"])
+        want = want or got
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), e
+        assert got[2] == want[2] or got[1].min() * 2.0 ** (2 * e) < 2.0**-126, e
