@@ -567,57 +567,64 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
             __syncwarp();
         }
     }
-    if (binary_walk) {
-        // exact walk over the binary records: leaf children go to the heap as soon as their parent
-        // is expanded, the nearer internal child is walked next, the farther one is stacked
-        int  cur = 0, sp = 0;
-        bool have = true;
+    if (__any_sync(FULL, binary_walk)) {
+        // exact walk over the binary records, the lanes together as above: leaf children within reach
+        // are queued, the nearer internal child is walked next, the farther one is stacked
+        int  cur = 0, sp = 0, qc = 0;
+        bool have  = binary_walk;
         auto needs = [&](D d2) { return !(heap_key<T>(d2) > kthr); };
-        while (have) {
-            if (--budget < 0) {
-                atomicOr(status, STATUS_TRAVERSAL_LIMIT);
-                break;
-            }
-            ++visits;
-            T   lb[6], rb[6];
-            int l, r;
-            load_rec<T, COH>(t.recs, cur, lb, rb, l, r);
-            const D    ld2 = Metric<T>::template dist<(PER != 0), (PER == 2)>(px, py, pz, lb[0], lb[1], lb[2], lb[3], lb[4], lb[5]);
-            const D    rd2 = Metric<T>::template dist<(PER != 0), (PER == 2)>(px, py, pz, rb[0], rb[1], rb[2], rb[3], rb[4], rb[5]);
-            const bool lleaf = l >= n - 1, rleaf = r >= n - 1;
-            const int  lr = l - (n - 1), rr = r - (n - 1);
-#pragma unroll 1
-            for (int side = 0; side < 2; ++side) {
-                const D   d2   = side ? rd2 : ld2;
-                const int leaf = side ? rr : lr;
-                if ((side ? rleaf : lleaf) && needs(d2) && (leaf < w0 || leaf > w1) && leaf != self)
-                    insert_k(d2, heap_key<T>(d2), leaf);
-            }
-            const bool li = !lleaf && needs(ld2), ri = !rleaf && needs(rd2);
-            if (li && ri) {
-                const bool ln = ld2 <= rd2;
-                if (sp >= kWalkStack) {
-                    flag = true; // cannot stack it: the reference traversal reruns the query
-                    break;
+        for (;;) {
+            const bool any = __any_sync(FULL, have);
+            if (!any || __any_sync(FULL, qc > kQueue - 2)) {
+                const int keep = any ? kOfferLanes : 1;
+                while (__popc(__ballot_sync(FULL, qc > 0)) >= keep || __any_sync(FULL, qc > kQueue - 2)) {
+                    if (qc > 0) offer(queue[--qc * kThreads]);
                 }
-                lane_stack[sp++] = ((unsigned long long)__float_as_uint(heap_key<T>(ln ? rd2 : ld2)) << 32) |
-                                   (uint32_t)(ln ? r : l);
-                cur = ln ? l : r;
-            } else if (li) {
-                cur = l;
-            } else if (ri) {
-                cur = r;
-            } else {
+                if (!any) break;
+            }
+            if (have && --budget < 0) {
+                atomicOr(status, STATUS_TRAVERSAL_LIMIT);
                 have = false;
-                while (sp > 0) {
-                    const unsigned long long e = lane_stack[--sp];
-                    if (!(__uint_as_float((uint32_t)(e >> 32)) > kthr)) {
-                        cur  = (int)(uint32_t)e;
-                        have = true;
-                        break;
+            }
+            if (have) {
+                ++visits;
+                T   lb[6], rb[6];
+                int l, r;
+                load_rec<T, COH>(t.recs, cur, lb, rb, l, r);
+                const D    ld2 = Metric<T>::template dist<(PER != 0), (PER == 2)>(px, py, pz, lb[0], lb[1], lb[2], lb[3], lb[4], lb[5]);
+                const D    rd2 = Metric<T>::template dist<(PER != 0), (PER == 2)>(px, py, pz, rb[0], rb[1], rb[2], rb[3], rb[4], rb[5]);
+                const bool ln = needs(ld2), rn = needs(rd2);
+                const int  lr = l - (n - 1), rr = r - (n - 1); // ranks of leaves
+                if (ln && lr >= 0 && (lr < w0 || lr > w1) && lr != self) queue[qc++ * kThreads] = lr;
+                if (rn && rr >= 0 && (rr < w0 || rr > w1) && rr != self) queue[qc++ * kThreads] = rr;
+                const bool li = ln && lr < 0, ri = rn && rr < 0;
+                if (li && ri) {
+                    const bool left = ld2 <= rd2;
+                    if (sp >= kWalkStack) {
+                        flag = true; // cannot stack it: the reference traversal reruns the query
+                        have = false;
+                    } else {
+                        lane_stack[sp++] = ((unsigned long long)__float_as_uint(heap_key<T>(left ? rd2 : ld2)) << 32) |
+                                           (uint32_t)(left ? r : l);
+                        cur = left ? l : r;
+                    }
+                } else if (li) {
+                    cur = l;
+                } else if (ri) {
+                    cur = r;
+                } else {
+                    have = false;
+                    while (sp > 0) {
+                        const unsigned long long e = lane_stack[--sp];
+                        if (!(__uint_as_float((uint32_t)(e >> 32)) > kthr)) {
+                            cur  = (int)(uint32_t)e;
+                            have = true;
+                            break;
+                        }
                     }
                 }
             }
+            __syncwarp();
         }
     }
     __syncwarp();
