@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(256)
         const long long slot = no + n - 1 + j;
         qpts[g]              = qpoint<T>(mnx[slot], mny[slot], mnz[slot], f, periodic != 0, flag + s);
         if (j < n - 1 && (j == 0 || leaves[ro + j] > kBucket))
-            qrec_node<T>(j, n, recs + ro, leaves + ro, f, qrec + ro, flag + s);
+            qrec_node<T>(j, n, recs + ro, leaves + ro, f, qrec + ro);
     }
 }
 

@@ -459,7 +459,7 @@ FT_D void cta_build_set(int n, const T *__restrict__ x, const T *__restrict__ y,
             const int slot = n - 1 + j;
             o.qpts[j]      = qpoint<T>(o.mnx[slot], o.mny[slot], o.mnz[slot], f, o.periodic != 0, o.qflag);
             if (j < n - 1 && (j == 0 || o.leaves[j] > kBucket))
-                qrec_node<T>(j, n, o.recs, o.leaves, f, o.qrec, o.qflag);
+                qrec_node<T>(j, n, o.recs, o.leaves, f, o.qrec);
         }
     }
     if (tid == 0) *set_height = __ldcg(o.height);

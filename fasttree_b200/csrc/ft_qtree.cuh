@@ -39,7 +39,8 @@ namespace ft {
 #define FT_BUCKET 8
 #endif
 static constexpr int      kBucket     = FT_BUCKET; // most leaves of a bucket (a 3-bit count)
-static constexpr uint32_t kQBucket    = 0x80000000u, kQEmpty = 0xffffffffu;
+// References: a bucket, no child, or a node (28 bits), marked when the frame does not resolve it.
+static constexpr uint32_t kQBucket = 0x80000000u, kQEmpty = 0xffffffffu, kQDense = 0x40000000u, kQNode = 0x0fffffffu;
 static constexpr int      kQMaxLeaves = (1 << 28) - 64; // a bucket's first leaf takes 28 bits
 static_assert(kBucket >= 1 && kBucket <= 8, "a bucket reference has three bits for its size");
 
@@ -49,16 +50,19 @@ FT_HD uint32_t qref_bucket(int first, int count) {
 FT_HD int qref_first(uint32_t r) { return (int)(r & 0x0fffffffu); }
 FT_HD int qref_count(uint32_t r) { return (int)((r >> 28) & 7u) + 1; }
 
-// Bits of the per-tree flag (0: the frame serves the walks).  DENSE, FRAME (no frame for the root
-// box): the exact binary walk serves the tree.  NONFINITE (a coordinate is not finite), OVERFLOW
+// Bits of the per-tree flag (0: the frame serves the walks).  FRAME (no frame for the root box): the
+// exact binary walk serves the tree.  NONFINITE (a coordinate is not finite), OVERFLOW
 // (integer gaps whose squares may leave 64 bits): box distances are not monotone, so only the
 // reference traversal gives its rows.  BOXES (a leaf slot of the caller's whose minimum is not its
 // maximum): the walks take leaves for points, the reference traversal measures to their boxes.
-enum : uint32_t { QFLAG_NONFINITE = 1u, QFLAG_DENSE = 2u, QFLAG_FRAME = 4u, QFLAG_OVERFLOW = 8u, QFLAG_BOXES = 16u };
+enum : uint32_t { QFLAG_NONFINITE = 1u, QFLAG_FRAME = 4u, QFLAG_OVERFLOW = 8u, QFLAG_BOXES = 16u };
 static constexpr uint32_t kQFlagPlain = QFLAG_NONFINITE | QFLAG_OVERFLOW | QFLAG_BOXES;
 // A node of more than kDenseLeaves leaves whose box spans at most 2 kDenseUnits units on every
-// axis: the frame no longer tells its leaves apart (QFLAG_DENSE; the exact walk serves the tree).
-static constexpr int      kDenseLeaves = 256;
+// axis: the frame no longer tells its leaves apart.  Its parent's record marks it (kQDense), and a
+// query that reaches one starts again with the exact walk; the others never see it.  (More than 256 /
+// 1024 leaves, a clump of 600 in 1M points, 1M self and 200K external queries, k = 16: float64 3.25 /
+// 3.63 and 2.19 / 1.89 ms, 42-bit periodic 2.47 / 2.36 and 1.63 / 1.55 ms.)
+static constexpr int      kDenseLeaves = 1024;
 static constexpr uint32_t kDenseUnits  = 8;
 
 template <class T> struct QFrame {
@@ -191,8 +195,7 @@ FT_D float qdist(const int32_t u[3], int32_t cx, int32_t cy, int32_t cz, uint32_
 // The record of internal node v: v's two children, then twice the child with the most leaves
 // (more than kBucket) replaced by its own two.
 template <class T>
-FT_D void qrec_node(int v, int n, const NodeRec<T> *recs, const int32_t *leaves, const QFrame<T> &f, QRec *out,
-                    uint32_t *flag) {
+FT_D void qrec_node(int v, int n, const NodeRec<T> *recs, const int32_t *leaves, const QFrame<T> &f, QRec *out) {
     int      id[4];
     uint32_t cn[4];
     bool     rt[4]; // a right child (its first leaf is its index; a left child's last leaf is)
@@ -261,7 +264,6 @@ FT_D void qrec_node(int v, int n, const NodeRec<T> *recs, const int32_t *leaves,
         ++c;
     }
     QRec       q;
-    bool       dense = false;
     const bool lossy = Coord<T>::is_float || f.shift > 0; // exact frames lose nothing
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -282,10 +284,8 @@ FT_D void qrec_node(int v, int n, const NodeRec<T> *recs, const int32_t *leaves,
         else if (leaf) q.ref[i] = qref_bucket(id[i] - (n - 1), 1);
         else if (cn[i] <= (uint32_t)kBucket)
             q.ref[i] = qref_bucket(rt[i] ? id[i] : id[i] - (int)cn[i] + 1, (int)cn[i]);
-        else q.ref[i] = (uint32_t)id[i];
-        dense = dense || (lossy && !flat && i < c && cn[i] > (uint32_t)kDenseLeaves && hm <= kDenseUnits);
+        else q.ref[i] = (uint32_t)id[i] | (lossy && !flat && cn[i] > (uint32_t)kDenseLeaves && hm <= kDenseUnits ? kQDense : 0u);
     }
-    if (dense) atomicOr(flag, QFLAG_DENSE);
     const uint4 *src = reinterpret_cast<const uint4 *>(&q);
     uint4       *dst = reinterpret_cast<uint4 *>(out + v);
 #pragma unroll

@@ -731,10 +731,11 @@ FT_D float qfar(const int32_t u[3], const uint32_t w[6]) {
 // its own ball, leftmost child first, so it meets its leaves in leaf order.  Lanes whose next
 // node is an internal one expand together and lanes whose next is a bucket test it together.
 // STOP: a lane ends as soon as its row is full (*filled), leaving the count to
-// range_count_group; otherwise it counts on, subtrees inside the shell whole.
+// range_count_group; otherwise it counts on, subtrees inside the shell whole.  A lane that reaches a
+// node the frame does not resolve (kQDense) ends with `dense` set: the caller walks it exactly.
 template <class T, int PER, bool STOP>
 FT_D int range_rows(const TreeDev<T> &t, bool go, const RangePoint<T, PER> &pt, const RangeLimits &lim,
-                    int32_t *__restrict__ results, size_t off, int max_per, int ret_orig, uint32_t *status,
+                    int32_t *__restrict__ results, size_t off, int max_per, int ret_orig, uint32_t *status, bool &dense,
                     bool *filled = nullptr) {
     constexpr int  kRows = 100; // right siblings of a path: at most 1.5 per level of a tree of height <= 62
     const unsigned FULL  = 0xffffffffu;
@@ -760,13 +761,14 @@ FT_D int range_rows(const TreeDev<T> &t, bool go, const RangePoint<T, PER> &pt, 
         bool pop = false;
         if (mb == 0u || 2 * __popc(mi) >= __popc(mb)) {
             if (inner) {
-                const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + cur);
+                const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + (cur & kQNode));
                 uint4        v[8];
 #pragma unroll
                 for (int i = 0; i < (STOP ? 7 : 8); ++i) v[i] = __ldg(p + i);
                 const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
-                if (--budget < 0 || sp + 3 > kRows) {
-                    atomicOr(status, STATUS_TRAVERSAL_LIMIT);
+                if (--budget < 0 || sp + 3 > kRows || (cur & kQDense)) {
+                    if (cur & kQDense) dense = true;
+                    else atomicOr(status, STATUS_TRAVERSAL_LIMIT);
                     have = false;
                 } else {
                     pop = true;
@@ -866,8 +868,9 @@ __global__ void __launch_bounds__(128)
     RangeLimits  lim;
     const bool   framed = range_prepare<T, PER>(t, fr, pt, lim);
     const size_t off    = (size_t)q * (size_t)max_per;
-    int          cnt    = range_rows<T, PER, false>(t, active && framed, pt, lim, results, off, max_per, ret_orig, status);
-    if (active && !framed)
+    bool         dense  = false;
+    int          cnt    = range_rows<T, PER, false>(t, active && framed, pt, lim, results, off, max_per, ret_orig, status, dense);
+    if (active && (!framed || dense))
         cnt = range_one<T, PER>(t, pt.px, pt.py, pt.pz, pt.rm2, pt.RM2, results, off, max_per, ret_orig, status);
     if (active) counts[q] = cnt;
 }
@@ -1063,6 +1066,10 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
         const int base = top - m;
         const int node = lane < m ? sh.stk[base + lane] : -1;
         top            = base;
+        if (__any_sync(FULL, node >= 0 && (node & (int)kQDense))) { // (each lane's own walk then)
+            overflow = true;
+            break;
+        }
         __syncwarp();
         unsigned kl = 0, ki = 0;
         uint32_t rf[4] = {0, 0, 0, 0};
@@ -1124,7 +1131,7 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
 // range_query on trees of height <= 62 with a monotone box distance (default): phase 1 writes
 // each row in the reference's order and stops once the row is full; phase 2 counts the full
 // rows' shells with range_count_group (per lane when the group's bounds cannot help).  Lanes
-// whose query the frame does not hold walk the binary records.
+// whose query the frame does not hold or that meet a dense node walk the binary records.
 template <class T, int PER, bool FORCE = false>
 __global__ void __launch_bounds__(32 * kRangeWarps, FT_RANGE_MINB)
     range_split_kernel(TreeDev<T> t, const T *__restrict__ qx, const T *__restrict__ qy, const T *__restrict__ qz,
@@ -1147,16 +1154,16 @@ __global__ void __launch_bounds__(32 * kRangeWarps, FT_RANGE_MINB)
     RangeLimits  lim;
     const bool   framed = range_prepare<T, PER>(t, fr, pt, lim);
     const size_t off    = (size_t)q * (size_t)max_per;
-    bool         filled = false;
-    int cnt = range_rows<T, PER, true>(t, active && framed, pt, lim, results, off, max_per, ret_orig, status, &filled);
+    bool         filled = false, dense = false;
+    int cnt = range_rows<T, PER, true>(t, active && framed, pt, lim, results, off, max_per, ret_orig, status, dense, &filled);
     const bool need = active && filled;
     if (__any_sync(0xffffffffu, need)) {
         int        total = 0;
         const bool done  = range_count_group<T, PER, FORCE>(t, need, fr, pt, lim, s_sh[warp], total);
-        if (!done) total = range_rows<T, PER, false>(t, need, pt, lim, results, off, 0, ret_orig, status);
+        if (!done) total = range_rows<T, PER, false>(t, need, pt, lim, results, off, 0, ret_orig, status, dense);
         if (need) cnt = total;
     }
-    if (active && !framed)
+    if (active && (!framed || dense))
         cnt = range_one<T, PER>(t, pt.px, pt.py, pt.pz, pt.rm2, pt.RM2, results, off, max_per, ret_orig, status);
     if (active) counts[q] = cnt;
 }

@@ -107,7 +107,7 @@ struct TreeletChild {
 // with the most leaves (more than kBucket) replaced by its own two.  split(c): the split of
 // internal child c; box(c, b): its box.
 template <class T, class Split, class Box>
-FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, uint32_t *flag, Split split, Box box) {
+FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, Split split, Box box) {
     TreeletChild ch[4] = {{l, s, false}, {s + 1, r, true}, {0, -1, false}, {0, -1, false}};
     int          c     = 2;
 #pragma unroll
@@ -133,7 +133,6 @@ FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, uint3
         ++c;
     }
     uint32_t   w[32];
-    bool       dense = false;
     const bool lossy = Coord<T>::is_float || f.shift > 0; // exact frames lose nothing
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -151,11 +150,12 @@ FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, uint3
             flat              = flat && !(b[2 * a] < b[2 * a + 1]);
         }
         const int cnt = ch[i].count();
-        w[24 + i]     = i >= c ? kQEmpty : cnt <= kBucket ? qref_bucket(ch[i].l, cnt) : (uint32_t)ch[i].node();
-        w[28 + i]     = i >= c ? 0u : (uint32_t)cnt;
-        dense         = dense || (lossy && !flat && i < c && cnt > kDenseLeaves && hm <= kDenseUnits);
+        const bool dense = lossy && !flat && cnt > kDenseLeaves && hm <= kDenseUnits;
+        w[24 + i]        = i >= c ? kQEmpty
+                           : cnt <= kBucket ? qref_bucket(ch[i].l, cnt)
+                                            : (uint32_t)ch[i].node() | (dense ? kQDense : 0u);
+        w[28 + i]        = i >= c ? 0u : (uint32_t)cnt;
     }
-    if (dense) atomicOr(flag, QFLAG_DENSE);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         unsigned long long v[4];
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
         treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, cl.count(), cr.count(), l == sp ? 0 : s.nh[sp - b0],
                            sp + 1 == r ? 0 : s.nh[sp + 1 - b0]);
         if (v == 0 || r - l + 1 > kBucket)
-            treelet_qrec<T>(l, r, sp, f, a.qrec + v, a.qflag,
+            treelet_qrec<T>(l, r, sp, f, a.qrec + v,
                             [&](const TreeletChild &c) { return b0 + (int)s.ns[c.node() - b0]; }, child_box);
     }
     __syncthreads();
@@ -770,7 +770,7 @@ __global__ void __launch_bounds__(128) treelet_qrec_kernel(const TreeletArgs<T> 
             const int x = a.left[node];
             return x >= n - 1 ? x - (n - 1) : x;
         };
-        treelet_qrec<T>(l, r, split_of(v), f, a.qrec + v, a.qflag,
+        treelet_qrec<T>(l, r, split_of(v), f, a.qrec + v,
                         [&](const TreeletChild &ch) { return split_of(ch.node()); },
                         [&](const TreeletChild &ch, T b[6]) {
                             const int id = ch.l == ch.r ? ch.l + n - 1 : ch.node();

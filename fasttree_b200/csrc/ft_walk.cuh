@@ -415,8 +415,8 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
     // offered from the middle outwards, nearest on the curve first, so most of it fails the
     // k-th key at once.
     const int W  = seeded ? min(n, 2 * half_window + 1) : 0;
-    const int w0 = active ? max(0, min(rank - half_window, n - W)) : 0;
-    const int w1 = active ? w0 + W - 1 : -1;
+    int       w0 = active ? max(0, min(rank - half_window, n - W)) : 0;
+    int       w1 = active ? w0 + W - 1 : -1;
     {
         const int m  = min(W, k + (self >= 0 ? 1 : 0));
         const int m0 = active ? max(w0, min(rank - (m >> 1), w0 + W - m)) : 0;
@@ -444,7 +444,7 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
     // ---- 2. walk ----
     // A subtree is skipped only when its bound exceeds the limit, so it holds no leaf within
     // the k-th distance; leaves at exactly that distance reach insert_k and raise the tie flag.
-    const bool binary_walk = active && !framed && n > 1;
+    bool exact_walk = active && !framed && n > 1;
     {
         // Warp-synchronous: lanes whose next node is an internal one expand it; a lane that meets a
         // bucket puts it aside and goes on, and waits at its second one, until more lanes wait
@@ -477,7 +477,7 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                 if (inner) {
                     --budget;
                     ++visits;
-                    const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + cur);
+                    const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + (cur & kQNode));
                     uint4        v[7];
 #pragma unroll
                     for (int i = 0; i < 7; ++i) v[i] = ld_rec16<COH>(p + i);
@@ -511,10 +511,14 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                     cx(0, 2);
                     cx(1, 3);
                     cx(1, 2);
-                    if (sp + 3 > kWalkStack || budget < 0) {
-                        // cannot stack them all: the reference traversal reruns the query
-                        if (budget < 0) atomicOr(status, STATUS_TRAVERSAL_LIMIT);
-                        flag = true;
+                    if (sp + 3 > kWalkStack || budget < 0 || (cur & kQDense)) {
+                        if (cur & kQDense) {
+                            exact_walk = true; // the frame does not resolve this node
+                            qc         = 0;
+                        } else { // cannot stack them all: the reference traversal reruns the query
+                            if (budget < 0) atomicOr(status, STATUS_TRAVERSAL_LIMIT);
+                            flag = true;
+                        }
                         have = false;
                         pb   = kQEmpty;
                     } else {
@@ -567,11 +571,19 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
             __syncwarp();
         }
     }
-    if (__any_sync(FULL, binary_walk)) {
+    if (framed && exact_walk) { // from an empty heap: the leaves in it are offered again
+        count  = 0;
+        flag   = false;
+        kthr   = kB;
+        budget = 2ll * n + 64;
+        w0     = 0;
+        w1     = -1;
+    }
+    if (__any_sync(FULL, exact_walk)) {
         // exact walk over the binary records, the lanes together as above: leaf children within reach
         // are queued, the nearer internal child is walked next, the farther one is stacked
         int  cur = 0, sp = 0, qc = 0;
-        bool have  = binary_walk;
+        bool have  = exact_walk;
         auto needs = [&](D d2) { return !(heap_key<T>(d2) > kthr); };
         for (;;) {
             const bool any = __any_sync(FULL, have);

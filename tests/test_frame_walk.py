@@ -235,3 +235,35 @@ def test_walks_do_not_depend_on_the_unit(coord, powers):
         want = want or got
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), e
         assert got[2] == want[2] or got[1].min() * 2.0 ** (2 * e) < 2.0**-126, e
+
+
+@pytest.mark.parametrize("size", [257, 3000])
+@pytest.mark.parametrize("coord,sfc,per", [("f32", "ph", False), ("f64", "morton", False), ("u64", "ph", True),
+                                           ("u64", "ph", False)], ids=["f32", "f64", "u64-per", "u64"])
+def test_dense_nodes_among_others(coord, sfc, per, size):
+    """A clump the frame does not resolve in a box of ordinary points: queries that reach it start
+    again with exact distances, the others do not; single trees, batches of both build methods."""
+    rng = np.random.default_rng(size)
+    b = box(coord)
+    p = rng.random((3, 5000 + size)) * b
+    tight = {"f32": 1e-9, "f64": 1e-11, "u64": 6000.0}[coord]  # (float positions near 0 are that fine)
+    p[:, :size] = (0.0 if coord == "f32" else 0.5 * b) + rng.random((3, size)) * tight
+    xyz = [a.astype(NP[coord]) for a in (np.floor(p) if coord[0] == "u" else p)]
+    ctx, tree = build(coord, sfc, per, xyz)
+    check_self(ctx, tree, (1, 8, 33))
+    q = p[:, rng.permutation(p.shape[1])[:600]] + rng.normal(0, 1e-4 * b, (3, 600)) * (rng.random(600) < 0.5)
+    q = [dev(a.clip(0, b * (1 - 1e-6)).astype(NP[coord])) for a in q]
+    check_points(ctx, tree, q, (8, 40))
+    for r0, r1, rows in ((0, 0.3 * tight, 10), (0, 2e-4 * b, 100), (0.01 * b, 0.1 * b, 8), (0, 0.05 * b, 0)):
+        check_range(ctx, tree, q, r0, r1, rows)
+    if coord == "u64" and not per:
+        return
+    other = [np.concatenate([a[:40], a, a[size:]]) for a in xyz]
+    off = np.array([0, 40, 40 + len(xyz[0]), len(other[0])])
+    bt = ft.BatchedSets(ctx, len(other[0]), 3)
+    for method in ("default", "persistent"):
+        bt.set_build_method(method)
+        bt.build(off, *other)
+        want = bt.self_knn(16, method="plain")
+        want = (want[0].clone(), want[1].clone())
+        assert same(want, bt.self_knn(16)), method
