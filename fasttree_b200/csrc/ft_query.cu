@@ -693,15 +693,26 @@ template <class T, class D> FT_D RangeLimits range_limits(const QFrame<T> &f, D 
     return l;
 }
 
+// Upper bound of the squared distance, in units^2, between the query and any point of a box.
+FT_D float qfar(const int32_t u[3], const uint32_t w[6]) {
+    float f[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        f[a] = (float)(uint32_t)abs((int32_t)((uint32_t)u[a] - w[a])) + (float)w[3 + a];
+    return fmaf(f[2], f[2], fmaf(f[1], f[1], f[0] * f[0])) * (1.0f + 0x1p-20f);
+}
+
 // The point test of one leaf: exactly node_distance_sq's distance against the shell.  From the
-// QPoint where it holds the whole position; else the frame's bound first.
+// QPoint where it holds the whole position; else the frame's bounds first, and the distance from the
+// leaf's coordinates only where they cannot tell (1M float64 points, 200K queries of 600 leaves: every
+// leaf within reach tested exactly 3618 us, so 2868).
 template <class T, int PER> struct RangePoint {
     using D = typename Coord<T>::dist_t;
     T           px, py, pz;
     int32_t     u[3];
     uint32_t    ul[3], m;
     D           rm2, RM2;
-    float       out;
+    float       out, in, ge; // RangeLimits
     const T    *lx, *ly, *lz; // leaf coordinates by rank
     FT_D bool operator()(const uint4 &v, int leaf) const {
         D d;
@@ -711,21 +722,15 @@ template <class T, int PER> struct RangePoint {
         } else if constexpr (qpoint_whole<T, PER>()) {
             d = qexact42(v, u, ul);
         } else {
-            if (qdist(u, (int32_t)v.x, (int32_t)v.y, (int32_t)v.z, m, m, m) > out) return false;
+            const float near = qdist(u, (int32_t)v.x, (int32_t)v.y, (int32_t)v.z, m, m, m);
+            if (near > out) return false;
+            const uint32_t w[6] = {v.x, v.y, v.z, m, m, m};
+            if (near >= ge && qfar(u, w) <= in) return true;
             d = Metric<T>::template point<(PER != 0), (PER == 2)>(px, py, pz, lx[leaf], ly[leaf], lz[leaf]);
         }
         return d >= rm2 && d <= RM2;
     }
 };
-
-// Upper bound of the squared distance, in units^2, between the query and any point of a box.
-FT_D float qfar(const int32_t u[3], const uint32_t w[6]) {
-    float f[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-        f[a] = (float)(uint32_t)abs((int32_t)((uint32_t)u[a] - w[a])) + (float)w[3 + a];
-    return fmaf(f[2], f[2], fmaf(f[1], f[1], f[0] * f[0])) * (1.0f + 0x1p-20f);
-}
 
 // The rows of a warp's queries (every lane calls it; lanes without `go` idle): each lane walks
 // its own ball, leftmost child first, so it meets its leaves in leaf order.  Lanes whose next
@@ -842,6 +847,8 @@ FT_D bool range_prepare(const TreeDev<T> &t, QFrame<T> &fr, RangePoint<T, PER> &
     pt.m   = fr.m;
     lim    = range_limits<T>(fr, pt.rm2, pt.RM2);
     pt.out = lim.out;
+    pt.in  = lim.in;
+    pt.ge  = lim.ge;
     pt.lx  = t.min_x + (t.n - 1);
     pt.ly  = t.min_y + (t.n - 1);
     pt.lz  = t.min_z + (t.n - 1);

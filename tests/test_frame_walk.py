@@ -267,3 +267,23 @@ def test_dense_nodes_among_others(coord, sfc, per, size):
         want = bt.self_knn(16, method="plain")
         want = (want[0].clone(), want[1].clone())
         assert same(want, bt.self_knn(16)), method
+
+
+@pytest.mark.parametrize("coord,per", [("f32", False), ("f64", False), ("u32", True), ("u32", False), ("u64", True),
+                                       ("u64", False)], ids=["f32", "f64", "u32-per", "u32", "u64-per", "u64"])
+def test_shells_that_pass_through_leaves(coord, per):
+    """Points on a lattice and radii at, one step below and one step above its distances: the bounds
+    that decide most leaves must leave those at the shell's edges to the exact distance."""
+    rng = np.random.default_rng(3)
+    n, step = 8000, {"f32": 1 / 16, "f64": 1 / 16, "u32": 1 << 16, "u64": 1 << 37}[coord]
+    xyz = [(rng.integers(0, 16, n) * step).astype(NP[coord]) for _ in range(3)]
+    ctx, tree = build(coord, "ph", per, xyz)
+    q = [dev(a[:500]) for a in xyz]
+    for m in (1, 2, 5):
+        r = NP[coord](m * step)
+        unit = NP[coord]({"u32": 1, "u64": 1 << 11}.get(coord, 0))
+        below, above = (r - unit, r + unit) if coord[0] == "u" else (np.nextafter(r, NP[coord](0)),
+                                                                     np.nextafter(r, NP[coord](9)))
+        for r0, r1 in ((0, r), (0, below), (0, above), (r, r), (below, r), (above, r + r), (below, above)):
+            check_range(ctx, tree, q, r0, r1, 0)
+            check_range(ctx, tree, q, r0, r1, 40)
