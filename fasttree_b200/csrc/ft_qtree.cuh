@@ -182,6 +182,20 @@ template <class T> struct QFrame {
     }
 };
 
+// Open integers: whether the squares of a point's gaps to the root box `rb` may leave 64 bits.  Its
+// box distances are not monotone then (a tree of that span is flagged, QFLAG_OVERFLOW).
+template <class T> FT_D bool open_gaps_wrap(T px, T py, T pz, const T rb[6]) {
+    const T            p[3] = {px, py, pz};
+    unsigned long long g    = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const T lo = rb[2 * a], hi = rb[2 * a + 1];
+        g          = max(g, max((unsigned long long)(p[a] > lo ? p[a] - lo : lo - p[a]),
+                                (unsigned long long)(p[a] > hi ? p[a] - hi : hi - p[a])));
+    }
+    return ((g >> Coord<T>::dist_shift) >> 31) != 0;
+}
+
 // Bound of one axis: |u - c| - h, not below zero.
 FT_D float qgap(int32_t u, int32_t c, uint32_t h) {
     const uint32_t a = (uint32_t)abs((int32_t)((uint32_t)u - (uint32_t)c));

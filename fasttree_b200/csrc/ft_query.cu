@@ -852,6 +852,8 @@ FT_D bool range_prepare(const TreeDev<T> &t, QFrame<T> &fr, RangePoint<T, PER> &
     pt.lx  = t.min_x + (t.n - 1);
     pt.ly  = t.min_y + (t.n - 1);
     pt.lz  = t.min_z + (t.n - 1);
+    if constexpr (PER == 0 && !Coord<T>::is_float)
+        if (open_gaps_wrap<T>(pt.px, pt.py, pt.pz, rb)) return false;
     return fr.ok && a && b && c;
 }
 

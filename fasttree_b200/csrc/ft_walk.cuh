@@ -260,6 +260,12 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
     {
         const T rb[6] = {t.min_x[0], t.max_x[0], t.min_y[0], t.max_y[0], t.min_z[0], t.max_z[0]};
         fr.make(rb, n, PER != 0);
+        if constexpr (PER == 0 && !Coord<T>::is_float) {
+            if (ext && active && open_gaps_wrap<T>(px, py, pz, rb)) { // only the reference traversal applies
+                force_replay = true;
+                active       = false;
+            }
+        }
         framed = !binary && fr.ok && *t.qflag == 0u;
         if (framed) {
             const bool a = fr.template query<(PER != 0)>(px, 0, u[0]), b = fr.template query<(PER != 0)>(py, 1, u[1]),

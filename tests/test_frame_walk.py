@@ -287,3 +287,20 @@ def test_shells_that_pass_through_leaves(coord, per):
         for r0, r1 in ((0, r), (0, below), (0, above), (r, r), (below, r), (above, r + r), (below, above)):
             check_range(ctx, tree, q, r0, r1, 0)
             check_range(ctx, tree, q, r0, r1, 40)
+
+
+@pytest.mark.parametrize("coord,bits", [("u64", 42), ("u32", 31)], ids=["u64", "u32"])
+def test_query_points_whose_squared_gaps_wrap(coord, bits):
+    """External points so far off that the squares of their gaps leave 64 bits: such distances wrap,
+    and rows are the reference traversal's."""
+    rng = np.random.default_rng(1)
+    xyz = [(rng.random(6000) * 2.0**bits).astype(NP[coord]) for _ in range(3)]
+    ctx, tree = build(coord, "ph", False, xyz)
+    top = 2.0 ** (32 - bits) if coord == "u32" else 1e5
+    for lo, hi in ((1.0, 1.3), (1.0, 1.9), (0.5, 3.0), (3.0, 30.0), (1e3, 1e5)):
+        q = [(lo + (min(hi, top * 0.999) - lo) * rng.random(500)) * 2.0**bits for _ in range(3)]
+        if lo < top:
+            q = [dev(a.astype(NP[coord])) for a in q]
+            check_points(ctx, tree, q, (1, 8, 40))
+            for r in (0.1, 0.9):
+                check_range(ctx, tree, q, 0, r * 2.0**bits, 20)
