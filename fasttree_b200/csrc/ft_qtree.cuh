@@ -39,8 +39,8 @@ namespace ft {
 #define FT_BUCKET 8
 #endif
 static constexpr int      kBucket     = FT_BUCKET; // most leaves of a bucket (a 3-bit count)
-// References: a bucket, no child, or a node (28 bits), marked when the frame does not resolve it.
-static constexpr uint32_t kQBucket = 0x80000000u, kQEmpty = 0xffffffffu, kQDense = 0x40000000u, kQNode = 0x0fffffffu;
+// References: a node, a bucket, or no child.  A record without any child is a dense node's (below).
+static constexpr uint32_t kQBucket = 0x80000000u, kQEmpty = 0xffffffffu;
 static constexpr int      kQMaxLeaves = (1 << 28) - 64; // a bucket's first leaf takes 28 bits
 static_assert(kBucket >= 1 && kBucket <= 8, "a bucket reference has three bits for its size");
 
@@ -58,8 +58,8 @@ FT_HD int qref_count(uint32_t r) { return (int)((r >> 28) & 7u) + 1; }
 enum : uint32_t { QFLAG_NONFINITE = 1u, QFLAG_FRAME = 4u, QFLAG_OVERFLOW = 8u, QFLAG_BOXES = 16u };
 static constexpr uint32_t kQFlagPlain = QFLAG_NONFINITE | QFLAG_OVERFLOW | QFLAG_BOXES;
 // A node of more than kDenseLeaves leaves whose box spans at most 2 kDenseUnits units on every
-// axis: the frame no longer tells its leaves apart.  Its parent's record marks it (kQDense), and a
-// query that reaches one starts again with the exact walk; the others never see it.  (More than 256 /
+// axis: the frame no longer tells its leaves apart.  Its record has no children, and a query that
+// reaches it starts again with the exact walk; the others never see it.  (More than 256 /
 // 1024 leaves, a clump of 600 in 1M points, 1M self and 200K external queries, k = 16: float64 3.25 /
 // 3.63 and 2.19 / 1.89 ms, 42-bit periodic 2.47 / 2.36 and 1.63 / 1.55 ms.)
 static constexpr int      kDenseLeaves = 1024;
@@ -196,6 +196,19 @@ template <class T> FT_D bool open_gaps_wrap(T px, T py, T pz, const T rb[6]) {
     return ((g >> Coord<T>::dist_shift) >> 31) != 0;
 }
 
+// Whether a node of n leaves and the box b is dense.
+template <class T> FT_D bool qdense(int n, const T b[6], const QFrame<T> &f) {
+    if (n <= kDenseLeaves || !(Coord<T>::is_float || f.shift > 0)) return false; // exact frames lose nothing
+    uint32_t hm   = 0;
+    bool     flat = true; // copies of one point: no frame tells them apart
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        hm   = max(hm, (uint32_t)f.pos(b[2 * a + 1], a) - (uint32_t)f.pos(b[2 * a], a));
+        flat = flat && !(b[2 * a] < b[2 * a + 1]);
+    }
+    return !flat && hm <= 2 * kDenseUnits;
+}
+
 // Bound of one axis: |u - c| - h, not below zero.
 FT_D float qgap(int32_t u, int32_t c, uint32_t h) {
     const uint32_t a = (uint32_t)abs((int32_t)((uint32_t)u - (uint32_t)c));
@@ -234,6 +247,13 @@ FT_D void qrec_node(int v, int n, const NodeRec<T> *recs, const int32_t *leaves,
         cn[1] = count_of(id[1], ir);
         rt[1] = true;
     }
+    T own[6];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        own[2 * a]     = box_min(bx[0][2 * a], bx[1][2 * a]);
+        own[2 * a + 1] = box_max(bx[0][2 * a + 1], bx[1][2 * a + 1]);
+    }
+    const bool dense = qdense<T>((int)(cn[0] + cn[1]), own, f);
 #pragma unroll
     for (int step = 0; step < 2; ++step) {
         int      b  = -1, bid = 0;
@@ -277,20 +297,15 @@ FT_D void qrec_node(int v, int n, const NodeRec<T> *recs, const int32_t *leaves,
         }
         ++c;
     }
-    QRec       q;
-    const bool lossy = Coord<T>::is_float || f.shift > 0; // exact frames lose nothing
+    QRec q;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        uint32_t hm   = 0;
-        bool     flat = true; // copies of one point: no frame tells them apart
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const uint32_t lo = (uint32_t)f.pos(bx[i][2 * a], a), hi = (uint32_t)f.pos(bx[i][2 * a + 1], a);
             const uint32_t ce = lo + ((hi - lo) >> 1);
             q.c[i][a]         = (int32_t)ce;
             q.c[i][3 + a]     = (int32_t)((hi - ce) + f.m);
-            hm                = max(hm, hi - ce);
-            flat              = flat && !(bx[i][2 * a] < bx[i][2 * a + 1]);
         }
         const bool leaf = id[i] >= n - 1;
         q.cnt[i]        = i < c ? cn[i] : 0u;
@@ -298,7 +313,8 @@ FT_D void qrec_node(int v, int n, const NodeRec<T> *recs, const int32_t *leaves,
         else if (leaf) q.ref[i] = qref_bucket(id[i] - (n - 1), 1);
         else if (cn[i] <= (uint32_t)kBucket)
             q.ref[i] = qref_bucket(rt[i] ? id[i] : id[i] - (int)cn[i] + 1, (int)cn[i]);
-        else q.ref[i] = (uint32_t)id[i] | (lossy && !flat && cn[i] > (uint32_t)kDenseLeaves && hm <= kDenseUnits ? kQDense : 0u);
+        else q.ref[i] = (uint32_t)id[i];
+        if (dense) q.ref[i] = kQEmpty;
     }
     const uint4 *src = reinterpret_cast<const uint4 *>(&q);
     uint4       *dst = reinterpret_cast<uint4 *>(out + v);

@@ -737,7 +737,7 @@ template <class T, int PER> struct RangePoint {
 // node is an internal one expand together and lanes whose next is a bucket test it together.
 // STOP: a lane ends as soon as its row is full (*filled), leaving the count to
 // range_count_group; otherwise it counts on, subtrees inside the shell whole.  A lane that reaches a
-// node the frame does not resolve (kQDense) ends with `dense` set: the caller walks it exactly.
+// dense node ends with `dense` set: the caller walks it exactly.
 template <class T, int PER, bool STOP>
 FT_D int range_rows(const TreeDev<T> &t, bool go, const RangePoint<T, PER> &pt, const RangeLimits &lim,
                     int32_t *__restrict__ results, size_t off, int max_per, int ret_orig, uint32_t *status, bool &dense,
@@ -766,15 +766,17 @@ FT_D int range_rows(const TreeDev<T> &t, bool go, const RangePoint<T, PER> &pt, 
         bool pop = false;
         if (mb == 0u || 2 * __popc(mi) >= __popc(mb)) {
             if (inner) {
-                const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + (cur & kQNode));
+                const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + cur);
                 uint4        v[8];
 #pragma unroll
                 for (int i = 0; i < (STOP ? 7 : 8); ++i) v[i] = __ldg(p + i);
                 const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
-                if (--budget < 0 || sp + 3 > kRows || (cur & kQDense)) {
-                    if (cur & kQDense) dense = true;
-                    else atomicOr(status, STATUS_TRAVERSAL_LIMIT);
+                if (--budget < 0 || sp + 3 > kRows) {
+                    atomicOr(status, STATUS_TRAVERSAL_LIMIT);
                     have = false;
+                } else if (w[24] == kQEmpty) {
+                    dense = true;
+                    have  = false;
                 } else {
                     pop = true;
 #pragma unroll
@@ -1075,10 +1077,6 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
         const int base = top - m;
         const int node = lane < m ? sh.stk[base + lane] : -1;
         top            = base;
-        if (__any_sync(FULL, node >= 0 && (node & (int)kQDense))) { // (each lane's own walk then)
-            overflow = true;
-            break;
-        }
         __syncwarp();
         unsigned kl = 0, ki = 0;
         uint32_t rf[4] = {0, 0, 0, 0};
@@ -1109,6 +1107,10 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
                 else if (rf[i] & kQBucket) kl |= 1u << i;
                 else ki |= 1u << i;
             }
+        }
+        if (__any_sync(FULL, node >= 0 && rf[0] == kQEmpty)) { // a dense node: each lane's own walk
+            overflow = true;
+            break;
         }
         const int nl = __popc(kl), ni = __popc(ki);
         int       incl = nl | (ni << 16);

@@ -103,11 +103,11 @@ struct TreeletChild {
     FT_D int node() const { return right ? l : r; } // internal number (l < r)
 };
 
-// The walk record of a node covering [l, r] with split s: its two children, then twice the child
+// The walk record of a node covering [l, r] with split s and box `own`: its two children, then twice the child
 // with the most leaves (more than kBucket) replaced by its own two.  split(c): the split of
 // internal child c; box(c, b): its box.
 template <class T, class Split, class Box>
-FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, Split split, Box box) {
+FT_D void treelet_qrec(int l, int r, int s, const T own[6], const QFrame<T> &f, QRec *out, Split split, Box box) {
     TreeletChild ch[4] = {{l, s, false}, {s + 1, r, true}, {0, -1, false}, {0, -1, false}};
     int          c     = 2;
 #pragma unroll
@@ -133,28 +133,21 @@ FT_D void treelet_qrec(int l, int r, int s, const QFrame<T> &f, QRec *out, Split
         ++c;
     }
     uint32_t   w[32];
-    const bool lossy = Coord<T>::is_float || f.shift > 0; // exact frames lose nothing
+    const bool dense = qdense<T>(r - l + 1, own, f);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         T b[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
         if (i < c) box(ch[i], b);
-        uint32_t hm   = 0;
-        bool     flat = true; // copies of one point: no frame tells them apart
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const uint32_t lo = (uint32_t)f.pos(b[2 * a], a), hi = (uint32_t)f.pos(b[2 * a + 1], a);
             const uint32_t ce = lo + ((hi - lo) >> 1);
             w[6 * i + a]      = ce;
             w[6 * i + 3 + a]  = (hi - ce) + f.m;
-            hm                = max(hm, hi - ce);
-            flat              = flat && !(b[2 * a] < b[2 * a + 1]);
         }
         const int cnt = ch[i].count();
-        const bool dense = lossy && !flat && cnt > kDenseLeaves && hm <= kDenseUnits;
-        w[24 + i]        = i >= c ? kQEmpty
-                           : cnt <= kBucket ? qref_bucket(ch[i].l, cnt)
-                                            : (uint32_t)ch[i].node() | (dense ? kQDense : 0u);
-        w[28 + i]        = i >= c ? 0u : (uint32_t)cnt;
+        w[24 + i]     = i >= c || dense ? kQEmpty : cnt <= kBucket ? qref_bucket(ch[i].l, cnt) : (uint32_t)ch[i].node();
+        w[28 + i]     = i >= c ? 0u : (uint32_t)cnt;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -405,22 +398,22 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
         T                  lb[6], rb[6];
         child_box(cl, lb);
         child_box(cr, rb);
+        T own[6];
 #pragma unroll
-        for (int d = 0; d < 6; ++d) a.soa[d][v] = s.bx[d][j];
+        for (int d = 0; d < 6; ++d) own[d] = s.bx[d][j];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) a.soa[d][v] = own[d];
         a.left[v]   = lc;
         a.right[v]  = rc;
         a.parent[lc] = v;
         a.parent[rc] = v;
         a.leaves[v] = r - l + 1;
         a.height[v] = (uint8_t)h;
-        if (v == 0) { // (number 0 is the root's)
-            const T rb0[6] = {s.bx[0][0], s.bx[1][0], s.bx[2][0], s.bx[3][0], s.bx[4][0], s.bx[5][0]};
-            treelet_root<T>(a, rb0);
-        }
+        if (v == 0) treelet_root<T>(a, own); // (number 0 is the root's)
         treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, cl.count(), cr.count(), l == sp ? 0 : s.nh[sp - b0],
                            sp + 1 == r ? 0 : s.nh[sp + 1 - b0]);
         if (v == 0 || r - l + 1 > kBucket)
-            treelet_qrec<T>(l, r, sp, f, a.qrec + v,
+            treelet_qrec<T>(l, r, sp, own, f, a.qrec + v,
                             [&](const TreeletChild &c) { return b0 + (int)s.ns[c.node() - b0]; }, child_box);
     }
     __syncthreads();
@@ -770,7 +763,10 @@ __global__ void __launch_bounds__(128) treelet_qrec_kernel(const TreeletArgs<T> 
             const int x = a.left[node];
             return x >= n - 1 ? x - (n - 1) : x;
         };
-        treelet_qrec<T>(l, r, split_of(v), f, a.qrec + v,
+        T own[6];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) own[d] = a.soa[d][v];
+        treelet_qrec<T>(l, r, split_of(v), own, f, a.qrec + v,
                         [&](const TreeletChild &ch) { return split_of(ch.node()); },
                         [&](const TreeletChild &ch, T b[6]) {
                             const int id = ch.l == ch.r ? ch.l + n - 1 : ch.node();

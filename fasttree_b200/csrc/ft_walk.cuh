@@ -450,7 +450,6 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
     // ---- 2. walk ----
     // A subtree is skipped only when its bound exceeds the limit, so it holds no leaf within
     // the k-th distance; leaves at exactly that distance reach insert_k and raise the tie flag.
-    bool exact_walk = active && !framed && n > 1;
     {
         // Warp-synchronous: lanes whose next node is an internal one expand it; a lane that meets a
         // bucket puts it aside and goes on, and waits at its second one, until more lanes wait
@@ -483,7 +482,7 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                 if (inner) {
                     --budget;
                     ++visits;
-                    const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + (cur & kQNode));
+                    const uint4 *p = reinterpret_cast<const uint4 *>(t.qrec + cur);
                     uint4        v[7];
 #pragma unroll
                     for (int i = 0; i < 7; ++i) v[i] = ld_rec16<COH>(p + i);
@@ -517,14 +516,10 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                     cx(0, 2);
                     cx(1, 3);
                     cx(1, 2);
-                    if (sp + 3 > kWalkStack || budget < 0 || (cur & kQDense)) {
-                        if (cur & kQDense) {
-                            exact_walk = true; // the frame does not resolve this node
-                            qc         = 0;
-                        } else { // cannot stack them all: the reference traversal reruns the query
-                            if (budget < 0) atomicOr(status, STATUS_TRAVERSAL_LIMIT);
-                            flag = true;
-                        }
+                    if (sp + 3 > kWalkStack || budget < 0) {
+                        // cannot stack them all: the reference traversal reruns the query
+                        if (budget < 0) atomicOr(status, STATUS_TRAVERSAL_LIMIT);
+                        flag = true;
                         have = false;
                         pb   = kQEmpty;
                     } else {
@@ -534,7 +529,14 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
                         sp += max(nv - 1, 0);
                         cur = nv == 1 ? oc[0] : nv == 2 ? oc[1] : nv == 3 ? oc[2] : oc[3];
                         pop = nv == 0;
-                        if (!pop && (cur & kQBucket) && pb == kQEmpty) {
+                        if (pop) {
+                            if (oc[0] == kQEmpty) { // (unsorted) a dense node: the exact walk takes the query
+                                count = -1;
+                                have = pop = false;
+                                pb         = kQEmpty;
+                                qc         = 0;
+                            }
+                        } else if ((cur & kQBucket) && pb == kQEmpty) {
                             pb  = cur;
                             pop = true;
                         }
@@ -577,7 +579,8 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
             __syncwarp();
         }
     }
-    if (framed && exact_walk) { // from an empty heap: the leaves in it are offered again
+    const bool exact_walk = active && n > 1 && (!framed || count < 0);
+    if (count < 0) { // from an empty heap: the leaves in it are offered again
         count  = 0;
         flag   = false;
         kthr   = kB;
