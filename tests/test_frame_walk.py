@@ -304,3 +304,52 @@ def test_query_points_whose_squared_gaps_wrap(coord, bits):
             check_points(ctx, tree, q, (1, 8, 40))
             for r in (0.1, 0.9):
                 check_range(ctx, tree, q, 0, r * 2.0**bits, 20)
+
+
+@pytest.mark.parametrize("coord", ["f32", "f64"])
+@pytest.mark.parametrize("n", [40, 3000, 9000])
+def test_coordinates_that_are_not_finite(coord, n):
+    """NaN and infinite coordinates in a build, a refit, one set of a batch and query points: the
+    default method's rows are the reference traversal's."""
+    rng = np.random.default_rng(n)
+    ok = [rng.random(n).astype(NP[coord]) for _ in range(3)]
+    bad = [a.copy() for a in ok]
+    bad[0][3], bad[1][n // 2], bad[2][n - 2] = np.nan, np.inf, -np.inf
+    ctx, tree = build(coord, "morton", False, bad)
+    check_self(ctx, tree, (1, 8, 33))
+    q = [dev(a[:40]) for a in ok]
+    check_points(ctx, tree, q, (4, 40))
+    ft.refit_bvh(ctx, ft.particles(*ok), tree)
+    check_self(ctx, tree, (8,))
+    ft.refit_bvh(ctx, ft.particles(*bad), tree)
+    check_self(ctx, tree, (8,))
+    ctx, tree = build(coord, "morton", False, ok)
+    odd = rng.random((3, 64)).astype(NP[coord])
+    odd[0, ::7], odd[1, ::11], odd[2, ::13] = np.nan, np.inf, -np.inf
+    check_points(ctx, tree, [dev(a) for a in odd], (1, 9, 40))
+    off = np.array([0, n, 2 * n, 2 * n + 1, 3 * n + 1])
+    one = np.full(1, np.nan, NP[coord])
+    xyz = [np.concatenate([a, b, one, a]) for a, b in zip(ok, bad)]
+    b = ft.BatchedSets(ctx, len(xyz[0]), 4)
+    for method in ("default", "persistent"):
+        b.set_build_method(method)
+        b.build(off, *xyz)
+        want = b.self_knn(8, method="plain")
+        want = (want[0].clone(), want[1].clone())
+        got = b.self_knn(8)
+        assert same(want, got), method
+
+
+@pytest.mark.parametrize("k", [4, 8, 40])
+@pytest.mark.parametrize("shift", [0, 1, 2, 4])
+def test_rows_that_start_off_a_sector(k, shift):
+    """Output arrays 8, 16 and 32 bytes into an allocation: the same rows as aligned ones."""
+    xyz = to_coord(points("uniform", 5000, "u64", 3), "u64")
+    ctx, tree = build("u64", "ph", True, xyz)
+    want = ft.self_knn_query(ctx, tree, k, max_k=64, method="plain")
+    idx = torch.zeros(5000 * k + 8, dtype=want[0].dtype, device="cuda")
+    dist = torch.zeros(5000 * k + 8, dtype=want[1].dtype, device="cuda")
+    for a, b in ((shift, shift), (0, shift), (shift, 0)):
+        i, d = idx[a:a + 5000 * k], dist[b:b + 5000 * k]
+        ft.self_knn_query(ctx, tree, k, i, d, max_k=64)
+        assert same((want[0].reshape(-1), want[1].reshape(-1)), (i, d)), (a, b)

@@ -248,10 +248,10 @@ def test_fast_self_knn_matches_oracle(cfg, kind, k):
 
 
 @pytest.mark.parametrize("cfg", CONFIGS, ids=CONFIG_IDS)
-@pytest.mark.parametrize("variant", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("variant", [2, 4])
 def test_fast_walk_variants_match_oracle(cfg, variant):
-    """Every walk of the fast path (1 per-lane, 2 compact per-lane, 3 warp-shared, 4 over the
-    4-wide records, 5 the group walk) gives the reference's output, ties included."""
+    """Every walk of the fast path (2 the exact binary walk, 4 over the 4-wide records) gives the
+    reference's output, ties included."""
     coord, sfc, per = cfg
     ctx, opts = make(coord, sfc, per)
     for kind, k in (("clustered", 32), ("degenerate", 16), ("uniform", 64)):
@@ -283,7 +283,7 @@ def test_fast_self_knn_subset_and_orig(cfg):
             assert np.array_equal(dist_bits(gd.cpu().numpy()), dist_bits(od))
 
 
-@pytest.mark.parametrize("method,variant", [("plain", 0), ("fast", 0), ("fast", 5)])
+@pytest.mark.parametrize("method,variant", [("plain", 0), ("fast", 0), ("fast", 2)])
 def test_periodic_wrap_edges_u64(method, variant):
     """42-bit periodic distances at the wrap: points at 0, 2^41 (half the period) and
     2^42 - 1, where the wrapped gap reaches its extreme values."""

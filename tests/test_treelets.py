@@ -229,3 +229,90 @@ def test_scratch_of_small_trees_from_a_shared_pool():
             torch.cuda.synchronize()
             w = want[(k + j) % 8]
             assert torch.equal(r[0], w[0]) and torch.equal(r[1], w[1])
+
+
+def spine_keys(blocks, bits):
+    """Sorted keys whose common prefixes fall from the edges of each block of 512 leaves towards its
+    middle, about bits / 4 leaves deep on either side: each of those leaves' parents reaches beyond the
+    block's edge."""
+    low = bits - 6  # a slot of keys for each block
+    c = int("01" * (low // 2 + 1), 2) & ((1 << low) - 1)
+    below = sorted(((c >> j) ^ 1) << j for j in range(low) if c >> j & 1)
+    above = sorted(((c >> j) | 1) << j for j in range(low) if not c >> j & 1)
+    keys = []
+    for b in range(blocks):
+        lo, hi = b << low, (b + 1) << low
+        left, right = [lo + a for a in above], [hi + v for v in below] + [hi + c]
+        fill = 512 - len(left) - len(right)
+        step = (right[0] - left[-1]) // (fill + 1)
+        keys += left + [left[-1] + step * (i + 1) for i in range(fill)] + right
+    return keys
+
+
+def leaving(ot, n):
+    """Subtrees of each block of 512 leaves whose parent reaches beyond it."""
+    node = {}  # first and last leaf
+    for v in np.argsort(-depths(ot, n)):
+        if v >= n - 1:
+            node[v] = (v - (n - 1), v - (n - 1))
+        else:
+            node[v] = (node[ot.left_child[v]][0], node[ot.right_child[v]][1])
+    out = np.zeros((n + 511) // 512, np.int64)
+    for v, (a, b) in node.items():
+        if a // 512 != b // 512 or ot.parent[v] < 0:
+            continue
+        pa, pb = node[ot.parent[v]]
+        out[a // 512] += pa // 512 != pb // 512
+    return out
+
+
+def depths(ot, n):
+    d = np.zeros(2 * n - 1, np.int64)
+    p = ot.parent[:2 * n - 1].astype(np.int64)
+    while (p >= 0).any():
+        d += p >= 0
+        p = np.where(p >= 0, ot.parent[np.maximum(p, 0)], -1)
+    return d
+
+
+@pytest.mark.parametrize("coord", ["f32", "f64", "u64"])
+@pytest.mark.parametrize("blocks", [16, 33])
+def test_climbs_past_the_joins(coord, blocks):
+    """More climbs leave 16 blocks than a join takes: they are passed on, past both levels of joins
+    with 33 blocks, and end in global memory.  Every array and the rows of queries as the oracle's."""
+    cfg = {"f32": (O.F32, O.MORTON, False), "f64": (O.F64, O.PEANO_HILBERT, False),
+           "u64": (O.U64, O.PEANO_HILBERT, True)}[coord]
+    ctx, opts = make(cfg)
+    keys = spine_keys(blocks, 126 if coord == "u64" else 63)
+    n = len(keys)
+    hi = np.array([v >> 64 for v in keys], np.uint64)
+    lo = np.array([v & (2**64 - 1) for v in keys], np.uint64)
+    if cfg[1] == O.MORTON:
+        ref = lo
+    elif coord == "u64":
+        ref = np.stack([np.zeros(n, np.uint64), hi, lo], axis=1)
+    else:
+        ref = np.stack([np.zeros(n, np.uint64), lo >> np.uint64(32), lo & np.uint64(2**32 - 1)], axis=1).astype(np.uint32)
+    rng = np.random.default_rng(blocks)
+    unit = 2.0**42 if coord == "u64" else 1.0
+    xyz = [(p * unit).astype(O.NP_COORD[cfg[0]]) for p in
+           ((np.arange(n) + rng.random(n)) / n, rng.random(n) * 0.05, rng.random(n) * 0.05)]
+    orig = rng.permutation(n).astype(np.int32)
+    ids = rng.integers(0, 1 << 32, n).astype(np.uint32)
+    ghost = rng.integers(0, 2, n).astype(np.int8)
+    ot = O.build_tree(opts, hi if coord == "u64" else None, lo, *xyz, ids, ghost, orig)
+    out = leaving(ot, n)
+    assert out[:16].sum() > 512 and (blocks == 16 or (out[16:32].sum() > 512 and out.sum() > 512))
+    tree = ft.TreeSoA(ctx, n)
+    for a in ("id", "is_ghost", "orig_idx"):  # (build_tree leaves their internal slots alone)
+        getattr(tree, a).view(torch.int8).zero_()
+    ft.build_tree(ctx, tree, ref, *xyz, ids, ghost, orig)
+    assert_tree_equal(tree.to_numpy(), ot, n)
+    oi, od = O.self_knn(opts, ot, 8, True)
+    for method in ("plain", "fast"):
+        gi, gd = ft.self_knn_query(ctx, tree, 8, method=method)
+        torch.cuda.synchronize()
+        assert np.array_equal(gi.cpu().numpy(), oi) and np.array_equal(gd.cpu().numpy(), od), method
+    # the same tree from a refit whose leaves keep their places
+    ft.refit_bvh(ctx, ft.particles(*xyz), tree, leaf_order=True)
+    assert_tree_equal(tree.to_numpy(), ot, n)
