@@ -295,8 +295,8 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// The fast walks' view of every set's tree, as qtree_kernel's for one tree: global leaf g and,
-// inside its set, the internal node of the same number.
+// The fast walks' view of every set's tree (leaf positions and walk records): a thread takes global
+// leaf g and, inside its set, the internal node of the same number.
 template <class T>
 __global__ void __launch_bounds__(256)
     batch_qtree_kernel(const long long *__restrict__ off, const long long *__restrict__ node_off,
@@ -460,7 +460,7 @@ BatchImpl *batch_create(Context &ctx, size_t max_points, size_t max_sets) {
     s.perm        = dalloc<uint32_t>(P);
     s.tmp_perm    = dalloc<uint32_t>(P);
     s.hist        = dalloc<uint32_t>(16 * 256 + 16);
-    s.lookback_words = sort_lookback_words(P, 1);
+    s.lookback_words = sort_lookback_words(P);
     s.lookback       = dalloc<uint32_t>(s.lookback_words);
     s.tile_counter   = dalloc<uint32_t>(16);
     s.status         = dalloc<uint32_t>(4);
@@ -539,12 +539,12 @@ static void batch_build_typed(Context &ctx, BatchImpl &b, const long long *in_of
     FT_CUDA(cudaGetLastError());
     // (key, index) then set: 8 key digits, then the set id's digits
     static const int key_digits[8] = {0, 1, 2, 3, 4, 5, 6, 7};
-    sort_pairs_fixed(s, (size_t)N, 1, 8, key_digits, st);
+    sort_pairs_fixed(s, (size_t)N, 8, key_digits, st);
     if (S > 1) {
         batch_set_key_kernel<<<gN, 256, 0, st>>>(b.off, S, N, s.perm, (unsigned long long *)s.key_lo);
         FT_CUDA(cudaGetLastError());
         const int nd = (S - 1) < 256 ? 1 : (S - 1) < 65536 ? 2 : 3;
-        sort_pairs_fixed(s, (size_t)N, 1, nd, key_digits, st);
+        sort_pairs_fixed(s, (size_t)N, nd, key_digits, st);
     }
     // leaves; internal slots of parent = -1 and id / is_ghost / orig_idx = 0
     const size_t nodes = 2 * (size_t)N;

@@ -5,6 +5,7 @@
 // Reference pipeline: build_bvh (src/hlbvh.hpp:2165-2290) -> compute_bbox (462-572) ->
 // sfc_encode (357-423) -> oneDPL sort (2202-2232) -> gather (2266-2279) -> build_tree
 // (773-982: Karras 861-903, refit 925-969).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -755,32 +756,64 @@ static size_t sort_tiles(size_t n) { // the most tiles any tile size makes
 
 // A tree's scratch in one allocation: the driver maps device memory in blocks of 2 MB and more, some
 // 320 us an allocation above 1 MB whatever its size, and as much again to give it back.  Trees
-// whose scratch is at most kPooled take it from a pool of their context instead, which maps 32 MB at a
-// time (210 us) and hands out pieces in 2 us; it keeps at most kPoolKept unused and goes with its
-// context (with the last such tree, where that outlives it).  Host time of the first build on a new
+// whose scratch is at most kPooled take it from the device's pool instead, which maps 32 MB at a time
+// (210 us, and 140 to make the pool) and hands out pieces in 2 us; it keeps at most kPoolKept unused
+// and goes with the last context and tree that have used it.  Host time of the first build on a new
 // tree, earlier trees kept / destroyed: 4K float points 606 / 250 us with an allocation per array,
 // 800 / 458 with one of its own, 121 / 118 from the pool; 1K 242 / 237 with an allocation per array,
 // 104 / 104 from the pool; 100K double (one of its own) 2160 -> 566 us.  No room to grow is taken
 // beyond what the tree's node arrays hold.
 static constexpr size_t kPooled = size_t(8) << 20, kPoolKept = size_t(32) << 20;
 
+// The current driver context's number (a cudaDeviceReset makes another one); 0: it cannot be read.
+static unsigned long long driver_context_id() {
+    using GetId  = CUresult (*)(CUcontext, unsigned long long *);
+    static GetId fn = [] {
+        void                           *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<GetId>(p);
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0ull;
+}
+
+ScratchPool::~ScratchPool() {
+    int cur = device;
+    cudaGetDevice(&cur);
+    if (cur != device) cudaSetDevice(device);
+    if (pool && driver_context_id() == context) cudaMemPoolDestroy(pool); // (else it went with its context)
+    if (cur != device) cudaSetDevice(cur);
+}
+
 static void *pool_alloc(Context &ctx, size_t bytes, cudaStream_t st) {
-    static std::mutex           making; // (trees of one context may be built by several threads)
-    std::lock_guard<std::mutex> lock(making);
-    if (!ctx.pool) {
+    constexpr int                     kDevices = 64;
+    static std::mutex                 making; // (any thread's contexts and trees)
+    static std::weak_ptr<ScratchPool> pools[kDevices];
+    std::lock_guard<std::mutex>       lock(making);
+    const unsigned long long          context = driver_context_id();
+    if (context == 0 || ctx.device < 0 || ctx.device >= kDevices) return nullptr;
+    if (!ctx.pool) ctx.pool = pools[ctx.device].lock();
+    if (!ctx.pool || ctx.pool->context != context) {
         auto             pool = std::make_shared<ScratchPool>();
         cudaMemPoolProps props{};
         props.allocType         = cudaMemAllocationTypePinned;
         props.location.type     = cudaMemLocationTypeDevice;
         props.location.id       = ctx.device;
         pool->device            = ctx.device;
+        pool->context           = context;
         unsigned long long kept = kPoolKept;
         if (cudaMemPoolCreate(&pool->pool, &props) != cudaSuccess ||
             cudaMemPoolSetAttribute(pool->pool, cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess) {
             cudaGetLastError();
             return nullptr;
         }
-        ctx.pool = pool;
+        ctx.pool          = pool;
+        pools[ctx.device] = pool;
     }
     void *p = nullptr;
     if (cudaMallocFromPoolAsync(&p, bytes, ctx.pool->pool, st) == cudaSuccess) return p;
@@ -1039,8 +1072,7 @@ static int sort_tile_items(int items) { return items == 12 || items == 16 || ite
 
 // The same sort over a fixed list of digit positions of (key_lo, perm) (every listed pass runs),
 // used by the batched build and the query order.
-void sort_pairs_fixed(TreeImpl &s, size_t n, int words, int ndigits, const int *digits, cudaStream_t st) {
-    (void)words; // one-word keys
+void sort_pairs_fixed(TreeImpl &s, size_t n, int ndigits, const int *digits, cudaStream_t st) {
     if (n < 2 || ndigits <= 0) return;
     sort_clear(s, n, ndigits, kSortItems, st);
     radix_hist_kernel<<<grid_for(n, 256, 148 * 4), 256, 0, st>>>((const unsigned long long *)s.key_lo, n, s.hist);
@@ -1054,14 +1086,12 @@ void sort_pairs_fixed(TreeImpl &s, size_t n, int words, int ndigits, const int *
     }
 }
 
-size_t sort_lookback_words(size_t n, int words) {
-    (void)words;
+size_t sort_lookback_words(size_t n) {
     return kSortDigits * sort_tiles(n) * 256;
 }
 
-const int *sort_item_choices(int words, int *count) {
+const int *sort_item_choices(int *count) {
     static const int items[4] = {8, 12, 16, 20}; // the default first
-    (void)words;                                 // (126-bit keys are sorted by their high word)
     *count = 4;
     return items;
 }

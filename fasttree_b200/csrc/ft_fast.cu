@@ -9,9 +9,10 @@
 //     operations in every coordinate type and never exceeds the exact distance, so a child
 //     beyond the k-th distance is skipped safely.  Subtrees of at most 8 leaves are buckets:
 //     their leaves' 32-bit positions are tested by the same bound, and only those within the
-//     k-th distance get the exact distance and the heap.  Trees or queries the frame does not
-//     serve (not finite, far outside the box, a box too long for its dense parts) walk the
-//     binary records with exact distances instead.
+//     k-th distance get the exact distance and the heap.  Queries the frame does not serve (a box
+//     without a frame, a point far outside it, a dense node within reach) walk the binary records
+//     with exact distances instead; trees whose box distances are not monotone (kQFlagPlain) take
+//     the reference traversal alone.
 //  3. Exactness: the result set is the exact k nearest; only the order among equal distances
 //     can differ from the reference (its visit order and heap history decide it).  A lane
 //     flags its query when any tie could matter -- equal distances inside the top k, a
@@ -164,7 +165,7 @@ static void ensure_query_sort(Context &ctx, size_t nq) {
     s.perm           = (uint32_t *)alloc(cap * 4);
     s.tmp_perm       = (uint32_t *)alloc(cap * 4);
     s.hist           = (uint32_t *)alloc((16 * 256 + 16) * 4);
-    s.lookback_words = sort_lookback_words(cap, 1);
+    s.lookback_words = sort_lookback_words(cap);
     s.lookback       = (uint32_t *)alloc(s.lookback_words * 4);
     s.tile_counter   = (uint32_t *)alloc(16 * 4);
     s.cap            = cap;
@@ -213,7 +214,7 @@ static const uint32_t *order_by_rank(Context &ctx, size_t nq, int n, cudaStream_
     int bytes = 1;
     while (bytes < 4 && ((unsigned long long)n >> (8 * bytes)) != 0) ++bytes;
     static const int digits[4] = {0, 1, 2, 3};
-    sort_pairs_fixed(qs, nq, 1, bytes, digits, st);
+    sort_pairs_fixed(qs, nq, bytes, digits, st);
     return qs.perm;
 }
 

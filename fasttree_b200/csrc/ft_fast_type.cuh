@@ -17,10 +17,10 @@
 
 namespace ft {
 
-// The fast walk over queries [0, num), one warp per 32 queries; or, with a list, a grid-stride
-// loop over the list's entries (the count lives on the device: no host synchronisation).
 // Resident blocks the walk is compiled for (a register budget).
 template <class T, int KC> constexpr int fast_min_blocks() { return KC <= 32 ? FT_FAST_MINB : 2 * FT_FAST_MINB; }
+// The fast walk over queries [0, num), `lanes` queries a warp; or, with a list, a grid-stride loop
+// over the list's entries (the count lives on the device: no host synchronisation).
 template <class T, int PER, int KC>
 __global__ void __launch_bounds__(32 * fast_warps<KC>(), fast_min_blocks<T, KC>())
     fast_self_knn_kernel(int lanes, QueryList lst, MissList miss, TreeDev<T> t_all, BatchDev bt, const T *__restrict__ qx,

@@ -27,16 +27,15 @@ void              check_cuda(cudaError_t e, const char *what);
 // Device status word bits (written by kernels instead of trapping).
 enum : uint32_t { STATUS_SPIN_LIMIT = 1u, STATUS_TRAVERSAL_LIMIT = 2u, STATUS_BAD_INPUT = 4u };
 
-// Device memory for the scratch of small trees: a context's, held by its trees too, so that it goes
-// when the last of them has (ensure_scratch).
+// Device memory for the scratch of small trees: one pool a device, shared by the contexts and trees
+// that have used it, so that it goes when the last of them has (ensure_scratch).
 struct ScratchPool {
-    cudaMemPool_t pool = nullptr;
-    int           device = 0;
+    cudaMemPool_t      pool    = nullptr;
+    int                device  = 0;
+    unsigned long long context = 0; // the driver context it belongs to (driver_context_id)
     ScratchPool() = default;
     ScratchPool(const ScratchPool &) = delete;
-    ~ScratchPool() {
-        if (pool) cudaMemPoolDestroy(pool);
-    }
+    ~ScratchPool();
 };
 
 // Library-owned per-tree acceleration data and build scratch (the persistent part plays
@@ -287,8 +286,8 @@ inline void stage_mark(Context *ctx, int i, cudaStream_t st) {
 void build_bvh(Context &ctx, ft_tree &tree, const void *x, const void *y, const void *z, size_t n,
                const uint32_t *id, const int8_t *ghost, const void *bbox_host, const void *caller_keys_dev,
                cudaStream_t st, int sort_items = 0, bool full_sort = false);
-// Tile sizes the build's sort offers for one- or two-word keys (the default first).
-const int *sort_item_choices(int words, int *count);
+// Tile sizes the build's sort offers (the default first).
+const int *sort_item_choices(int *count);
 int        key_words_of(const ft_options &o);
 void build_tree_from_keys(Context &ctx, ft_tree &tree, const void *keys_ref_dev, const void *sx,
                           const void *sy, const void *sz, const uint32_t *sid, const int8_t *sghost,
@@ -300,8 +299,8 @@ void sfc_encode_ref_layout(Context &ctx, TreeImpl &scratch, const void *x, const
 size_t ref_key_bytes(const ft_options &o);
 // Onesweep sort of (key_lo[, key_hi], perm) in s over a fixed digit list (8-bit digits,
 // d < 8: low word, 8 <= d < 16: high word); no host synchronisation.
-void   sort_pairs_fixed(TreeImpl &s, size_t n, int words, int ndigits, const int *digits, cudaStream_t st);
-size_t sort_lookback_words(size_t n, int words);
+void   sort_pairs_fixed(TreeImpl &s, size_t n, int ndigits, const int *digits, cudaStream_t st);
+size_t sort_lookback_words(size_t n);
 // Build scratch for n leaves with room to grow, but never for more than `most` (the leaves the
 // tree's node arrays hold).
 void   ensure_scratch(Context &ctx, TreeImpl &impl, size_t n, size_t most, cudaStream_t st);

@@ -1011,7 +1011,7 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
     int       mine = 0; // this lane's count from staged leaves
     long long part = 0; // leaves in nodes inside every lane's shell, found by this lane
     int       top = 1, lc = 0;
-    bool      overflow = false;
+    bool      overflow = false, dense = false;
     const uint4 *pts = reinterpret_cast<const uint4 *>(t.qpts);
     if (lane == 0) sh.stk[0] = 0;
     __syncwarp();
@@ -1108,10 +1108,7 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
                 else ki |= 1u << i;
             }
         }
-        if (__any_sync(FULL, node >= 0 && rf[0] == kQEmpty)) { // a dense node: each lane's own walk
-            overflow = true;
-            break;
-        }
+        dense = dense || (node >= 0 && rf[0] == kQEmpty);
         const int nl = __popc(kl), ni = __popc(ki);
         int       incl = nl | (ni << 16);
 #pragma unroll
@@ -1131,7 +1128,8 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
         top += tot >> 16;
         __syncwarp();
     }
-    if (overflow) return false; // warp-uniform (every lane ran the same steps)
+    // warp-uniform (every lane ran the same steps); a dense node: each lane's own walk
+    if (overflow || __any_sync(FULL, dense)) return false;
     flush();
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) part += __shfl_xor_sync(FULL, part, m);

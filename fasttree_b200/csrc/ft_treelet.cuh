@@ -10,9 +10,9 @@
 //
 // A block takes kTreeletLeaves consecutive leaves.  Climbs meet in shared memory as long as both
 // sides of a split lie in the block; one whose split or sibling reaches beyond the block's edge
-// is left for the end.  Then the
-// block writes every node it formed -- boxes, children, counts and heights as coalesced arrays,
-// node records, and the fast walks' records -- all of whose descendants are in shared memory.
+// is left for the end.  Then the block writes every node it formed -- boxes, children, counts and
+// heights as coalesced arrays, node records, and the fast walks' records -- all of whose
+// descendants are in shared memory.
 // The climbs that left their blocks (about one leaf in 25) meet again the same way, the climbs of
 // 16 blocks in one block, level by level (treelet_join_kernel).  Climbs that too large groups pass
 // on end in global memory, where the second arrival at a split (one acquire-release exchange)
@@ -47,6 +47,7 @@ FT_D int sort_parity(const uint32_t *skip, int passes) {
 }
 
 static constexpr int kTreeletLeaves = 512, kTreeletThreads = 256;
+static_assert(kTreeletLeaves <= kDenseLeaves, "no node inside a block is dense");
 
 // A point of the sort's input order in one 16- or 32-byte sector: the gather by permutation reads
 // one sector a leaf, not three.
@@ -103,11 +104,11 @@ struct TreeletChild {
     FT_D int node() const { return right ? l : r; } // internal number (l < r)
 };
 
-// The walk record of a node covering [l, r] with split s and box `own`: its two children, then twice the child
+// The walk record of a node covering [l, r] with split s (dense: see qdense): its two children, then twice the child
 // with the most leaves (more than kBucket) replaced by its own two.  split(c): the split of
 // internal child c; box(c, b): its box.
 template <class T, class Split, class Box>
-FT_D void treelet_qrec(int l, int r, int s, const T own[6], const QFrame<T> &f, QRec *out, Split split, Box box) {
+FT_D void treelet_qrec(int l, int r, int s, bool dense, const QFrame<T> &f, QRec *out, Split split, Box box) {
     TreeletChild ch[4] = {{l, s, false}, {s + 1, r, true}, {0, -1, false}, {0, -1, false}};
     int          c     = 2;
 #pragma unroll
@@ -132,8 +133,7 @@ FT_D void treelet_qrec(int l, int r, int s, const T own[6], const QFrame<T> &f, 
         }
         ++c;
     }
-    uint32_t   w[32];
-    const bool dense = qdense<T>(r - l + 1, own, f);
+    uint32_t w[32];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         T b[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
@@ -398,22 +398,22 @@ __global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(const TreeletA
         T                  lb[6], rb[6];
         child_box(cl, lb);
         child_box(cr, rb);
-        T own[6];
 #pragma unroll
-        for (int d = 0; d < 6; ++d) own[d] = s.bx[d][j];
-#pragma unroll
-        for (int d = 0; d < 6; ++d) a.soa[d][v] = own[d];
+        for (int d = 0; d < 6; ++d) a.soa[d][v] = s.bx[d][j];
         a.left[v]   = lc;
         a.right[v]  = rc;
         a.parent[lc] = v;
         a.parent[rc] = v;
         a.leaves[v] = r - l + 1;
         a.height[v] = (uint8_t)h;
-        if (v == 0) treelet_root<T>(a, own); // (number 0 is the root's)
+        if (v == 0) { // (number 0 is the root's)
+            const T rb0[6] = {s.bx[0][0], s.bx[1][0], s.bx[2][0], s.bx[3][0], s.bx[4][0], s.bx[5][0]};
+            treelet_root<T>(a, rb0);
+        }
         treelet_noderec<T>(a.recs + v, lb, rb, lc, rc, cl.count(), cr.count(), l == sp ? 0 : s.nh[sp - b0],
                            sp + 1 == r ? 0 : s.nh[sp + 1 - b0]);
         if (v == 0 || r - l + 1 > kBucket)
-            treelet_qrec<T>(l, r, sp, own, f, a.qrec + v,
+            treelet_qrec<T>(l, r, sp, false, f, a.qrec + v,
                             [&](const TreeletChild &c) { return b0 + (int)s.ns[c.node() - b0]; }, child_box);
     }
     __syncthreads();
@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(128) treelet_qrec_kernel(const TreeletArgs<T> 
         T own[6];
 #pragma unroll
         for (int d = 0; d < 6; ++d) own[d] = a.soa[d][v];
-        treelet_qrec<T>(l, r, split_of(v), own, f, a.qrec + v,
+        treelet_qrec<T>(l, r, split_of(v), qdense<T>(c, own, f), f, a.qrec + v,
                         [&](const TreeletChild &ch) { return split_of(ch.node()); },
                         [&](const TreeletChild &ch, T b[6]) {
                             const int id = ch.l == ch.r ? ch.l + n - 1 : ch.node();

@@ -213,7 +213,7 @@ void tune_build(Context &ctx, ft_tree &tree, const void *x, const void *y, const
     if (n < 2) fail(FT_ERR_INVALID_ARGUMENT, "autotuner: the build needs 2+ points");
     const int  words = key_words_of(ctx.opts);
     int        count = 0;
-    const int *items = sort_item_choices(words, &count);
+    const int *items = sort_item_choices(&count);
     const size_t words8 = (n * sizeof(int32_t) + 7) / 8; // leaf order as 64-bit words (zero padded)
     DevBuf       ref(words8 * 8), cur(words8 * 8), diff(8);
     FT_CUDA(cudaMemsetAsync(ref.p, 0, words8 * 8, st));

@@ -453,9 +453,9 @@ FT_D void fast_warp(const int qbase, const int lanes, const QueryList &lst, cons
     {
         // Warp-synchronous: lanes whose next node is an internal one expand it; a lane that meets a
         // bucket puts it aside and goes on, and waits at its second one, until more lanes wait
-        // than expand.  Then every lane with a bucket aside tests it.  Leaves within reach are queued and offered to the heaps when several
-        // lanes have some (one a lane and round: the exact distances and the heaps' sifts run
-        // with most lanes).
+        // than expand.  Then every lane with a bucket aside tests it.  Leaves within reach are
+        // queued and offered to the heaps when several lanes have some (one a lane and round: the
+        // exact distances and the heaps' sifts run with most lanes).
         uint32_t cur  = 0; // next: a node or a bucket
         uint32_t pb   = kQEmpty; // a bucket put aside
         int      sp   = 0;
