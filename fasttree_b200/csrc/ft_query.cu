@@ -771,12 +771,10 @@ FT_D int range_rows(const TreeDev<T> &t, bool go, const RangePoint<T, PER> &pt, 
 #pragma unroll
                 for (int i = 0; i < (STOP ? 7 : 8); ++i) v[i] = __ldg(p + i);
                 const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
-                if (--budget < 0 || sp + 3 > kRows) {
-                    atomicOr(status, STATUS_TRAVERSAL_LIMIT);
+                if (--budget < 0 || sp + 3 > kRows || w[24] == kQEmpty) {
+                    if (w[24] == kQEmpty) dense = true;
+                    else atomicOr(status, STATUS_TRAVERSAL_LIMIT);
                     have = false;
-                } else if (w[24] == kQEmpty) {
-                    dense = true;
-                    have  = false;
                 } else {
                     pop = true;
 #pragma unroll
@@ -1086,6 +1084,7 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = __ldg(p + i);
             const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
+            dense             = dense || w[24] == kQEmpty;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 rf[i] = w[24 + i];
@@ -1108,7 +1107,6 @@ FT_D bool range_count_group(const TreeDev<T> &t, bool need, const QFrame<T> &fr,
                 else ki |= 1u << i;
             }
         }
-        dense = dense || (node >= 0 && rf[0] == kQEmpty);
         const int nl = __popc(kl), ni = __popc(ki);
         int       incl = nl | (ni << 16);
 #pragma unroll
