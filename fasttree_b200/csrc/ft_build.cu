@@ -732,9 +732,11 @@ void free_scratch(TreeImpl &s) {
         int       cur = dev;
         cudaGetDevice(&cur);
         if (cur != dev) cudaSetDevice(dev);
-        cudaDeviceSynchronize();
-        cudaFreeAsync(s.arena, cudaStreamLegacy);
-        if (s.pool.use_count() == 1) cudaStreamSynchronize(cudaStreamLegacy); // (the pool goes with it)
+        if (cudaDeviceSynchronize() == cudaSuccess) { // (refused under a capture, as cudaFree is: the piece stays)
+            cudaFreeAsync(s.arena, cudaStreamLegacy);
+            if (s.pool.use_count() == 1) cudaStreamSynchronize(cudaStreamLegacy); // (the pool goes with it)
+        }
+        cudaGetLastError();
         if (cur != dev) cudaSetDevice(cur);
     } else if (s.arena) {
         cudaFree(s.arena); // a single tree's: everything below lies in it
